@@ -106,6 +106,10 @@ struct rdsim_handle {
   unsigned long long* obs_counts = nullptr;  // [1 + MAXT]
   int obs_cap = 0;
   unsigned long long* rdf_counts = nullptr;  // [RDF_MAX_BINS]
+  unsigned long long* pair_total = nullptr;  // [2]: neighbour pairs, longest row
+  // the last call ended with a device error: particles may be farther from
+  // their cells than the displacement check allows
+  bool moved_too_far = false;
   int ncells = 0, nscan = 0;
   int *cell_count = nullptr, *cell_start = nullptr, *bsum = nullptr;
   // Verlet-list kernels
@@ -458,6 +462,7 @@ int check_device_error(rdsim_handle* h) {
   CK(cudaMemcpyAsync(&e, h->err, sizeof e, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   if (e.code == 0) return 0;
+  h->moved_too_far = true;
   CK(cudaMemsetAsync(h->err, 0, sizeof(ErrDev), h->stream));
   if (h->period_on) {
     // a period kernel that stopped early may leave draws marked pending
@@ -528,6 +533,7 @@ int upload_state(rdsim_handle* h) {
 }
 
 int initial_drift(rdsim_handle* h) {
+  h->moved_too_far = false;
   CK(cudaMemsetAsync(h->rx_count, 0, 3 * sizeof(int), h->stream));
   int rc = rebuild(h, 0, false, false, h->period_on);
   if (rc) return rc;
@@ -708,7 +714,7 @@ void free_all(rdsim_handle* h) {
   F(h->meta_static_d); F(h->mol_static_d); F(h->flag_d);
   F(h->inj_xi); F(h->inj_u1); F(h->inj_u2); F(h->traj_x); F(h->traj_t);
   F(h->olaws_d); F(h->owalls_d); F(h->oterms_d); F(h->obs_part); F(h->obs_counts);
-  F(h->rdf_counts);
+  F(h->rdf_counts); F(h->pair_total);
   F(h->stamps);
   F(h->stamp_sum);
   for (auto& p : h->pending) {
@@ -736,6 +742,77 @@ float float_up(double v) {
 
 float guard2(double r, double unit) {
   return (float)(r * r * 2e-6 + 2.0 * r * 4.0 * unit + 1e-12);
+}
+
+// Stencil half-widths (cells) that hold every pair closer than r now: such a
+// pair was within r + 2 delta at the last rebuild.  After a call that ended
+// with a device error that bound may not hold: every cell.
+void stencil(const rdsim_handle* h, const SysDev& sd, double r, int* hw) {
+  double maxu = 0;
+  for (int k = 0; k < h->D; k++) maxu = std::max(maxu, (double)sd.unit_hi[k]);
+  for (int k = 0; k < h->D; k++) {
+    const double cell = sd.L[k] / sd.nc[k];
+    const double reach = r + 2.0 * (double)sd.delta * 1.01 + 8.0 * maxu;
+    hw[k] = h->moved_too_far ? sd.nc[k]
+                             : (int)std::min<double>(sd.nc[k], std::floor(reach / cell) + 1.0);
+  }
+}
+
+// Row lengths and offsets of system sys's neighbour pairs (observe.cuh) and
+// tot = {pairs, longest row}.  Scratch: arrays that only a rebuild, a state
+// transfer or the rates hook use, each within its own call.
+int count_pairs(rdsim_handle* h, int sys, PairArgs* o, unsigned long long* tot) {
+  const HostSys& q = h->hs[sys];
+  const SysDev& sd = h->sys_h[sys];
+  std::memset(o, 0, sizeof *o);
+  double maxu = 0;
+  for (int k = 0; k < h->D; k++) maxu = std::max(maxu, (double)sd.unit_hi[k]);
+  o->rs = q.rs;
+  o->rs2_lo = (float)(q.rs * q.rs) - guard2(q.rs, maxu);
+  o->rs2_hi = (float)(q.rs * q.rs) + guard2(q.rs, maxu);
+  o->sys = sys;
+  o->pid0 = q.pid0;
+  stencil(h, sd, q.rs, o->h);
+  o->count = h->tmp;
+  o->start = reinterpret_cast<unsigned long long*>(h->xbuf);
+  o->total = h->pair_total;
+  Args a = make_args(h);
+  const unsigned g = nblk(q.n, PAIR_WARPS);
+  if (h->D == 2) k_pairs_count<2><<<g, PAIR_WARPS * 32, 0, h->stream>>>(a, *o);
+  else if (h->D == 3) k_pairs_count<3><<<g, PAIR_WARPS * 32, 0, h->stream>>>(a, *o);
+  else k_pairs_count<1><<<g, PAIR_WARPS * 32, 0, h->stream>>>(a, *o);
+  k_pairs_scan<<<1, PSCAN_T, 0, h->stream>>>(*o, q.n);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(tot, o->total, 2 * sizeof *tot, cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  return 0;
+}
+
+// The counted pairs into o.out (device) and from there, sorted, to the host.
+int fill_pairs(rdsim_handle* h, const PairArgs& o, const unsigned long long* tot, int32_t* pairs) {
+  const size_t n = (size_t)tot[0];
+  const unsigned g = nblk(h->hs[o.sys].n, PAIR_WARPS);
+  Args a = make_args(h);
+  if (h->D == 2) k_pairs_fill<2><<<g, PAIR_WARPS * 32, 0, h->stream>>>(a, o);
+  else if (h->D == 3) k_pairs_fill<3><<<g, PAIR_WARPS * 32, 0, h->stream>>>(a, o);
+  else k_pairs_fill<1><<<g, PAIR_WARPS * 32, 0, h->stream>>>(a, o);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(pairs, o.out, sizeof(int) * 2 * n, cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  if (tot[1] > (unsigned long long)PAIR_ROW) {  // rows the device left unordered
+    struct P {
+      int32_t i, j;
+    };
+    P* v = reinterpret_cast<P*>(pairs);
+    for (size_t b = 0; b < n;) {
+      size_t e = b + 1;
+      while (e < n && v[e].i == v[b].i) e++;
+      if (e - b > (size_t)PAIR_ROW)
+        std::sort(v + b, v + e, [](const P& x, const P& y) { return x.j < y.j; });
+      b = e;
+    }
+  }
+  return 0;
 }
 
 }  // namespace
@@ -1331,6 +1408,7 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
   if ((rc = dalloc(&h->flag_d, 1, &B))) return bail(rc);
   if ((rc = dalloc(&h->err, 1, &B))) return bail(rc);
   if ((rc = dalloc(&h->step_dev, 1, &B))) return bail(rc);
+  if ((rc = dalloc(&h->pair_total, 2, &B))) return bail(rc);
   {
     if ((rc = dalloc(&h->chunks_d, h->chunks_h.size(), &B))) return bail(rc);
     if ((rc = dalloc(&h->nbr, (size_t)h->W * h->npad, &B))) return bail(rc);
@@ -1580,50 +1658,20 @@ int rdsim_get_reaction_rates(rdsim_handle* h, double* total) {
 int rdsim_get_pairs(rdsim_handle* h, int32_t sys, int32_t* pairs, int64_t cap, int64_t* n_pairs) {
   if (!h || sys < 0 || sys >= h->nsys || !n_pairs) return fail(RDSIM_ERR_ARG, "bad argument");
   CK(cudaSetDevice(h->device));
-  const HostSys& q = h->hs[sys];
-  const SysDev& sd = h->sys_h[sys];
-  unsigned long long* cnt = nullptr;
-  int* buf = nullptr;
-  size_t bcap = (size_t)std::max<int64_t>(cap, 1);
-  if (cudaMalloc(&cnt, sizeof(unsigned long long)) != cudaSuccess) {
+  PairArgs o;
+  unsigned long long tot[2] = {0ull, 0ull};
+  int rc = count_pairs(h, sys, &o, tot);
+  if (rc) return rc;
+  const unsigned long long n = tot[0];
+  *n_pairs = (int64_t)n;
+  if ((int64_t)n > cap) return fail(RDSIM_ERR_CAPACITY, "pair buffer too small");
+  if (n == 0 || !pairs) return 0;
+  if (cudaMalloc(&o.out, sizeof(int) * 2 * n) != cudaSuccess) {
     cudaGetLastError();
-    return fail(RDSIM_ERR_NOMEM, "pair counter");
-  }
-  if (cudaMalloc(&buf, sizeof(int) * 2 * bcap) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(cnt);
     return fail(RDSIM_ERR_NOMEM, "pair buffer");
   }
-  cudaMemsetAsync(cnt, 0, sizeof(unsigned long long), h->stream);
-  double maxu = 0;
-  for (int k = 0; k < h->D; k++) maxu = std::max(maxu, (double)sd.unit_hi[k]);
-  float rs2_hi = (float)(q.rs * q.rs) + guard2(q.rs, maxu);
-  Args a = make_args(h);
-  unsigned g = nblk(q.n);
-  if (h->D == 2) k_pairs<2><<<g, 256, 0, h->stream>>>(h->sys_d, sys, a, h->tmpl_d, q.rs, rs2_hi, q.p0, q.n, q.pid0, buf, (unsigned long long)cap, cnt);
-  else if (h->D == 3) k_pairs<3><<<g, 256, 0, h->stream>>>(h->sys_d, sys, a, h->tmpl_d, q.rs, rs2_hi, q.p0, q.n, q.pid0, buf, (unsigned long long)cap, cnt);
-  else k_pairs<1><<<g, 256, 0, h->stream>>>(h->sys_d, sys, a, h->tmpl_d, q.rs, rs2_hi, q.p0, q.n, q.pid0, buf, (unsigned long long)cap, cnt);
-  unsigned long long n = 0;
-  cudaError_t e1 = cudaGetLastError();
-  cudaMemcpyAsync(&n, cnt, sizeof n, cudaMemcpyDeviceToHost, h->stream);
-  cudaStreamSynchronize(h->stream);
-  *n_pairs = (int64_t)n;
-  int rc = 0;
-  if (e1 != cudaSuccess) rc = fail(RDSIM_ERR_CUDA, cudaGetErrorString(e1));
-  else if ((int64_t)n > cap) rc = fail(RDSIM_ERR_CAPACITY, "pair buffer too small");
-  else if (n > 0 && pairs) {
-    std::vector<int> tmp(2 * n);
-    cudaMemcpy(tmp.data(), buf, sizeof(int) * 2 * n, cudaMemcpyDeviceToHost);
-    std::vector<std::pair<int, int>> v(n);
-    for (size_t p = 0; p < n; p++) v[p] = {tmp[2 * p], tmp[2 * p + 1]};
-    std::sort(v.begin(), v.end());
-    for (size_t p = 0; p < n; p++) {
-      pairs[2 * p] = v[p].first;
-      pairs[2 * p + 1] = v[p].second;
-    }
-  }
-  cudaFree(cnt);
-  cudaFree(buf);
+  rc = fill_pairs(h, o, tot, pairs);
+  cudaFree(o.out);
   return rc;
 }
 
@@ -1720,11 +1768,8 @@ int rdsim_get_rdf(rdsim_handle* h, int32_t sys, int32_t type_a, int32_t type_b, 
     if (((sd.periodic >> k) & 1) && r_max > 0.5 * q.L[k])
       return fail(RDSIM_ERR_ARG, "r_max exceeds half of a periodic box length");
     maxu = std::max(maxu, (double)sd.unit_hi[k]);
-    // pairs closer than r_max now were within r_max + 2 delta at the rebuild
-    const double cell = q.L[k] / sd.nc[k];
-    const double reach = r_max + 2.0 * (double)sd.delta * 1.01 + 8.0 * maxu;
-    o.h[k] = (int)std::min<double>(sd.nc[k], std::floor(reach / cell) + 1.0);
   }
+  stencil(h, sd, r_max, o.h);
   CK(cudaSetDevice(h->device));
   if (!h->rdf_counts && cudaMalloc(&h->rdf_counts, sizeof(unsigned long long) * RDF_MAX_BINS) != cudaSuccess) {
     cudaGetLastError();
@@ -1734,6 +1779,10 @@ int rdsim_get_rdf(rdsim_handle* h, int32_t sys, int32_t type_a, int32_t type_b, 
   o.r_max = r_max;
   o.width = r_max / n_bins;
   o.r2_hi = (float)(r_max * r_max) + guard2(r_max, maxu);
+  // the float32 distance errs by less than 1e-6 r + 2 sqrt(3) units of the
+  // high word (and its quotient by 2e-7 of itself); the band is twice that
+  o.inv_width = (float)(1.0 / o.width);
+  o.edge = (float)((2.4e-6 * r_max + 8.0 * maxu) / o.width);
   o.sys = sys;
   o.type_a = type_a;
   o.type_b = type_b;
@@ -1741,7 +1790,7 @@ int rdsim_get_rdf(rdsim_handle* h, int32_t sys, int32_t type_a, int32_t type_b, 
   o.flags = flags;
   CK(cudaMemsetAsync(h->rdf_counts, 0, sizeof(unsigned long long) * n_bins, h->stream));
   Args a = make_args(h);
-  const unsigned nb = (unsigned)std::max(1, (q.n + OBS_BLOCK - 1) / OBS_BLOCK);
+  const unsigned nb = std::min(nblk(q.n, OBS_BLOCK / RDF_LANES), 6u * 152u);
   {
     ProfScope ps(h, 4, 1);
     if (h->D == 2) k_rdf<2><<<nb, OBS_BLOCK, 0, h->stream>>>(a, o);
@@ -1913,30 +1962,29 @@ int rdsim_test_withhold(rdsim_handle* h, int32_t chunk) {
 // ---------------------------------------------------------------------------
 // Neighbour pairs without allocation.
 //
-// rdsim_get_pairs allocates its device scratch (a pair counter and a pair
-// buffer) with cudaMalloc and releases it with cudaFree on every call.  Some
-// callers cannot do that: processes whose device memory is fully committed
-// (a preallocated pool, another framework's cache), where cudaMalloc fails,
-// and loops that must not pay the device-wide synchronisation of cudaFree.
-// rdsim_get_pairs_static computes the same sorted pair list into the
-// caller's host buffer with its scratch in the static device array below
-// instead.
+// rdsim_get_pairs allocates its device pair buffer with cudaMalloc and
+// releases it with cudaFree on every call.  Some callers cannot do that:
+// processes whose device memory is fully committed (a preallocated pool,
+// another framework's cache), where cudaMalloc fails, and loops that must not
+// pay the device-wide synchronisation of cudaFree.  rdsim_get_pairs_static
+// computes the same sorted pair list into the caller's host buffer with its
+// pair buffer in the static device array below instead (the row lengths and
+// offsets are scratch of the handle in both).
 //
-// The array is RDSIM_STATIC_PAIRS_MAX pairs (8 MiB) plus a counter; every GPU
-// that loads the library holds it until the process exits.  Its device
-// address belongs to the CUDA context that loaded the module: it is looked up
+// The array is RDSIM_STATIC_PAIRS_MAX pairs (8 MiB); every GPU that loads the
+// library holds it until the process exits.  Its device address belongs to the CUDA context that loaded the module: it is looked up
 // (cudaGetSymbolAddress, with that device current) by the first call in each
 // context on a device and again after the context changes (a cudaDeviceReset
 // makes a new primary context, and with it a new array), under a lock.  The
-// same set-up also loads k_pairs for every dimension, so that under lazy
-// module loading no later call loads code.  All calls share the array: the
-// counter is cleared at the start of every call, and calls that overlap on
-// the GPU (from several threads or handles at once) race on it.
+// same set-up also loads the pair kernels of every dimension, so that under
+// lazy module loading no later call loads code.  All calls share the array:
+// calls that overlap on the GPU (from several threads or handles at once)
+// race on it.
 namespace {
 
 constexpr long long kStaticPairsMax = RDSIM_STATIC_PAIRS_MAX;
-// [0]: pair counter; [1 + p]: pair p as two int32 (i, j)
-static __device__ __align__(256) unsigned long long g_pairs_scratch[1 + kStaticPairsMax];
+// pair p as two int32 (i, j)
+static __device__ __align__(256) unsigned long long g_pairs_scratch[kStaticPairsMax];
 
 constexpr int kMaxDevices = 64;
 struct ScratchSlot {
@@ -1991,11 +2039,13 @@ int static_scratch(int device, unsigned long long** out) {
     // load the pair kernels of every dimension now (lazy loading would
     // otherwise load each on its first launch)
     cudaFuncAttributes fa;
-    const cudaError_t e1 = cudaFuncGetAttributes(&fa, k_pairs<1>);
-    const cudaError_t e2 = cudaFuncGetAttributes(&fa, k_pairs<2>);
-    const cudaError_t e3 = cudaFuncGetAttributes(&fa, k_pairs<3>);
-    if (e1 != cudaSuccess || e2 != cudaSuccess || e3 != cudaSuccess)
-      return fail(RDSIM_ERR_CUDA, "loading the pair kernels failed");
+    const cudaError_t loads[7] = {
+        cudaFuncGetAttributes(&fa, k_pairs_count<1>), cudaFuncGetAttributes(&fa, k_pairs_fill<1>),
+        cudaFuncGetAttributes(&fa, k_pairs_count<2>), cudaFuncGetAttributes(&fa, k_pairs_fill<2>),
+        cudaFuncGetAttributes(&fa, k_pairs_count<3>), cudaFuncGetAttributes(&fa, k_pairs_fill<3>),
+        cudaFuncGetAttributes(&fa, k_pairs_scan)};
+    for (cudaError_t q : loads)
+      if (q != cudaSuccess) return fail(RDSIM_ERR_CUDA, "loading the pair kernels failed");
     slot.ptr = static_cast<unsigned long long*>(p);
     slot.ctx_id = id;
     slot.valid = have_id;
@@ -2013,24 +2063,10 @@ extern "C" int rdsim_get_pairs_static(rdsim_handle* h, int32_t sys, int32_t* pai
   unsigned long long* scratch = nullptr;
   int rc = static_scratch(h->device, &scratch);
   if (rc) return rc;
-  const HostSys& q = h->hs[sys];
-  const SysDev& sd = h->sys_h[sys];
-  CK(cudaMemsetAsync(scratch, 0, sizeof(unsigned long long), h->stream));
-  double maxu = 0;
-  for (int k = 0; k < h->D; k++) maxu = std::max(maxu, (double)sd.unit_hi[k]);
-  const float rs2_hi = (float)(q.rs * q.rs) + guard2(q.rs, maxu);
-  Args a = make_args(h);
-  const unsigned g = nblk(q.n);
-  int* buf = reinterpret_cast<int*>(scratch + 1);
-  unsigned long long* cnt = scratch;
-  const unsigned long long lim = (unsigned long long)kStaticPairsMax;
-  if (h->D == 2) k_pairs<2><<<g, 256, 0, h->stream>>>(h->sys_d, sys, a, h->tmpl_d, q.rs, rs2_hi, q.p0, q.n, q.pid0, buf, lim, cnt);
-  else if (h->D == 3) k_pairs<3><<<g, 256, 0, h->stream>>>(h->sys_d, sys, a, h->tmpl_d, q.rs, rs2_hi, q.p0, q.n, q.pid0, buf, lim, cnt);
-  else k_pairs<1><<<g, 256, 0, h->stream>>>(h->sys_d, sys, a, h->tmpl_d, q.rs, rs2_hi, q.p0, q.n, q.pid0, buf, lim, cnt);
-  CK(cudaGetLastError());
-  unsigned long long n = 0;
-  CK(cudaMemcpyAsync(&n, cnt, sizeof n, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
+  PairArgs o;
+  unsigned long long tot[2] = {0ull, 0ull};
+  if ((rc = count_pairs(h, sys, &o, tot))) return rc;
+  const unsigned long long n = tot[0];
   *n_pairs = (int64_t)n;
   if ((long long)n > kStaticPairsMax)
     return fail(RDSIM_ERR_CAPACITY,
@@ -2038,13 +2074,6 @@ extern "C" int rdsim_get_pairs_static(rdsim_handle* h, int32_t sys, int32_t* pai
                     std::to_string(kStaticPairsMax) + " pairs; use rdsim_get_pairs");
   if ((int64_t)n > cap) return fail(RDSIM_ERR_CAPACITY, "pair buffer too small");
   if (n == 0 || !pairs) return 0;
-  CK(cudaMemcpyAsync(pairs, buf, sizeof(int) * 2 * n, cudaMemcpyDeviceToHost, h->stream));
-  CK(cudaStreamSynchronize(h->stream));
-  // sort in the caller's buffer: (i, j) pairs of int32 viewed as one key each
-  struct P {
-    int32_t i, j;
-  };
-  P* v = reinterpret_cast<P*>(pairs);
-  std::sort(v, v + n, [](const P& x, const P& y) { return x.i != y.i ? x.i < y.i : x.j < y.j; });
-  return 0;
+  o.out = reinterpret_cast<int*>(scratch);
+  return fill_pairs(h, o, tot, pairs);
 }

@@ -1134,45 +1134,4 @@ __global__ void k_ref_cells(const SysDev* sysv, int sys, Args a, const double* c
   }
 }
 
-// neighbour list as the reference would rebuild it now (pyrdsim.pyx:1448-1587):
-// bonded-list pairs plus partner-type pairs of different molecules, d <= rs.
-template <int D>
-__global__ void k_pairs(const SysDev* sysv, int sys, Args a, const TmplDev* tmpl, double rs,
-                        float rs2_hi, int p0, int n, int pid0, int* out, unsigned long long cap,
-                        unsigned long long* count) {
-  pdl_trigger();
-  pdl_wait();
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const SysDev& s = sysv[sys];
-  const int gi = p0 + i;
-  const uint32_t mi = a.meta[gi];
-  const int pi = a.pid[gi] - pid0;
-  const int ti = mi & 0xff, loci = (mi >> 16) & 0xff, tmi = mi >> 24;
-  const uint32_t bmask = tmi != 0xff ? tmpl[tmi].bondmask[loci] : 0u;
-  for (int j = 0; j < n; j++) {
-    const int gj = p0 + j;
-    const int pj = a.pid[gj] - pid0;
-    if (pj <= pi) continue;
-    const uint32_t mj = a.meta[gj];
-    bool listed;
-    if (a.mol[gj] == a.mol[gi]) listed = (bmask >> ((mj >> 16) & 31)) & 1;
-    else listed = (s.partner[ti] >> (mj & 0xff)) & 1;
-    if (!listed) continue;
-    float r2 = 0.f;
-#pragma unroll
-    for (int k = 0; k < D; k++) {
-      float dx = (float)(int)(a.xh[k][gj] - a.xh[k][gi]) * s.unit_hi[k];
-      r2 += dx * dx;
-    }
-    if (r2 > rs2_hi) continue;
-    if (exact_dist<D>(s, a, gi, gj) > rs) continue;
-    unsigned long long slot = atomicAdd(count, 1ull);
-    if (slot < cap) {
-      out[2 * slot] = pi;
-      out[2 * slot + 1] = pj;
-    }
-  }
-}
-
 }  // namespace rd
