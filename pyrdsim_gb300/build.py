@@ -1,9 +1,10 @@
 """Builds the CUDA engine ``pyrdsim_gb300/_lib/librdsim.so`` for sm_103a.
 
-Three translation units (``csrc/engine.cu``: the step engine and
-observables; ``csrc/force64.cu``: the float64 drift kernels;
-``csrc/adjoint.cu``: the differentiable reaction-free steps) compiled by nvcc
-in parallel and linked into one plain shared library with a C ABI
+Seven translation units (``csrc/engine.cu``: the step engine and observables;
+``csrc/period1.cu`` to ``period3.cu``: the period kernel by dimension;
+``csrc/force32.cu`` and ``csrc/force64.cu``: the float32 and float64 drift
+kernels; ``csrc/adjoint.cu``: the differentiable reaction-free steps) compiled
+by nvcc in parallel and linked into one plain shared library with a C ABI
 (``include/rdsim.h``, ``include/rdsim_adjoint.h``); no PyTorch headers.
 """
 from __future__ import annotations
@@ -30,7 +31,7 @@ def _nvcc():
     raise RuntimeError("nvcc not found")
 
 
-UNITS = ["engine.cu", "force64.cu", "adjoint.cu"]
+UNITS = ["engine.cu", "force32.cu", "period1.cu", "period2.cu", "period3.cu", "force64.cu", "adjoint.cu"]
 
 
 def sources():

@@ -110,6 +110,7 @@ struct SysDev {
   float R2;                       // candidate radius^2 (forces + reactions)
   float Rrx2;                     // reaction radius^2 (guarded)
   float Rl2;                      // Verlet-list radius^2: range + 2 delta
+  float Rrl2;                     // the same for the reactions' range alone
   double dt;
   unsigned long long seed;
   float fp[MAXT], npf[MAXT];      // dt*D and sqrt(2 dt D) per type
@@ -120,7 +121,7 @@ struct SysDev {
   unsigned char rxmatch[MAXT * MAXT]; // bit r of [ti * MAXT + tj]: neighbour
                                       // reaction r has reactant ti and counts tj
   // Upper bound of a particle's total propensity for the reaction prefilter:
-  // rxA[t] + rxB[t] * (listed neighbours) >= the float64 total of a type-t
+  // rxA[t] + rxB[t] * (Args::rcnt) >= the float64 total of a type-t
   // particle (linear and inhibited rates in rxA, catalysed rates in rxB).
   double rxA[MAXT], rxB[MAXT];
   float rxAf[MAXT], rxBf[MAXT];   // the same as float32, rounded up
@@ -186,8 +187,11 @@ struct Args {
   const Chunk* chunks;            // list kernels: CTA -> particle run
   const int* nbr;                 // Verlet list (ELL, see list.cuh)
   const int* ncnt;                // entries per particle (may exceed W)
+  const int* rcnt;                // entries that can come within a reaction
+                                  // radius before the next rebuild
   int* nbr_out;
   int* ncnt_out;
+  int* rcnt_out;
   int W, npad;                    // list width and particle stride
   int4* rx_list;                  // [3][npad]: particles whose reaction draw
                                   // may succeed at a step, in slot step % 3,
@@ -202,45 +206,53 @@ struct Args {
   // values of each CTA's start and end, slot = step mod ring
   unsigned long long* stamps;
   int stamp_ring;
-  // period kernel (list.cuh: k_period), written by the list builder with
-  // F_PERIOD_PREP: per chunk, the bitmap of the chunks its particles read
-  // (list entries and bonded partners, itself included; PMASK_WORDS words),
-  // the particles whose reaction draw of the rebuild step may succeed
-  // (CAND_WORDS words, bit = particle within the chunk) and the progress word
-  uint32_t* nbmask;
-  uint32_t* cand0;
-  int* pflag;
+  // neighbour staging (list.cuh), written by the list builder: per chunk, the
+  // number of staged particles (-1: not staged), their sorted indices
+  // (stg_max per chunk) and the list rows as slot codes (kw words of two
+  // 16-bit codes per lane)
+  int* stg_n;
+  int* stg_g;
+  uint32_t* codes;
+  int stg_max, kw, rows_max;      // rows_max: most type pairs of a system
+  // period kernel (period.cuh): tagged records of every particle, by parity of
+  // the step within the launch
+  uint4* rec[2];                  // pair words, type word with the step's tag
+  uint4* recl[2];                 // low words, tag
+  uint4* rech[2];                 // high words, tag
   long long wait_ns;              // period kernel: limit of one wait (ns)
 };
 
-// Period kernel: a particle whose reaction draw of the next step is pending
-// carries this bit in that step's type word (bits 21-23 of the atom-index
-// byte are otherwise zero: at most 32 atoms per molecule) until its chunk
-// has resolved the draw and written the final word.
-constexpr uint32_t META_PENDING = 1u << 23;
+// Type word of a period kernel's record: the type after the step's reactions
+// (the type before them while the draw is pending), the type before them, the
+// pending mark, and the step within the launch as a 23-bit tag.
+constexpr int REC_OLD = 4, REC_TAG = 9;
+constexpr uint32_t REC_PENDING = 1u << 8;
+constexpr uint32_t REC_NONE = 0xffffffffu;  // no step yet
+__host__ __device__ inline uint32_t rec_word(int n, uint32_t type, uint32_t old, bool pending) {
+  return ((uint32_t)n << REC_TAG) | (old << REC_OLD) | type | (pending ? REC_PENDING : 0u);
+}
+// A record is of step n or later (a particle nobody lists here may be ahead).
+__device__ inline bool rec_ready(uint32_t word, int shift, int n) {
+  return (int)(((word >> shift) - (uint32_t)n) << shift) >= 0;
+}
 
-// Period kernel limits: chunks of one launch (bitmap width) and particles
-// per chunk (candidate mask width).
-constexpr int PMASK_WORDS = 40;
-constexpr int PMAX_CHUNKS = PMASK_WORDS * 32;
+// Most particles a chunk stages and most code words per lane (shared memory of
+// the period kernel: the limit is set to this much for every handle, whatever
+// it uses, because it belongs to the kernel and not to the handle).
+constexpr int STG_LIMIT = 2048;
+constexpr int KW_LIMIT = 64;
+
+// Words of a chunk's candidate mask (bit = particle within the chunk).
 constexpr int CAND_WORDS = 4;
-// Ints per progress word of the period kernel (32: one 128-byte line each,
-// so that the ~20 CTAs polling a chunk do not share a line with others).
-#ifndef RD_PERIOD_FLAG_STRIDE
-#define RD_PERIOD_FLAG_STRIDE 32
-#endif
-constexpr int PFLAG_STRIDE = RD_PERIOD_FLAG_STRIDE;
 
-// Arguments of the period kernel besides its four step-argument blocks.
+// Arguments of the period kernel besides its step arguments.
 struct PeriodArgs {
-  int nsteps;                     // steps of the rebuild period
-  int nchunks;                    // chunks = CTAs (all resident)
-  int rx;                         // prefiltered reaction phases run
+  int nsteps;                     // steps of the launch
   int first_rx;                   // the first step's reactions run here (its
                                   // candidates from the list builder); 0: done
                                   // before the launch
   int withhold;                   // test hook: this chunk never publishes
-                                  // its progress (-1: none)
+                                  // its records (-1: none)
   long long wait_ns;              // limit of one wait (global timer, ns)
 };
 
@@ -261,11 +273,10 @@ enum : int {
                                   // list the particles whose reaction draw of
                                   // the next step may succeed
   F_RX_HERE = 128,                // list builder: the same for its own step
-  F_PERIOD = 256,                 // step kernels inside k_period: the step
+  F_PERIOD = 256,                 // step functions inside k_period: the step
                                   // number is the CTA's current step
-  F_PERIOD_PREP = 512             // list builder: write the period kernel's
-                                  // neighbour-chunk bitmaps, progress words
-                                  // and (with F_RX_HERE) candidate masks
+  F_PERIOD_PREP = 512             // list builder: write the records of the
+                                  // period kernel's first step
 };
 
 // Slot of the candidate list of a step: three slots, so that a drift kernel

@@ -20,10 +20,12 @@
 #include "../../include/rdsim.h"
 #include "device.cuh"
 #include "kernels.cuh"
+#include "force32.h"
 #include "force64.h"
 #include "launch.cuh"
 #include "list.cuh"
 #include "observe.cuh"
+#include "period.h"
 
 using namespace rd;
 
@@ -46,6 +48,13 @@ int fail(int code, const std::string& msg) {
       return fail(RDSIM_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
     }                                                                             \
   } while (0)
+
+// Chunks per SM up to which the period kernel takes more lanes per chain (the
+// whole call, 100 steps, with 1 / 4 lanes: 648 / 551 us for the LJ fluid at
+// 1,024 particles, 981 / 913 us for the inhibited mixture at 5,003).  In 3D
+// never: a chunk of a quarter of the particles still stages two thirds of the
+// neighbours (1,945 / 2,499 us for 50 steps at 13,824 particles).
+constexpr int LPC_CHUNKS = 6;
 
 constexpr double TWO32 = 4294967296.0;
 constexpr double TWO64 = 18446744073709551616.0;
@@ -119,17 +128,28 @@ struct rdsim_handle {
   int* rx_count = nullptr;           // [3]
   int W = 0;                         // list width (entries per particle)
   int npad = 0;                      // particle stride of the list
-  // period kernel (list.cuh: k_period): one launch per graph-replayed period
+  // neighbour staging of the period kernel (list.cuh)
+  int stg_max = 0, kw = 0, rows = 1; // staged particles per chunk, code words per lane,
+                                     // type pairs
+  int* stg_n = nullptr;              // [chunks]
+  int* stg_g = nullptr;              // [chunks][stg_max]
+  uint32_t* codes = nullptr;         // [chunks][kw][LBLOCK]
+  // period kernel (period.cuh): the steps between two rebuilds in one launch
+  bool all_lj6 = true;               // every pair law is a single Lennard-Jones n = 6
   bool period_on = false;
-  uint32_t* nbmask = nullptr;        // [chunks][PMASK_WORDS]
-  uint32_t* cand0 = nullptr;         // [chunks][CAND_WORDS]
-  int* pflag = nullptr;              // [chunks] progress words
+  int lpc = 1;                       // its lanes per chain (period.cuh)
+  std::vector<Chunk> pchunks_h;      // its chunks
+  Chunk* pchunks_d = nullptr;
+  uint4* rec[2] = {};                // [N] records by parity of the step
+  uint4* recl[2] = {};
+  uint4* rech[2] = {};
   int withhold = -1;                 // test hook (rdsim_test_withhold)
   long long wait_ns = 1000000000LL;
   std::vector<Chunk> chunks_h;
   Chunk* chunks_d = nullptr;
   int* nbr = nullptr;
   int* ncnt = nullptr;
+  int* rcnt = nullptr;
   int *cell_of = nullptr, *rank_of = nullptr, *tmp = nullptr, *sid = nullptr, *slot_of = nullptr;
   uint32_t* xh[2][3] = {};
   uint32_t* xl[2][3] = {};
@@ -204,6 +224,12 @@ cudaEvent_t take_event(rdsim_handle* h) {
   return e;
 }
 
+// CTAs of the launches that record timestamps: the period kernel's, else the
+// drift kernel's.
+size_t stamp_ctas(const rdsim_handle* h) {
+  return std::max<size_t>(1, h->period_on ? h->pchunks_h.size() : h->chunks_h.size());
+}
+
 // Brackets the launches of one class with events when profiling is on.
 struct ProfScope {
   rdsim_handle* h;
@@ -275,8 +301,10 @@ Args make_args(rdsim_handle* h) {
   a.chunks = h->chunks_d;
   a.nbr = h->nbr;
   a.ncnt = h->ncnt;
+  a.rcnt = h->rcnt;
   a.nbr_out = h->nbr;
   a.ncnt_out = h->ncnt;
+  a.rcnt_out = h->rcnt;
   a.W = h->W;
   a.rx_list = h->rx_list;
   a.rx_count = h->rx_count;
@@ -288,25 +316,27 @@ Args make_args(rdsim_handle* h) {
     a.stamp_ring = h->stamp_ring;
   }
   if (!h->chunks_h.empty()) a.chunk1 = h->chunks_h[0];
-  a.nbmask = h->nbmask;
-  a.cand0 = h->cand0;
-  a.pflag = h->pflag;
+  a.stg_n = h->stg_n;
+  a.stg_g = h->stg_g;
+  a.codes = h->codes;
+  a.stg_max = h->stg_max;
+  a.kw = h->kw;
+  a.rows_max = h->rows;
+  for (int b = 0; b < 2; b++) {
+    a.rec[b] = h->rec[b];
+    a.recl[b] = h->recl[b];
+    a.rech[b] = h->rech[b];
+  }
   return a;
 }
 
-template <int D, int TPP>
-void launch_list(rdsim_handle* h, bool react, const Args& a) {
-  const dim3 grid((unsigned)h->chunks_h.size());
-  if (react) launch(k_react_l<D, TPP>, grid, LBLOCK, h->stream, a);
-  else launch(k_force_l<D, TPP>, grid, LBLOCK, h->stream, a);
-}
-
 template <int D>
-void launch_list_d(rdsim_handle* h, bool react, const Args& a) {
-  if (h->ltpp == 1) launch_list<D, 1>(h, react, a);
-  else if (h->ltpp == 2) launch_list<D, 2>(h, react, a);
-  else if (h->ltpp == 8) launch_list<D, 8>(h, react, a);
-  else launch_list<D, 4>(h, react, a);
+void launch_react(rdsim_handle* h, const Args& a) {
+  const unsigned g = (unsigned)h->chunks_h.size();
+  if (h->ltpp == 1) launch(k_react_l<D, 1>, g, LBLOCK, h->stream, a);
+  else if (h->ltpp == 2) launch(k_react_l<D, 2>, g, LBLOCK, h->stream, a);
+  else if (h->ltpp == 8) launch(k_react_l<D, 8>, g, LBLOCK, h->stream, a);
+  else launch(k_react_l<D, 4>, g, LBLOCK, h->stream, a);
 }
 
 template <int D>
@@ -317,20 +347,27 @@ void launch_listed(rdsim_handle* h, unsigned g, const Args& a) {
   else launch(k_react_listed<D, 4>, g, LBLOCK, h->stream, a);
 }
 
-template <int D>
-void launch_nlist(rdsim_handle* h, const Args& a) {
-  const dim3 grid((unsigned)h->chunks_h.size());
-  const unsigned per = (unsigned)(LBLOCK / h->ltpp * (D == 1 ? 1 : 3));
-  if (h->ltpp == 1) launch(k_nlist<D, 1>, grid, per, h->stream, a);
-  else if (h->ltpp == 2) launch(k_nlist<D, 2>, grid, per, h->stream, a);
-  else if (h->ltpp == 8) launch(k_nlist<D, 8>, grid, per, h->stream, a);
-  else launch(k_nlist<D, 4>, grid, per, h->stream, a);
+template <int D, int TPP, int LPC>
+void launch_nlist_v(rdsim_handle* h, const Args& a) {
+  const unsigned per = (unsigned)(LBLOCK / TPP / LPC * (D == 1 ? 1 : 3));
+  launch(k_nlist<D, TPP, LPC>, (unsigned)h->pchunks_h.size(), per, h->stream, a);
 }
 
-void launch_step_kernel(rdsim_handle* h, bool react, const Args& a) {
-  if (h->D == 2) launch_list_d<2>(h, react, a);
-  else if (h->D == 3) launch_list_d<3>(h, react, a);
-  else launch_list_d<1>(h, react, a);
+template <int D>
+void launch_nlist(rdsim_handle* h, Args a) {
+  a.chunks = h->pchunks_d;
+  if (h->ltpp == 1) launch_nlist_v<D, 1, 1>(h, a);
+  else if (h->ltpp == 8) launch_nlist_v<D, 8, 1>(h, a);
+  else if (h->ltpp == 4) launch_nlist_v<D, 4, 1>(h, a);
+  else if (h->lpc == 4) launch_nlist_v<D, 2, 4>(h, a);
+  else if (h->lpc == 2) launch_nlist_v<D, 2, 2>(h, a);
+  else launch_nlist_v<D, 2, 1>(h, a);
+}
+
+void launch_react(rdsim_handle* h, const Args& a) {
+  if (h->D == 2) launch_react<2>(h, a);
+  else if (h->D == 3) launch_react<3>(h, a);
+  else launch_react<1>(h, a);
 }
 
 unsigned nblk(int n, int b = 256) { return (unsigned)((n + b - 1) / b); }
@@ -398,7 +435,7 @@ int force(rdsim_handle* h, long long step, int flags, const double* xi_next, boo
   {
     ProfScope ps(h, P_FORCE, 1);
     if (h->f64) CK(launch_force64(h->D, h->ltpp, (unsigned)h->chunks_h.size(), h->stream, a));
-    else launch_step_kernel(h, false, a);
+    else CK(launch_force32(h->D, h->ltpp, h->all_lj6, (unsigned)h->chunks_h.size(), h->stream, a));
   }
   CK(cudaGetLastError());
   if (flags & F_EM) h->cx = 1 - h->cx;
@@ -423,7 +460,7 @@ int react(rdsim_handle* h, long long step, int flags, const double* u1, const do
       else if (h->D == 3) launch_listed<3>(h, g, a);
       else launch_listed<1>(h, g, a);
     } else {
-      launch_step_kernel(h, true, a);
+      launch_react(h, a);
     }
   }
   CK(cudaGetLastError());
@@ -464,11 +501,6 @@ int check_device_error(rdsim_handle* h) {
   if (e.code == 0) return 0;
   h->moved_too_far = true;
   CK(cudaMemsetAsync(h->err, 0, sizeof(ErrDev), h->stream));
-  if (h->period_on) {
-    // a period kernel that stopped early may leave draws marked pending
-    k_clear_pending<<<nblk(h->N), 256, 0, h->stream>>>(h->meta[0], h->meta[1], h->N);
-    CK(cudaGetLastError());
-  }
   char buf[256];
   if (e.code == RDSIM_ERR_OUT_OF_BOUNDS) {
     snprintf(buf, sizeof buf,
@@ -535,7 +567,7 @@ int upload_state(rdsim_handle* h) {
 int initial_drift(rdsim_handle* h) {
   h->moved_too_far = false;
   CK(cudaMemsetAsync(h->rx_count, 0, 3 * sizeof(int), h->stream));
-  int rc = rebuild(h, 0, false, false, h->period_on);
+  int rc = rebuild(h);
   if (rc) return rc;
   rc = force(h, h->step, F_STORE_DRIFT, nullptr);
   if (rc) return rc;
@@ -549,90 +581,43 @@ bool snapshot_in(rdsim_handle* h, long long a, long long b) {
   return first <= b;
 }
 
-template <int D>
-void launch_period_d(rdsim_handle* h, const Args* A, const PeriodArgs& p) {
-  const dim3 g((unsigned)p.nchunks);
-  if (h->ltpp == 1) launch(k_period<D, 1>, g, LBLOCK, h->stream, A[0], A[1], A[2], A[3], p);
-  else if (h->ltpp == 2) launch(k_period<D, 2>, g, LBLOCK, h->stream, A[0], A[1], A[2], A[3], p);
-  else if (h->ltpp == 8) launch(k_period<D, 8>, g, LBLOCK, h->stream, A[0], A[1], A[2], A[3], p);
-  else launch(k_period<D, 4>, g, LBLOCK, h->stream, A[0], A[1], A[2], A[3], p);
-}
-
-// Steps of one list period as one launch of the period kernel (the list's
-// last rebuild ran with period_prep): the drift arguments of steps of parity
-// P read positions xh[cx ^ P] and the types after the step's reactions; the
-// reaction arguments read the types before them.  rel: a whole period in a
-// graph capture, step numbers offsets from the device counter, the first
-// step's reactions in the kernel.  Otherwise (the rest of a period after a
-// call started inside it): `nsteps` steps from step `step0`, whose reactions
-// already ran on the reaction kernels.
+// Steps of one list period as one launch of the period kernel.  rel: a whole
+// period in a graph capture, step numbers offsets from the device counter, the
+// first step's reactions in the kernel (its records from the list builder).
+// Otherwise `nsteps` steps from step `step0`, whose reactions already ran on
+// the reaction kernels.
 int period_launch(rdsim_handle* h, int kf, bool pre, bool rel = true, long long step0 = 0,
                   int nsteps = 0) {
-  const int cx0 = h->cx;
-  const int cm0 = (!rel && h->has_rx) ? h->cm ^ 1 : h->cm;
-  Args A[4];
-  for (int P = 0; P < 2; P++) {
-    h->cx = cx0 ^ P;
-    h->cm = cm0 ^ P;
-    Args r = make_args(h);
-    h->cm = h->has_rx ? (cm0 ^ P ^ 1) : cm0;
-    Args d = make_args(h);
-    d.flags = F_EM | F_CHECK_SKIN | F_PERIOD | kf;
-    r.flags = F_PERIOD | kf;
-    d.step_base = r.step_base = rel ? h->step_dev : nullptr;
-    d.step = r.step = rel ? 0 : step0;
-    d.wait_ns = r.wait_ns = h->wait_ns;
-    if (!rel) d.stamps = r.stamps = nullptr;  // the timestamps cover whole periods
-    A[P] = d;
-    A[2 + P] = r;
-  }
-  h->cx = cx0;
-  h->cm = (!rel && h->has_rx) ? cm0 ^ 1 : cm0;
+  Args a0 = make_args(h);
+  a0.flags = F_EM | F_CHECK_SKIN | F_PERIOD | kf;
+  a0.step_base = rel ? h->step_dev : nullptr;
+  a0.step = rel ? 0 : step0;
+  a0.wait_ns = h->wait_ns;
+  if (!rel) a0.stamps = nullptr;  // the timestamps cover whole periods
   PeriodArgs p;
   std::memset(&p, 0, sizeof p);
   p.nsteps = rel ? h->freq : nsteps;
-  p.nchunks = (int)h->chunks_h.size();
-  p.rx = pre ? 1 : 0;
   p.first_rx = rel ? 1 : 0;
-  if (!rel)  // progress words of a launch without the list builder before it
-    CK(cudaMemsetAsync(h->pflag, 0, sizeof(int) * (size_t)p.nchunks * PFLAG_STRIDE, h->stream));
   p.withhold = h->withhold;
   p.wait_ns = h->wait_ns;
+  // the launch leaves the state where the per-step kernels would: one flip
+  // per update, one per reaction step
+  const int cx = h->cx ^ (p.nsteps & 1);
+  const int cm = h->cm ^ ((rel ? p.nsteps : p.nsteps - 1) & 1);
+  for (int k = 0; k < 3; k++) {
+    a0.xh_out[k] = h->xh[cx][k];
+    a0.xl_out[k] = h->xl[cx][k];
+    a0.xp_out[k] = h->xp[cx][k];
+  }
+  a0.meta_out = h->meta[cm];
+  if (!rel) launch_first_records(h->D, h->stream, a0);
   {
     ProfScope ps(h, P_FORCE, 1);
-    if (h->D == 2) launch_period_d<2>(h, A, p);
-    else if (h->D == 3) launch_period_d<3>(h, A, p);
-    else launch_period_d<1>(h, A, p);
+    a0.chunks = h->pchunks_d;
+    CK(launch_period(PeriodVariant{h->D, h->ltpp, h->lpc, pre}, (unsigned)h->pchunks_h.size(),
+                     h->stream, a0, p));
   }
-  CK(cudaGetLastError());
   return 0;
-}
-
-// Resident CTAs of the period kernel on the handle's device (0 if unknown).
-template <int D>
-int period_capacity_d(int tpp) {
-  int nb = 0;
-  cudaError_t e;
-  if (tpp == 1) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_period<D, 1>, LBLOCK, 0);
-  else if (tpp == 2) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_period<D, 2>, LBLOCK, 0);
-  else if (tpp == 8) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_period<D, 8>, LBLOCK, 0);
-  else e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_period<D, 4>, LBLOCK, 0);
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  return nb;
-}
-
-int period_capacity(rdsim_handle* h) {
-  int sms = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  const int nb = h->D == 2 ? period_capacity_d<2>(h->ltpp)
-                           : (h->D == 3 ? period_capacity_d<3>(h->ltpp) : period_capacity_d<1>(h->ltpp));
-  return nb * sms;
 }
 
 // One rebuild period (steps s .. s+freq-1, each ending with the fused EM
@@ -702,8 +687,9 @@ void free_all(rdsim_handle* h) {
   F(h->sys_d); F(h->laws_d); F(h->walls_d); F(h->rx_d); F(h->tmpl_d);
   F(h->terms_d); F(h->atomterm_d); F(h->cell_count); F(h->cell_start); F(h->bsum);
   F(h->cell_of); F(h->rank_of); F(h->tmp); F(h->sid); F(h->slot_of);
-  F(h->chunks_d); F(h->nbr); F(h->ncnt); F(h->rx_list); F(h->rx_count);
-  F(h->nbmask); F(h->cand0); F(h->pflag);
+  F(h->chunks_d); F(h->pchunks_d); F(h->nbr); F(h->ncnt); F(h->rcnt); F(h->rx_list); F(h->rx_count);
+  F(h->stg_n); F(h->stg_g); F(h->codes);
+  for (int b = 0; b < 2; b++) { F(h->rec[b]); F(h->recl[b]); F(h->rech[b]); }
   for (int b = 0; b < 2; b++) {
     for (int k = 0; k < 3; k++) { F(h->xh[b][k]); F(h->xl[b][k]); F(h->xp[b][k]); }
     F(h->meta[b]); F(h->mol[b]); F(h->pid[b]);
@@ -742,6 +728,29 @@ float float_up(double v) {
 
 float guard2(double r, double unit) {
   return (float)(r * r * 2e-6 + 2.0 * r * 4.0 * unit + 1e-12);
+}
+
+// Runs of `per` consecutive particles of every system.
+std::vector<Chunk> make_chunks(const std::vector<SysDev>& systems, int per) {
+  std::vector<Chunk> out;
+  for (int si = 0; si < (int)systems.size(); si++) {
+    const SysDev& sd = systems[si];
+    for (int b = 0; b < sd.n; b += per) {
+      Chunk c;
+      std::memset(&c, 0, sizeof c);
+      c.sys = si;
+      c.beg = sd.p0 + b;
+      c.cnt = std::min(per, sd.n - b);
+      c.law0 = sd.law0;
+      c.nlaws = sd.nlaws;
+      c.wall0 = sd.wall0;
+      c.nwalls = sd.nwalls;
+      c.rx0 = sd.rx0;
+      c.nrx = sd.nrx;
+      out.push_back(c);
+    }
+  }
+  return out;
 }
 
 // Stencil half-widths (cells) that hold every pair closer than r now: such a
@@ -1074,6 +1083,7 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
         // bit 15: the pair has a single Lennard-Jones law with n = 6 (the
         // drift kernel evaluates it inline)
         const bool lj6 = v.size() == 1 && v[0].law == RDSIM_LAW_LJ && v[0].n == 6;
+        if (!lj6) h->all_lj6 = false;
         unsigned short code = (unsigned short)((first << 5) | (int)v.size() | (lj6 ? 0x8000 : 0));
         sd.ppair[a * MAXT + b] = code;
         sd.ppair[b * MAXT + a] = code;
@@ -1167,6 +1177,8 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
       const double rr = std::sqrt((double)std::max(R2, Rrx2)) + 2.0 * delta;
       const double rl = rr * (1.0 + 1e-6) + 8.0 * max_unit;
       sd.Rl2 = (float)(rl * rl);
+      const double rx = (std::sqrt((double)Rrx2) + 2.0 * delta) * (1.0 + 1e-6) + 8.0 * max_unit;
+      sd.Rrl2 = (float)(rx * rx);
       double vol = 1.0, ball = D == 1 ? 2.0 * rl : (D == 2 ? M_PI * rl * rl : 4.0 / 3.0 * M_PI * rl * rl * rl);
       for (int k = 0; k < D; k++) vol *= S.L[k];
       const double expect = std::min((double)S.n_particles, S.n_particles / vol * ball);
@@ -1332,24 +1344,7 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
   // list kernels: CTA chunks per system; list width from the expected
   // population (rows beyond it are regenerated from the cells)
   {
-    const int per = LBLOCK / h->ltpp;
-    for (int si = 0; si < (int)h->sys_h.size(); si++) {
-      const SysDev& sd = h->sys_h[si];
-      for (int b = 0; b < sd.n; b += per) {
-        Chunk c;
-        std::memset(&c, 0, sizeof c);
-        c.sys = si;
-        c.beg = sd.p0 + b;
-        c.cnt = std::min(per, sd.n - b);
-        c.law0 = sd.law0;
-        c.nlaws = sd.nlaws;
-        c.wall0 = sd.wall0;
-        c.nwalls = sd.nwalls;
-        c.rx0 = sd.rx0;
-        c.nrx = sd.nrx;
-        h->chunks_h.push_back(c);
-      }
-    }
+    h->chunks_h = make_chunks(h->sys_h, LBLOCK / h->ltpp);
     int W = (int)std::ceil(2.0 * list_expect + 16.0);
     W = std::max(16, std::min(W, 2048));
     h->npad = (h->N + 31) / 32 * 32;
@@ -1413,22 +1408,69 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
     if ((rc = dalloc(&h->chunks_d, h->chunks_h.size(), &B))) return bail(rc);
     if ((rc = dalloc(&h->nbr, (size_t)h->W * h->npad, &B))) return bail(rc);
     if ((rc = dalloc(&h->ncnt, N, &B))) return bail(rc);
+    if ((rc = dalloc(&h->rcnt, N, &B))) return bail(rc);
     if ((rc = dalloc(&h->rx_list, 3 * (size_t)h->npad, &B))) return bail(rc);
     if ((rc = dalloc(&h->rx_count, 3, &B))) return bail(rc);
     if (cudaMemsetAsync(h->rx_count, 0, 3 * sizeof(int), h->stream) != cudaSuccess)
       return bail(fail(RDSIM_ERR_CUDA, "memset"));
   }
   h->graphs = opt.use_graphs >= 0;
-  // period kernel: float32 forces, every chunk resident at once (its CTAs
-  // wait for each other) and within the neighbour-chunk bitmap
   if (opt.sync_wait_ms > 0) h->wait_ns = (long long)opt.sync_wait_ms * 1000000LL;
+  if (!h->f64 && opt.period_kernel >= 0) {
+    int sms = 0;
+    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, h->device) != cudaSuccess) {
+      cudaGetLastError();
+      sms = 0;
+    }
+    // lanes per chain: as many as keep the chunks below LPC_CHUNKS per SM
+    if (h->ltpp == 2 && D < 3)
+      for (int lpc = 4; lpc > 1 && h->lpc == 1; lpc /= 2)
+        if ((long long)make_chunks(h->sys_h, LBLOCK / 2 / lpc).size() <= (long long)sms * LPC_CHUNKS)
+          h->lpc = lpc;
+    const int per = LBLOCK / h->ltpp / h->lpc;
+    const int nch = (int)make_chunks(h->sys_h, per).size();
+    // neighbour staging: a chunk of P particles touches about its own run and
+    // three cells more in every row of cells around it; a third more for
+    // denser places (a chunk that touches more gathers from memory)
+    double want = 64;
+    int largest = 1;
+    for (const SysDev& sd : h->sys_h) {
+      double cells = 1;
+      for (int k = 0; k < D; k++) cells *= sd.nc[k];
+      const double rows = D == 3 ? 9 : (D == 2 ? 3 : 1);
+      want = std::max(want, rows * (per + 3.0 * sd.n / cells) * 1.3 + 64);
+      largest = std::max(largest, sd.n);
+      h->rows = std::max(h->rows, sd.ntypes * sd.ntypes);
+    }
+    auto slots = [](double v) { return ((int)v + 63) / 64 * 64; };
+    h->stg_max = std::min(slots(std::min(want, (double)largest)), STG_LIMIT);
+    // slot codes for half again the expected row and some (shared memory taken
+    // here is taken from the SM's L1)
+    const int row = std::min(h->W, (int)(1.5 * list_expect) + 12), lanes = 2 * h->ltpp * h->lpc;
+    h->kw = std::min((row + lanes - 1) / lanes, KW_LIMIT);
+    // every chunk resident at once (its CTAs wait for each other), with less
+    // room for staging if need be
+    const PeriodVariant v{D, h->ltpp, h->lpc, h->has_rx};
+    for (int m = h->stg_max; m >= 64 && m >= h->stg_max / 4 && !h->period_on; m = m / 128 * 64)
+      if ((long long)period_blocks_per_sm(v, m, h->kw, h->rows) * sms >= nch) {
+        h->period_on = true;
+        h->stg_max = m;
+      }
+    if (!h->period_on) h->lpc = 1;
+  }
+  h->pchunks_h = make_chunks(h->sys_h, LBLOCK / h->ltpp / h->lpc);
   {
-    const int nch = (int)h->chunks_h.size();
-    if (opt.period_kernel >= 0 && !h->f64 && nch <= PMAX_CHUNKS && nch <= period_capacity(h)) {
-      if ((rc = dalloc(&h->nbmask, (size_t)nch * PMASK_WORDS, &B))) return bail(rc);
-      if ((rc = dalloc(&h->cand0, (size_t)nch * CAND_WORDS, &B))) return bail(rc);
-      if ((rc = dalloc(&h->pflag, (size_t)nch * PFLAG_STRIDE, &B))) return bail(rc);
-      h->period_on = true;
+    const size_t nch = h->pchunks_h.size();
+    if ((rc = dalloc(&h->pchunks_d, nch, &B))) return bail(rc);
+    if (h->period_on) {
+      if ((rc = dalloc(&h->stg_n, nch, &B))) return bail(rc);
+      if ((rc = dalloc(&h->stg_g, nch * h->stg_max, &B))) return bail(rc);
+      if ((rc = dalloc(&h->codes, nch * h->kw * LBLOCK, &B))) return bail(rc);
+      for (int b = 0; b < 2; b++) {
+        if ((rc = dalloc(&h->rec[b], N, &B))) return bail(rc);
+        if ((rc = dalloc(&h->recl[b], N, &B))) return bail(rc);
+        if ((rc = dalloc(&h->rech[b], N, &B))) return bail(rc);
+      }
     }
   }
   if ((rc = dalloc(&h->cl_d, (size_t)3 * h->nsys, &B))) return bail(rc);
@@ -1442,6 +1484,8 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
     for (int k = 0; k < D; k++) cl[3 * s + k] = h->hs[s].cl_ref[k];
   if ((rc = up(h->sys_d, h->sys_h.data(), sizeof(SysDev) * h->sys_h.size()))) return bail(rc);
   if ((rc = up(h->chunks_d, h->chunks_h.data(), sizeof(Chunk) * h->chunks_h.size())))
+    return bail(rc);
+  if ((rc = up(h->pchunks_d, h->pchunks_h.data(), sizeof(Chunk) * h->pchunks_h.size())))
     return bail(rc);
   if ((rc = up(h->laws_d, laws.data(), sizeof(PairLaw) * laws.size()))) return bail(rc);
   if ((rc = up(h->walls_d, walls.data(), sizeof(WallLaw) * walls.size()))) return bail(rc);
@@ -1541,26 +1585,8 @@ int rdsim_step(rdsim_handle* h, int32_t n_steps, int32_t flags, const double* xi
       flagged = false;
       continue;
     }
-    // a call that starts inside a list period: the step's reactions on the
-    // reaction kernels, then the rest of the period in one period-kernel
-    // launch (not when a trajectory frame or the call's last step falls in it)
-    const long long e = (s / h->freq + 1) * h->freq - 1;
-    const int m = (int)(e - s + 1);
-    if (graphable && h->period_on && (pre || !h->has_rx) && s % h->freq != 0 && left > m &&
-        !snapshot_in(h, s, e)) {
-      if (h->has_rx &&
-          (rc = react(h, s, kf, nullptr, nullptr, false, flagged)))
-        return rc;
-      if ((rc = period_launch(h, kf, pre, false, s, m))) return rc;
-      h->cx ^= m & 1;
-      if (h->has_rx) h->cm ^= (m - 1) & 1;
-      h->step = e;
-      q += m;
-      flagged = false;
-      continue;
-    }
     if (s % h->freq == 0) {
-      if ((rc = rebuild(h, s, pre, false, h->period_on))) return rc;
+      if ((rc = rebuild(h, s, pre))) return rc;
       flagged = pre;  // the builder listed this step's candidates
     }
     if (h->has_rx) {
@@ -1571,6 +1597,22 @@ int rdsim_step(rdsim_handle* h, int32_t n_steps, int32_t flags, const double* xi
     if (h->traj_frames > 0 && s % h->traj_stride == 0) {
       long long m = (s / h->traj_stride - 1) % h->traj_frames;
       if ((rc = snapshot(h, h->traj_x + (size_t)m * N * D, h->traj_t + (size_t)m * N))) return rc;
+    }
+    // the drifts from here up to the next rebuild, the next trajectory frame
+    // or the call's last step (it stores the drift) in one launch
+    if (graphable && h->period_on && (pre || !h->has_rx)) {
+      long long e = std::min((s / h->freq + 1) * h->freq - 1, s + left - 2);
+      if (h->traj_frames > 0) e = std::min(e, (s / h->traj_stride + 1) * h->traj_stride - 1);
+      const int m = (int)(e - s + 1);
+      if (m >= 2) {
+        if ((rc = period_launch(h, kf, pre, false, s, m))) return rc;
+        h->cx ^= m & 1;
+        if (h->has_rx) h->cm ^= (m - 1) & 1;
+        h->step = e;
+        q += m;
+        flagged = false;
+        continue;
+      }
     }
     const bool last = q == n_steps - 1;
     const double* xn = (dxi && !last) ? dxi + (size_t)(q + 1) * N * D : nullptr;
@@ -1883,7 +1925,7 @@ int rdsim_set_profiling(rdsim_handle* h, int32_t enable) {
     h->stamp_on = stamp;
   }
   if (stamp && !h->stamps) {
-    const size_t nctas = std::max<size_t>(1, h->chunks_h.size());
+    const size_t nctas = stamp_ctas(h);
     const size_t ring = std::min<size_t>(32768, std::max<size_t>(64, (512u << 20) / (16 * nctas)));
     int64_t dummy = 0;
     int rc;
@@ -1903,7 +1945,7 @@ int rdsim_get_profile(rdsim_handle* h, rdsim_profile* p) {
   p->drift_span_ms = 0.0;
   p->drift_spans = 0;
   if (h->stamps) {
-    const int nctas = (int)std::max<size_t>(1, h->chunks_h.size());
+    const int nctas = (int)stamp_ctas(h);
     CK(cudaMemsetAsync(h->stamp_sum, 0, 2 * sizeof(unsigned long long), h->stream));
     k_stamp_spans<<<h->stamp_ring, 256, 0, h->stream>>>(h->stamps, h->stamp_ring, nctas,
                                                         h->stamp_sum, h->stamp_sum + 1);

@@ -369,7 +369,7 @@ __global__ void __launch_bounds__(LBLOCK) k_force_d(Args a) {
     if (a.flags & F_RX_NEXT) {
       a.meta_out[ib] = mb;
       rec = make_int4(ib, (int)mb, a.ncnt[ib], pid);
-      listed = rx_may_react<D>(s, (int)(mb & 0xff), rec.z, pid, eff_em_step(a), &w0);
+      listed = rx_may_react<D>(s, (int)(mb & 0xff), a.rcnt[ib], pid, eff_em_step(a), &w0);
     }
   }
   if (a.flags & F_RX_NEXT) {

@@ -34,16 +34,19 @@ __device__ inline void record_error(ErrDev* e, int code, long long particle, int
 __device__ inline void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ inline void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// The step the CTA of a period kernel is at (F_PERIOD): its drift of step n
-// performs the update of step n + 1.
+// The step of the reactions and pair drifts that the CTA of a period kernel is
+// at (F_PERIOD), and its number within the launch.  Written before the barrier
+// that starts the step; the per-particle tails may still run while the next
+// one is written, so they take their step as an argument.
 static __shared__ long long period_step;
+static __shared__ int period_n;
+static __shared__ int period_failed;  // a wait of this CTA ran out
 
 __device__ inline long long eff_step(const Args& a) {
   if (a.flags & F_PERIOD) return period_step;
   return a.step_base ? *a.step_base + a.step : a.step;
 }
 __device__ inline long long eff_em_step(const Args& a) {
-  if (a.flags & F_PERIOD) return period_step + 1;
   return a.step_base ? *a.step_base + a.em_step : a.em_step;
 }
 
@@ -139,37 +142,137 @@ __host__ __device__ inline bool fixed_from_double(double x, double L, bool perio
   return true;
 }
 
-// Words that other CTAs of a running period kernel write (positions and
-// type words of other particles) are read there with strong relaxed loads
-// (coherent at GPU scope, not cached in L1), so that no acquire fence has
-// to invalidate the SM's L1, which holds the list rows and the CTA's own
-// words.  Elsewhere plain loads.  RD_PERIOD_CG: 0 plain loads after an
-// acquire fence, 1 ld.global.cg, 2 ld.relaxed.gpu.
-#ifndef RD_PERIOD_CG
-#define RD_PERIOD_CG 2
-#endif
-__device__ inline uint32_t ldw(const Args& a, const uint32_t* p) {
-#if RD_PERIOD_CG == 1
-  if (a.flags & F_PERIOD) return __ldcg(p);
-#elif RD_PERIOD_CG == 2
-  if (a.flags & F_PERIOD) {
-    uint32_t v;
-    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
-    return v;
+// 128-bit accesses at GPU scope, single-copy atomic (a record and its tag are
+// read together) and not cached in L1.
+__device__ inline uint4 ld_rec(const uint4* p) {
+  unsigned __int128 v;
+  asm volatile("ld.relaxed.gpu.global.b128 %0, [%1];" : "=q"(v) : "l"(p) : "memory");
+  return make_uint4((uint32_t)v, (uint32_t)(v >> 32), (uint32_t)(v >> 64), (uint32_t)(v >> 96));
+}
+__device__ inline void st_rec(uint4* p, uint32_t x, uint32_t y, uint32_t z, uint32_t w) {
+  const unsigned __int128 v = (unsigned __int128)x | ((unsigned __int128)y << 32) |
+                              ((unsigned __int128)z << 64) | ((unsigned __int128)w << 96);
+  asm volatile("st.relaxed.gpu.global.b128 [%0], %1;" ::"l"(p), "q"(v) : "memory");
+}
+
+// A wait of a period kernel that began at t0 ends: a.wait_ns have passed, or
+// some CTA has recorded an error.
+__device__ inline bool wait_over(const Args& a, unsigned long long t0) {
+  return *(volatile int*)&a.err->code != 0 || (long long)(global_timer() - t0) > a.wait_ns;
+}
+
+// Marks the CTA failed after such a wait (it returns at the next step's
+// barrier) and records RDSIM_ERR_SYNC if no error is recorded yet.
+__device__ inline void wait_failed(const Args& a, int n) {
+  record_error(a.err, RDSIM_ERR_SYNC, (long long)blockIdx.x, -1, (double)n, eff_step(a));
+  period_failed = 1;
+}
+
+// Polls a record until it is of step n (and, with `pend`, its draw is
+// resolved); after a failed wait the last value is used.  Out of line, for the
+// rare readers; the staging loop polls inline.
+static __device__ __noinline__ uint4 rec_wait(const Args& a, const uint4* p, int shift, int n,
+                                              bool pend) {
+  const unsigned long long t0 = global_timer();
+  for (int k = 1;; k++) {
+    const uint4 v = ld_rec(p);
+    if (rec_ready(v.w, shift, n) && !(pend && (v.w & REC_PENDING))) return v;
+    if ((k & 31) == 0 && wait_over(a, t0)) {
+      wait_failed(a, n);
+      return v;
+    }
   }
-#endif
-  return *p;
+}
+
+// The type word of a record whose draw is pending, once resolved (inline: the
+// pair loop it is in holds no call).
+__device__ inline uint32_t pending_word(const Args& a, const uint32_t* p) {
+  unsigned long long t0 = 0ull;
+  uint32_t w;
+  for (int k = 1;; k++) {
+    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(w) : "l"(p) : "memory");
+    if (!(w & REC_PENDING)) return w;
+    if ((k & 63) == 0) {
+      if (k == 64) {
+        t0 = global_timer();
+      } else if (wait_over(a, t0)) {
+        wait_failed(a, period_n);
+        return w;
+      }
+    }
+  }
+}
+
+__device__ inline uint4 get_rec(const Args& a, const uint4* p, int shift, int n) {
+  const uint4 v = ld_rec(p);
+  return rec_ready(v.w, shift, n) ? v : rec_wait(a, p, shift, n, false);
+}
+
+struct Words {
+  uint32_t h[3], l[3];
+};
+
+// High and low words of particle j: in a period kernel from its records of
+// step n of the launch (other CTAs write them), else from the arrays.
+template <int D>
+__device__ inline void load_full(const Args& a, int j, int n, uint32_t* h, uint32_t* l) {
+  if (a.flags & F_PERIOD) {
+    const uint4 vl = get_rec(a, a.recl[n & 1] + j, 0, n);
+    const uint4 vh = get_rec(a, a.rech[n & 1] + j, 0, n);
+    const uint32_t hh[3] = {vh.x, vh.y, vh.z}, ll[3] = {vl.x, vl.y, vl.z};
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+      h[k] = hh[k];
+      l[k] = ll[k];
+    }
+  } else {
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+      h[k] = a.xh[k][j];
+      l[k] = a.xl[k][j];
+    }
+  }
+}
+
+// The loads of load_full (j < 0: none) without the wait: the tags still have to
+// be looked at in a period kernel.
+struct RawWords {
+  uint4 h, l;
+};
+
+template <int D>
+__device__ inline RawWords load_raw(const Args& a, int j, int n) {
+  RawWords r;
+  r.h = r.l = make_uint4(0u, 0u, 0u, (uint32_t)n);
+  if (j < 0) return r;
+  if (a.flags & F_PERIOD) {
+    r.h = ld_rec(a.rech[n & 1] + j);
+    r.l = ld_rec(a.recl[n & 1] + j);
+  } else {
+    r.h.x = a.xh[0][j];
+    r.l.x = a.xl[0][j];
+    if (D > 1) r.h.y = a.xh[1][j];
+    if (D > 1) r.l.y = a.xl[1][j];
+    if (D > 2) r.h.z = a.xh[2][j];
+    if (D > 2) r.l.z = a.xl[2][j];
+  }
+  return r;
 }
 
 // Distance of two particles exactly as pyrdsim.pyx:1619-1633 computes it
-// (float64, C round() minimum image, pow(v, 2) summed in dimension order).
+// (float64, C round() minimum image, pow(v, 2) summed in dimension order).  Out
+// of line: rare in the drift kernels, whose registers it would take.
 template <int D>
-__device__ double exact_dist(const SysDev& s, const Args& a, int gi, int gj) {
+__device__ __noinline__ double exact_dist(const SysDev& s, const Args& a, int gi, int gj) {
   double d2 = 0.0;
+  uint32_t hi[3], li[3], hj[3], lj[3];
+  const int n = (a.flags & F_PERIOD) ? period_n : 0;
+  load_full<D>(a, gi, n, hi, li);
+  load_full<D>(a, gj, n, hj, lj);
 #pragma unroll
   for (int k = 0; k < D; k++) {
-    double xi = fixed_to_double(s, k, ldw(a, a.xh[k] + gi), ldw(a, a.xl[k] + gi));
-    double xj = fixed_to_double(s, k, ldw(a, a.xh[k] + gj), ldw(a, a.xl[k] + gj));
+    double xi = fixed_to_double(s, k, hi[k], li[k]);
+    double xj = fixed_to_double(s, k, hj[k], lj[k]);
     double v = __dsub_rn(xj, xi);
     // minimum image; round(v / L) is 0 whenever |v| < 0.49 L, which holds for
     // every pair of adjacent cells except in boxes of three cells or fewer
@@ -217,10 +320,14 @@ __device__ inline float u128_to_float(unsigned __int128 v) {
 // Displacement x_j - x_i along dimension k from the full fixed-point words
 // (minimum image in periodic dimensions), rounded once to float32 before the
 // unit is applied: bonded terms, whose partners may lie anywhere in the box.
-__device__ inline float disp_full(const SysDev& s, const Args& a, int k, int gi, int gj) {
-  const unsigned long long Xi = ((unsigned long long)ldw(a, a.xh[k] + gi) << 32) | ldw(a, a.xl[k] + gi);
-  const unsigned long long Xj = ((unsigned long long)ldw(a, a.xh[k] + gj) << 32) | ldw(a, a.xl[k] + gj);
-  return __ll2float_rn((long long)(Xj - Xi)) * s.unitf[k];
+__device__ inline long long full_diff(uint32_t hi, uint32_t li, uint32_t hj, uint32_t lj) {
+  const unsigned long long Xi = ((unsigned long long)hi << 32) | li;
+  const unsigned long long Xj = ((unsigned long long)hj << 32) | lj;
+  return (long long)(Xj - Xi);
+}
+__device__ inline float disp_full(const SysDev& s, int k, uint32_t hi, uint32_t li, uint32_t hj,
+                                  uint32_t lj) {
+  return __ll2float_rn(full_diff(hi, li, hj, lj)) * s.unitf[k];
 }
 
 // f / r of one pair law at squared distance r2 (float32); inv_r2 = recip(r2).
@@ -260,10 +367,10 @@ __device__ inline float eval_pair(const PairLaw& L, float r2, float inv_r2) {
 
 // f / r summed over the laws of one type pair (pp = first << 5 | count) at
 // squared distance r2; near a cutoff the float64 distance decides
-// (pyrdsim.pyx:1988-2030).  gi, gj: sorted indices of the pair.
-template <int D>
+// (pyrdsim.pyx:1988-2030).  gi, gj(): sorted indices of the pair.
+template <int D, class J>
 __device__ inline float pair_force(const SysDev& s, const PairLaw* laws, const Args& a, int gi,
-                                   int gj, unsigned int pp, float r2) {
+                                   J&& gj, unsigned int pp, float r2) {
   const int nl = pp & 31, l0 = (pp >> 5) & 0x3ff;
   const float inv_r2 = recip(r2);
   float fr = 0.f;
@@ -272,13 +379,13 @@ __device__ inline float pair_force(const SysDev& s, const PairLaw* laws, const A
     const PairLaw& L = laws[l];
     if (r2 > L.rc2_hi) continue;
     if (r2 >= L.rc2_lo) {
-      if (dexact < 0) dexact = exact_dist<D>(s, a, gi, gj);
+      if (dexact < 0) dexact = exact_dist<D>(s, a, gi, gj());
       if (dexact > L.rc) continue;
     }
     if (L.law == RDSIM_LAW_PIECEWISE_LINEAR) {
       if (r2 < L.in2_lo) continue;
       if (r2 <= L.in2_hi) {
-        if (dexact < 0) dexact = exact_dist<D>(s, a, gi, gj);
+        if (dexact < 0) dexact = exact_dist<D>(s, a, gi, gj());
         if (dexact < L.rin) continue;
       }
     }
@@ -310,6 +417,25 @@ struct WordLoad {
     }
   }
 };
+
+// pair_force where no law's cutoff is within its guard band of r2; `close` is
+// set (and the sum not valid) where one is.
+__device__ inline float laws_over_r(const PairLaw* laws, unsigned int pp, float r2, bool& close) {
+  const int nl = pp & 31, l0 = (pp >> 5) & 0x3ff;
+  const float inv_r2 = recip(r2);
+  float fr = 0.f;
+  for (int l = l0; l < l0 + nl; l++) {
+    const PairLaw& L = laws[l];
+    if (r2 > L.rc2_hi) continue;
+    close = close || r2 >= L.rc2_lo;
+    if (L.law == RDSIM_LAW_PIECEWISE_LINEAR) {
+      if (r2 < L.in2_lo) continue;
+      close = close || r2 <= L.in2_hi;
+    }
+    fr += eval_pair(L, r2, inv_r2);
+  }
+  return fr;
+}
 
 __device__ inline long long delta_fixed(float d, float inv_unit_hi, bool* bad) {
   float v = d * inv_unit_hi;
@@ -381,14 +507,14 @@ __device__ inline void gaussians(const U4& w, float* xi) {
   }
 }
 
-// Advances coordinate k of particle gi by d fixed units (|d| < 2^62) and
-// applies the boundary condition (pyrdsim.pyx:2253-2292): an exact wrap in
-// periodic dimensions, a reflection at 0 and L in reflecting ones, where X
-// lies in [-S, S] (S = 2^62), so X + d and the reflections stay within
-// int64.  Writes the high, low and pair words.
-// X: the coordinate's current fixed-point value.
-__device__ inline void advance_x(const SysDev& s, const Args& a, int gi, int pid, int k,
-                                 long long d, long long em_step, unsigned long long X) {
+// Coordinate k (fixed-point value X) of caller index pid advanced by d fixed
+// units (|d| < 2^62), with the boundary condition (pyrdsim.pyx:2253-2292): an
+// exact wrap in periodic dimensions, a reflection at 0 and L in reflecting
+// ones, where X lies in [-S, S] (S = 2^62), so X + d and the reflections stay
+// within int64.
+__device__ inline unsigned long long advance_x(const SysDev& s, const Args& a, int pid, int k,
+                                               long long d, long long em_step,
+                                               unsigned long long X) {
   if ((s.periodic >> k) & 1) {
     X += (unsigned long long)d;
   } else {
@@ -407,6 +533,12 @@ __device__ inline void advance_x(const SysDev& s, const Args& a, int gi, int pid
     }
     X = (unsigned long long)(long long)Xs;
   }
+  return X;
+}
+
+// The high, low and pair words of coordinate k of particle gi.
+__device__ inline void store_words(const SysDev& s, const Args& a, int gi, int k,
+                                   unsigned long long X) {
   a.xh_out[k][gi] = (uint32_t)(X >> 32);
   a.xl_out[k][gi] = (uint32_t)X;
   a.xp_out[k][gi] = (uint32_t)(X >> s.ps[k]);
@@ -414,8 +546,9 @@ __device__ inline void advance_x(const SysDev& s, const Args& a, int gi, int pid
 
 __device__ inline void advance(const SysDev& s, const Args& a, int gi, int pid, int k,
                                long long d, long long em_step) {
-  advance_x(s, a, gi, pid, k, d, em_step,
-            ((unsigned long long)a.xh[k][gi] << 32) | a.xl[k][gi]);
+  store_words(s, a, gi, k,
+              advance_x(s, a, pid, k, d, em_step,
+                        ((unsigned long long)a.xh[k][gi] << 32) | a.xl[k][gi]));
 }
 
 // The words of one particle that its per-particle tail reads, loaded by the
@@ -428,10 +561,11 @@ struct TailIn {
 
 // Euler-Maruyama update + boundary conditions of one particle in fixed point
 // (pyrdsim.pyx:2240-2292): x += dt D a + sqrt(2 dt D) xi, then reflect or wrap.
+// X receives the new coordinates.
 template <int D>
-__device__ inline void em_update_in(const SysDev& s, const Args& a, int gi, int pid, int type,
+__device__ inline void em_update_in(const SysDev& s, const Args& a, int pid, int type,
                                     const float* acc, long long em_step, int flags,
-                                    const U4* w0, const TailIn& t) {
+                                    const U4* w0, const TailIn& t, unsigned long long* X) {
   float xi[3] = {0.f, 0.f, 0.f};
   if (!(flags & F_NO_NOISE)) {
     if (t.xi) {
@@ -451,7 +585,7 @@ __device__ inline void em_update_in(const SysDev& s, const Args& a, int gi, int 
     float dl = fp * acc[k] + np * xi[k];
     long long d = delta_fixed(dl, s.inv_unit_hi[k], &bad);
     if (bad) record_error(a.err, RDSIM_ERR_NONFINITE, pid, k, (double)dl, em_step);
-    advance_x(s, a, gi, pid, k, d, em_step, ((unsigned long long)t.xh[k] << 32) | t.xl[k]);
+    X[k] = advance_x(s, a, pid, k, d, em_step, ((unsigned long long)t.xh[k] << 32) | t.xl[k]);
   }
 }
 
@@ -472,28 +606,57 @@ template <int D>
 __device__ inline void em_update(const SysDev& s, const Args& a, int gi, int pid, int type,
                                  const float* acc, long long em_step, int flags,
                                  const U4* w0 = nullptr) {
-  em_update_in<D>(s, a, gi, pid, type, acc, em_step, flags, w0, tail_load<D>(a, gi));
+  unsigned long long X[3];
+  em_update_in<D>(s, a, pid, type, acc, em_step, flags, w0, tail_load<D>(a, gi), X);
+#pragma unroll
+  for (int k = 0; k < D; k++) store_words(s, a, gi, k, X[k]);
 }
 
 // ---------------------------------------------------------------------------
 // Bonded terms of one particle (pyrdsim.pyx:2037-2066), gathered: the
 // particle evaluates every bond and angle it takes part in, reading its
-// partners' positions through slot_of (caller index -> sorted slot).
+// partners' positions through slot_of (caller index -> sorted slot).  own: its
+// words; n: a period kernel's step within the launch.  Returns acc0 plus the
+// terms.  Out of line and by value: its registers stay out of the drift
+// kernels' budget, and nothing they keep in registers has its address taken.
 template <int D>
-__device__ inline void bonded_terms(const SysDev& s, const Args& a, int gi, int pid, uint32_t mi,
-                                    float* acc) {
+__device__ __noinline__ float3 bonded_terms(const SysDev& s, const Args& a, Words own, int pid,
+                                            uint32_t mi, int n, float3 acc0) {
+  float acc[3] = {acc0.x, acc0.y, acc0.z};
+  const uint32_t *xh = own.h, *xl = own.l;
   const int tm = mi >> 24;
-  if (tm == 0xff) return;
   const TmplDev& T = a.tmpl[tm];
   const int loc = (mi >> 16) & 0xff;
   const int mbase = pid - loc;
   float xo[3];
-  for (int e = a.atomterm[T.atom0 + loc]; e < a.atomterm[T.atom0 + loc + 1]; e++) {
+  const int eb = a.atomterm[T.atom0 + loc], ee = a.atomterm[T.atom0 + loc + 1];
+  // the bond partners' words are loaded three terms ahead (one round trip for a
+  // particle of up to three bonds instead of one per bond)
+  auto partner = [&](int e) {
+    if (e >= ee) return -1;
+    const int code = a.atomterm[e];
+    const TermDev& tr = a.terms[code >> 2];
+    return tr.kind == RDSIM_TERM_BOND ? a.slot_of[mbase + ((code & 3) == 0 ? tr.j : tr.i)] : -1;
+  };
+  int j0 = partner(eb), j1 = partner(eb + 1), j2 = partner(eb + 2);
+  RawWords r0 = load_raw<D>(a, j0, n), r1 = load_raw<D>(a, j1, n), r2 = load_raw<D>(a, j2, n);
+#pragma unroll 1
+  for (int e = eb; e < ee; e++) {
     const int code = a.atomterm[e];
     const TermDev& tr = a.terms[code >> 2];
     const int role = code & 3;
+    const int other = j0;
+    RawWords cur = r0;
+    r0 = r1;
+    j0 = j1;
+    r1 = r2;
+    j1 = j2;
+    j2 = partner(e + 3);
+    r2 = load_raw<D>(a, j2, n);
     if (tr.kind == RDSIM_TERM_BOND) {
-      const int other = a.slot_of[mbase + (role == 0 ? tr.j : tr.i)];
+      if (!rec_ready(cur.l.w, 0, n)) cur.l = rec_wait(a, a.recl[n & 1] + other, 0, n, false);
+      if (!rec_ready(cur.h.w, 0, n)) cur.h = rec_wait(a, a.rech[n & 1] + other, 0, n, false);
+      const uint32_t oh[3] = {cur.h.x, cur.h.y, cur.h.z}, ol[3] = {cur.l.x, cur.l.y, cur.l.z};
       // f = k (d - r0) / d (pyrdsim.pyx:2037-2047).  A stiff bond near rest
       // cancels in d - r0: where every dimension has the same fixed unit,
       // d^2 - r0^2 is formed exactly in 128-bit integers (units unit^2) and
@@ -504,10 +667,7 @@ __device__ inline void bonded_terms(const SysDev& s, const Args& a, int gi, int 
         unsigned __int128 S2 = 0;
 #pragma unroll
         for (int k = 0; k < D; k++) {
-          const unsigned long long Xi = ((unsigned long long)a.xh[k][gi] << 32) | a.xl[k][gi];
-          const unsigned long long Xj =
-              ((unsigned long long)ldw(a, a.xh[k] + other) << 32) | ldw(a, a.xl[k] + other);
-          const long long dd = (long long)(Xj - Xi);
+          const long long dd = full_diff(xh[k], xl[k], oh[k], ol[k]);
           const unsigned long long m = dd < 0 ? 0ull - (unsigned long long)dd : (unsigned long long)dd;
           S2 += (unsigned __int128)m * m;
           xo[k] = __ll2float_rn(dd) * s.unitf[k];
@@ -522,7 +682,7 @@ __device__ inline void bonded_terms(const SysDev& s, const Args& a, int gi, int 
         float d2 = 0.f;
 #pragma unroll
         for (int k = 0; k < D; k++) {
-          xo[k] = disp_full(s, a, k, gi, other);
+          xo[k] = disp_full(s, k, xh[k], xl[k], oh[k], ol[k]);
           d2 = fmaf(xo[k], xo[k], d2);
         }
         const float d = sqrtf(d2);
@@ -534,10 +694,14 @@ __device__ inline void bonded_terms(const SysDev& s, const Args& a, int gi, int 
       const int s1 = a.slot_of[mbase + tr.i], s2 = a.slot_of[mbase + tr.j],
                 s3 = a.slot_of[mbase + tr.k];
       float v1[3], v2[3], n1 = 0.f, n2 = 0.f;
+      uint32_t h1[3], l1[3], h2[3], l2[3], h3[3], l3[3];
+      load_full<D>(a, s1, n, h1, l1);
+      load_full<D>(a, s2, n, h2, l2);
+      load_full<D>(a, s3, n, h3, l3);
 #pragma unroll
       for (int k = 0; k < D; k++) {
-        v1[k] = disp_full(s, a, k, s2, s1);
-        v2[k] = disp_full(s, a, k, s2, s3);
+        v1[k] = disp_full(s, k, h2[k], l2[k], h1[k], l1[k]);
+        v2[k] = disp_full(s, k, h2[k], l2[k], h3[k], l3[k]);
         n1 = fmaf(v1[k], v1[k], n1);
         n2 = fmaf(v2[k], v2[k], n2);
       }
@@ -580,25 +744,21 @@ __device__ inline void bonded_terms(const SysDev& s, const Args& a, int gi, int 
       }
     }
   }
+  return make_float3(acc[0], acc[1], acc[2]);
 }
 
-// Per-particle tail of the drift kernels, on one thread per particle: walls
-// (pyrdsim.pyx:1979-1986), bonded terms, drift store, finiteness and skin
-// checks, and the fused Euler-Maruyama update.  acc holds the pair drift.
+// The walls' drift on one particle of type ti with words xh, xl
+// (pyrdsim.pyx:1979-1986), added to acc.
 template <int D>
-__device__ inline void force_tail_in(const SysDev& s, const WallLaw* walls, const Args& a, int gi,
-                                     int pid, const TailIn& t, uint32_t mi, float* acc,
-                                     const U4* w0 = nullptr) {
-  const uint32_t* xo_h = t.xh;
-  const int ti = mi & 0xff;
-  // walls (pyrdsim.pyx:1979-1986)
+__device__ inline void wall_terms(const SysDev& s, const WallLaw* walls, const uint32_t* xh,
+                                  const uint32_t* xl, int ti, float* acc) {
   for (int w = 0; w < s.nwalls; w++) {
     const WallLaw& W = walls[w];
     if (W.type != ti) continue;
-    uint32_t h = xo_h[0];
+    uint32_t h = xh[0];
 #pragma unroll
     for (int k = 1; k < D; k++)
-      if (k == W.dim) h = xo_h[k];
+      if (k == W.dim) h = xh[k];
     float f;
     if (W.law == RDSIM_LAW_WALL) {
       const float z = (float)((long long)h - W.hr0) * s.unit_hi[W.dim] * W.c2;
@@ -612,10 +772,10 @@ __device__ inline void force_tail_in(const SysDev& s, const WallLaw* walls, cons
       if (yh > W.rc_hi) continue;
       // the full coordinate; reflecting ones are signed (an initial
       // position may lie below 0)
-      uint32_t l = t.xl[0];
+      uint32_t l = xl[0];
 #pragma unroll
       for (int k = 1; k < D; k++)
-        if (k == W.dim) l = t.xl[k];
+        if (k == W.dim) l = xl[k];
       const unsigned long long X = ((unsigned long long)h << 32) | l;
       const float y = (((s.periodic >> W.dim) & 1) ? __ull2float_rn(X)
                                                     : __ll2float_rn((long long)X)) *
@@ -632,14 +792,29 @@ __device__ inline void force_tail_in(const SysDev& s, const WallLaw* walls, cons
     for (int k = 0; k < D; k++)
       if (k == W.dim) acc[k] += -f;
   }
-  bonded_terms<D>(s, a, gi, pid, mi, acc);
-  if (a.flags & F_STORE_DRIFT) {
-#pragma unroll
-    for (int k = 0; k < D; k++) a.drift[k][gi] = acc[k];
+}
+
+// A particle's bonded terms, if it has any, added to acc.
+template <int D>
+__device__ inline void add_bonded(const SysDev& s, const Args& a, const uint32_t* xh,
+                                  const uint32_t* xl, int pid, uint32_t mi, int n, float* acc) {
+  if ((mi >> 24) != 0xff) {
+    const Words own = {{xh[0], xh[1], xh[2]}, {xl[0], xl[1], xl[2]}};
+    const float3 b = bonded_terms<D>(
+        s, a, own, pid, mi, n, make_float3(acc[0], D > 1 ? acc[1] : 0.f, D > 2 ? acc[2] : 0.f));
+    acc[0] = b.x;
+    if (D > 1) acc[1] = b.y;
+    if (D > 2) acc[2] = b.z;
   }
+}
+
+// Finiteness and displacement checks of one particle's drift at step `step`.
+template <int D>
+__device__ inline void tail_checks(const SysDev& s, const Args& a, int pid, const uint32_t* xh,
+                                   const uint32_t* xr, const float* acc, long long step) {
 #pragma unroll
   for (int k = 0; k < D; k++)
-    if (!isfinite(acc[k])) record_error(a.err, RDSIM_ERR_NONFINITE, pid, k, (double)acc[k], eff_step(a));
+    if (!isfinite(acc[k])) record_error(a.err, RDSIM_ERR_NONFINITE, pid, k, (double)acc[k], step);
   if (a.flags & F_CHECK_SKIN) {
     // displacement since the last rebuild: keeps every pair within range in
     // adjacent cells, in the Verlet list and within rs of each other at that
@@ -647,16 +822,18 @@ __device__ inline void force_tail_in(const SysDev& s, const WallLaw* walls, cons
     float rel2 = 0.f;
 #pragma unroll
     for (int k = 0; k < D; k++) {
-      const float rel = (float)(int)(xo_h[k] - t.xr[k]) * s.unit_hi[k];
+      const float rel = (float)(int)(xh[k] - xr[k]) * s.unit_hi[k];
       rel2 += rel * rel;
     }
     if (rel2 > s.delta * s.delta)
-      record_error(a.err, RDSIM_ERR_SKIN, pid, -1, (double)sqrtf(rel2), eff_step(a));
+      record_error(a.err, RDSIM_ERR_SKIN, pid, -1, (double)sqrtf(rel2), step);
   }
-  if (a.flags & F_EM) em_update_in<D>(s, a, gi, pid, ti, acc, eff_em_step(a), a.flags, w0, t);
 }
 
-// The same with the words loaded here (xo_h: the current high words).
+// Per-particle tail of the drift kernels, on one thread per particle: walls
+// (pyrdsim.pyx:1979-1986), bonded terms, drift store, finiteness and skin
+// checks, and the fused Euler-Maruyama update.  acc holds the pair drift;
+// xo_h: the current high words.
 template <int D>
 __device__ inline void force_tail(const SysDev& s, const WallLaw* walls, const Args& a, int gi,
                                   int pid, const uint32_t* xo_h, uint32_t mi, float* acc,
@@ -664,7 +841,20 @@ __device__ inline void force_tail(const SysDev& s, const WallLaw* walls, const A
   TailIn t = tail_load<D>(a, gi);
 #pragma unroll
   for (int k = 0; k < D; k++) t.xh[k] = xo_h[k];
-  force_tail_in<D>(s, walls, a, gi, pid, t, mi, acc, w0);
+  const int ti = mi & 0xff;
+  wall_terms<D>(s, walls, t.xh, t.xl, ti, acc);
+  add_bonded<D>(s, a, t.xh, t.xl, pid, mi, 0, acc);
+  if (a.flags & F_STORE_DRIFT) {
+#pragma unroll
+    for (int k = 0; k < D; k++) a.drift[k][gi] = acc[k];
+  }
+  tail_checks<D>(s, a, pid, t.xh, t.xr, acc, eff_step(a));
+  if (a.flags & F_EM) {
+    unsigned long long X[3];
+    em_update_in<D>(s, a, pid, ti, acc, eff_em_step(a), a.flags, w0, t, X);
+#pragma unroll
+    for (int k = 0; k < D; k++) store_words(s, a, gi, k, X[k]);
+  }
 }
 
 // ---------------------------------------------------------------------------

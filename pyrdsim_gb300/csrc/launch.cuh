@@ -10,11 +10,11 @@ namespace rd {
 // and table staging overlap that kernel's tail); every kernel waits
 // (griddepcontrol.wait) before it reads what earlier work writes.
 template <class... P, class... A>
-void launch(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+void launch_dyn(void (*k)(P...), dim3 grid, dim3 block, size_t shared, cudaStream_t st, A... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
+  cfg.dynamicSmemBytes = shared;
   cfg.stream = st;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -22,6 +22,11 @@ void launch(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) 
   cfg.attrs = at;
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+
+template <class... P, class... A>
+void launch(void (*k)(P...), dim3 grid, dim3 block, cudaStream_t st, A... args) {
+  launch_dyn(k, grid, block, 0, st, args...);
 }
 
 }  // namespace rd

@@ -22,8 +22,20 @@
 // particles.  Phase A: TPP lanes per particle walk its list and combine with
 // shuffles into shared memory.  Phase B: one thread per particle runs the
 // per-particle tail (walls, bonded terms, Euler-Maruyama update; or the
-// reaction draw).  The data phase B needs and the warp's list rows are
-// prefetched into L1 at kernel start.
+// reaction draw).
+//
+// Neighbour staging (the period kernel).  A chunk's particles are neighbours in
+// space, so their lists name the same few hundred particles over and over.
+// k_nlist also writes, per chunk, the sorted indices of the particles in the
+// runs its rows scan (stg_g: the touched part of every touched chunk, side by
+// side) and every list row as 16-bit slot codes into that table (slot << 4,
+// bit 0: same molecule), two codes per word, the word of a lane next to its
+// neighbours'.  A step loads the staged particles once, coalesced, into shared
+// memory as 16-byte records and walks the rows there, in list order and with
+// the arithmetic of the gathers (the sums are the same bit for bit).  In small
+// systems LPC lanes share what one lane would walk (period.cuh).  A row
+// longer than the codes hold, or a chunk that touches more particles than fit,
+// gathers from memory instead.
 #pragma once
 
 #include "kernels.cuh"
@@ -32,6 +44,12 @@
 #ifndef RD_LIST_MIN_BLOCKS
 #define RD_LIST_MIN_BLOCKS 8
 #endif
+// the same where every pair law is a single Lennard-Jones n = 6 law: more
+// warps in flight are worth the registers there (wall fluid, 1,048,576
+// particles, 40 steps: 5,329 us at 8 with the general walk; the walk of
+// lj_walk 5,676 / 5,059 / 4,860 us at 8 / 10 / 12, 8,450 us at 14, where it
+// spills in the loop; the general walk is slower at 7 and at 10 than at 8)
+constexpr int LJ_MIN_BLOCKS = 12;
 // list entries loaded per lane before their neighbours are gathered
 #ifndef RD_LIST_BATCH
 #define RD_LIST_BATCH 2
@@ -276,32 +294,26 @@ struct Nb {
   int v;  // entry: sorted index | LIST_SAME_MOL
 };
 
-// The final type word of sorted particle j whose reaction draw is still
-// pending (period kernel): polled until its chunk writes it, for at most
-// a.wait_ns; then RDSIM_ERR_SYNC is recorded and the old word is used.
-__device__ inline uint32_t wait_final_meta(const Args& a, int j, uint32_t v) {
-  const unsigned long long t0 = global_timer();
-  while (v & META_PENDING) {
-    asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(a.meta + j) : "memory");
-    if ((long long)(global_timer() - t0) > a.wait_ns) {
-      record_error(a.err, RDSIM_ERR_SYNC, (long long)j, -2, 0.0, eff_step(a));
-      return v & ~META_PENDING;
-    }
-  }
-  return v;
-}
-
-// PEND (period kernel): a neighbour whose draw of this step is pending is
-// waited for, so that its type is the one after this step's reactions.
+// PEND (period kernel): the neighbour's record of this step, waited for until
+// it is written and its reaction draw resolved.
 template <int D, bool PEND = false>
 __device__ inline Nb gather(const Args& a, int v) {
   Nb n;
   const int j = v & 0x7fffffff;
   n.v = v;
+  if (PEND) {
+    const int st = period_n;
+    uint4 r = get_rec(a, a.rec[st & 1] + j, REC_TAG, st);
+    if (r.w & REC_PENDING) r = rec_wait(a, a.rec[st & 1] + j, REC_TAG, st, true);
+    n.x[0] = r.x;
+    n.x[1] = r.y;
+    n.x[2] = r.z;
+    n.m = r.w & 0xfu;
+  } else {
 #pragma unroll
-  for (int k = 0; k < 3; k++) n.x[k] = k < D ? (PEND ? ldw(a, a.xp[k] + j) : a.xp[k][j]) : 0u;
-  n.m = PEND ? ldw(a, a.meta + j) : a.meta[j];
-  if (PEND && (n.m & META_PENDING)) n.m = wait_final_meta(a, j, n.m);
+    for (int k = 0; k < 3; k++) n.x[k] = k < D ? a.xp[k][j] : 0u;
+    n.m = a.meta[j];
+  }
   return n;
 }
 
@@ -350,15 +362,16 @@ __device__ inline void for_entries(const SysDev& s, const Args& a, int i, int la
 
 // Reaction prefilter of a step (sorted particle gi of type ti): the
 // float64 total propensity of that step grows monotonically with every
-// neighbour count, so rxA + rxB * (list entries), with a relative margin far
-// above the rounding of the reference's repeated additions, bounds it from
-// above.  If dt times the bound does not exceed the step's u1 (the same
+// neighbour count, so rxA + rxB * cnt, with cnt the list entries that can come
+// within a reaction radius before the next rebuild (within it plus twice the
+// allowed displacement at the last one) and a relative margin far above the
+// rounding of the reference's repeated additions, bounds it from above.  If dt times the bound does not exceed the step's u1 (the same
 // counter-based draw the reaction kernel makes), the draw `dt * total > u1`
 // (pyrdsim.pyx:2211-2213) cannot succeed and the particle keeps its type.
 // The bound and the comparison are float32: rxAf, rxBf and dtf are rounded
 // up, the relative margin 1e-5 covers the float32 rounding, and the uniform
 // is replaced by the lower bound of its top 24 bits.  Returns true when the
-// draw may succeed (cnt: list entries, pid: caller index, w0: the tag-0
+// draw may succeed (pid: caller index, w0: the tag-0
 // words of the next step).
 template <int D>
 __device__ inline bool rx_may_react(const SysDev& s, int ti, int cnt, int pid, long long step,
@@ -372,6 +385,35 @@ __device__ inline bool rx_may_react(const SysDev& s, int ti, int cnt, int pid, l
   return s.dtf * ub > u1lo;
 }
 
+// The period kernel's records of sorted particle i before its first step: the
+// state as step 0, "no step yet" for the other parity.
+template <int D>
+__device__ inline void first_records(const Args& a, int i, uint32_t mi, bool pending) {
+  uint32_t p[3] = {0u, 0u, 0u}, l[3] = {0u, 0u, 0u}, h[3] = {0u, 0u, 0u};
+#pragma unroll
+  for (int k = 0; k < D; k++) {
+    p[k] = a.xp[k][i];
+    l[k] = a.xl[k][i];
+    h[k] = a.xh[k][i];
+  }
+  const uint32_t ty = mi & 0xfu;
+  a.rec[0][i] = make_uint4(p[0], p[1], p[2], rec_word(0, ty, ty, pending));
+  a.recl[0][i] = make_uint4(l[0], l[1], l[2], 0u);
+  a.rech[0][i] = make_uint4(h[0], h[1], h[2], 0u);
+  a.rec[1][i].w = REC_NONE;
+  a.recl[1][i].w = REC_NONE;
+  a.rech[1][i].w = REC_NONE;
+}
+
+// The same for a launch of the period kernel that no list builder precedes.
+template <int D>
+__global__ void k_first_records(Args a) {
+  pdl_trigger();
+  pdl_wait();
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < a.n_total) first_records<D>(a, i, a.meta[i], false);
+}
+
 // Rebuild: every particle's list row and entry count.  NT threads per
 // particle (3 for D >= 2: one per row of cells in 2D, one per three rows in
 // 3D) scan their rows' runs in candidate order, four candidates per batch of
@@ -380,15 +422,30 @@ __device__ inline bool rx_may_react(const SysDev& s, int ti, int cnt, int pid, l
 // thread whose rows hold more than BCAP listed pairs rescans them to write
 // the rest.  With F_RX_HERE the first thread of each particle also runs the
 // reaction prefilter of its step with the fresh entry count.  With
-// F_PERIOD_PREP (CTA = chunk of the period kernel) it also writes the
-// chunk's neighbour-chunk bitmap (the chunks of every list entry, of the
-// bonded partners and the chunk itself), its candidate mask of the rebuild
-// step (their type words carry META_PENDING until resolved, by the period
-// kernel or by the listed reaction kernel, which also gets the candidate
-// list) and its progress word (0).
-template <int D, int TPP>
-__global__ void __launch_bounds__((LBLOCK / TPP) * (D == 1 ? 1 : 3)) k_nlist(Args a) {
-  constexpr int PER = LBLOCK / TPP;
+// F_PERIOD_PREP it also writes the period kernel's records of its particles:
+// of step 0 (candidates of the rebuild step marked pending), and "no step yet"
+// for the other parity.  Chunks' staging tables and slot codes: see the top of
+// this file.
+// Position, in 16-bit codes, of entry e of particle p of a chunk: chain e % TPP of
+// its row is shared by LPC lanes, which take its entries in turn.
+template <int TPP, int LPC>
+__device__ inline int code_at(int p, int e) {
+  const int k = e / TPP, m = k / LPC;
+  return (((m >> 1) * LBLOCK) + (p * TPP + e % TPP) * LPC + k % LPC) * 2 + (m & 1);
+}
+
+constexpr int STG_HASH = 128;  // touched chunks of a chunk (open addressing)
+
+struct StageHash {
+  int key[STG_HASH], lo[STG_HASH], hi[STG_HASH], off[STG_HASH];
+  int total, on;
+};
+
+// LPC: see period.cuh (the period kernel's lanes per chain of a row; its chunks
+// are this kernel's).
+template <int D, int TPP, int LPC>
+__global__ void __launch_bounds__((LBLOCK / TPP / LPC) * (D == 1 ? 1 : 3)) k_nlist(Args a) {
+  constexpr int PER = LBLOCK / TPP / LPC;
   constexpr int NT = D == 1 ? 1 : 3;
   constexpr int NTH = PER * NT;
   constexpr int NROW = D == 3 ? 9 : (D == 2 ? 3 : 1);
@@ -398,9 +455,8 @@ __global__ void __launch_bounds__((LBLOCK / TPP) * (D == 1 ? 1 : 3)) k_nlist(Arg
   constexpr int BCAP = 24;
   __shared__ SysDev sys;
   __shared__ int sbuf[NTH][BCAP];
-  __shared__ int scnt[NTH];
-  __shared__ uint32_t sbits[PMASK_WORDS];
-  __shared__ uint32_t scand[CAND_WORDS];
+  __shared__ int2 scnt[NTH];
+  __shared__ StageHash sth;
   pdl_trigger();
   const Chunk ch = chunk_at<PER>(a, (int)blockIdx.x);
   {
@@ -410,9 +466,17 @@ __global__ void __launch_bounds__((LBLOCK / TPP) * (D == 1 ? 1 : 3)) k_nlist(Arg
     ls.store(reinterpret_cast<int*>(&sys), NS);
   }
   const bool prep = (a.flags & F_PERIOD_PREP) != 0;
-  if (prep) {
-    for (int w = (int)threadIdx.x; w < PMASK_WORDS; w += NTH) sbits[w] = 0u;
-    for (int w = (int)threadIdx.x; w < CAND_WORDS; w += NTH) scand[w] = 0u;
+  const bool stage = a.codes != nullptr;
+  if (stage) {
+    for (int q = (int)threadIdx.x; q < STG_HASH; q += NTH) {
+      sth.key[q] = 0;
+      sth.lo[q] = 0x7fffffff;
+      sth.hi[q] = -1;
+    }
+    if (threadIdx.x == 0) {
+      sth.total = 0;
+      sth.on = 1;
+    }
   }
   pdl_wait();
   __syncthreads();
@@ -451,7 +515,8 @@ __global__ void __launch_bounds__((LBLOCK / TPP) * (D == 1 ? 1 : 3)) k_nlist(Arg
     rb[2 * r + 1] = two ? cs[lo1] : 0;
     re[2 * r + 1] = two ? cs[hi1 + 1] : 0;
   }
-  // the listed pairs of this thread's rows, in candidate order: emit(k, entry)
+  // the listed pairs of this thread's rows, in candidate order: emit(k, entry,
+  // squared distance)
   auto scan_rows = [&](auto&& emit) {
     int k = 0;
 #pragma unroll
@@ -487,44 +552,91 @@ __global__ void __launch_bounds__((LBLOCK / TPP) * (D == 1 ? 1 : 3)) k_nlist(Arg
             hit = (pmask >> ((mj[u] >> 8) & 0xff)) & 1;
             ent = j;
           }
-          if (hit) emit(k++, ent);
+          if (hit) emit(k++, ent, r2);
         }
       }
     }
     return k;
   };
-  // period kernel: the chunk of sorted particle j of this system (a
-  // system's chunks are consecutive runs of PER particles) into the bitmap;
-  // runs of entries fall into one chunk, so only changes are marked
-  const int chunk0 = (int)blockIdx.x - (ch.beg - s.p0) / PER;
-  int lastc = -1;
-  auto mark = [&](int j) {
-    const int c = chunk0 + (j - s.p0) / PER;
-    if (c != lastc) {
-      atomicOr(&sbits[c >> 5], 1u << (c & 31));
-      lastc = c;
+  // slot of chunk key - 1 (of this system) in the hash, -1 if absent
+  auto find = [&](int key, bool insert) {
+    for (int q = 0, h = key & (STG_HASH - 1); q < STG_HASH; q++, h = (h + 1) & (STG_HASH - 1)) {
+      const int k = insert ? atomicCAS(&sth.key[h], 0, key) : sth.key[h];
+      if (k == key || (insert && k == 0)) return h;
+      if (k == 0) return -1;
     }
+    return -1;
   };
-  const int cnt = scan_rows([&](int k, int ent) {
-    if (k < BCAP) sbuf[tid][k] = ent;
-    if (prep) mark(ent & 0x7fffffff);
-  });
-  if (prep && valid) {
-    mark(i);
-    if (t == 0 && tmi != 0xff) {  // bonded partners: every atom of the molecule
-      const int mb = a.pid[i] - loci, na = a.tmpl[tmi].n_atoms;
-      for (int b = 0; b < na; b++) mark(a.slot_of[mb + b]);
+  if (stage && valid) {
+    // the runs of the first particle of each cell: those of the others too
+    bool first = pp == 0;
+    if (!first) {
+#pragma unroll
+      for (int k = 0; k < D; k++) first = first || cell_coord(s, k, a.xr[k][i - 1]) != c[k];
+    }
+    if (first) {
+#pragma unroll
+      for (int q = 0; q < NRUN; q++)
+        for (int b = rb[q]; b < re[q];) {
+          const int cc = (b - s.p0) / PER, e = min(re[q], s.p0 + (cc + 1) * PER);
+          const int h = find(cc + 1, true);
+          if (h < 0) {
+            sth.on = 0;
+          } else {
+            atomicMin(&sth.lo[h], b);
+            atomicMax(&sth.hi[h], e - 1);
+          }
+          b = e;
+        }
     }
   }
-  scnt[tid] = cnt;
+  int rcnt = 0;
+  const int cnt = scan_rows([&](int k, int ent, float r2) {
+    if (k < BCAP) sbuf[tid][k] = ent;
+    rcnt += r2 < s.Rrl2 ? 1 : 0;
+  });
+  scnt[tid] = make_int2(cnt, rcnt);
   __syncthreads();
-  int off = 0, total = 0;
+  int off = 0, total = 0, rtotal = 0;
 #pragma unroll
   for (int u = 0; u < NT; u++) {
-    const int cu = scnt[pp * NT + u];
-    if (u < t) off += cu;
-    total += cu;
+    const int2 cu = scnt[pp * NT + u];
+    if (u < t) off += cu.x;
+    total += cu.x;
+    rtotal += cu.y;
   }
+  if (stage) {
+    // table positions, in whatever order the counter hands them out
+    for (int q = tid; q < STG_HASH; q += NTH)
+      if (sth.key[q]) {
+        const int len = sth.hi[q] - sth.lo[q] + 1;
+        sth.off[q] = atomicAdd(&sth.total, len) - sth.lo[q];
+      }
+    __syncthreads();
+    const bool on = sth.on && sth.total <= a.stg_max;
+    if (tid == 0) a.stg_n[blockIdx.x] = on ? sth.total : -1;
+    if (on) {
+      int* g = a.stg_g + (size_t)blockIdx.x * a.stg_max;
+      for (int q = tid / 16; q < STG_HASH; q += NTH / 16)
+        if (sth.key[q])
+          for (int j = sth.lo[q] + tid % 16; j <= sth.hi[q]; j += 16) g[sth.off[q] + j] = j;
+    }
+  }
+  // the slot code of entry e of this particle
+  unsigned short* codes = reinterpret_cast<unsigned short*>(a.codes) +
+                          (size_t)blockIdx.x * a.kw * LBLOCK * 2;
+  const bool coded = stage && total <= a.kw * 2 * TPP * LPC;
+  int lastc = -1, lasto = 0;
+  auto put_code = [&](int e, int ent) {
+    if (!coded) return;
+    const int j = ent & 0x7fffffff, cc = (j - s.p0) / PER;
+    if (cc != lastc) {
+      const int h = find(cc + 1, false);
+      lastc = cc;
+      lasto = h >= 0 ? sth.off[h] : 0;
+    }
+    codes[code_at<TPP, LPC>(pp, e)] = (unsigned short)(((j + lasto) << 4) | (ent < 0 ? 1 : 0));
+  };
   int4 rec = make_int4(0, 0, 0, 0);
   bool listed = false;
   if (valid) {
@@ -532,28 +644,27 @@ __global__ void __launch_bounds__((LBLOCK / TPP) * (D == 1 ? 1 : 3)) k_nlist(Arg
     const int W = a.W, npad = a.npad;
     const int nb = min(cnt, BCAP);
     for (int k = 0; k < nb; k++)
-      if (off + k < W) nbr[ell_index<TPP>(off + k, i, npad)] = sbuf[tid][k];
+      if (off + k < W) {
+        nbr[ell_index<TPP>(off + k, i, npad)] = sbuf[tid][k];
+        put_code(off + k, sbuf[tid][k]);
+      }
     if (cnt > BCAP && off + BCAP < W)
-      scan_rows([&](int k, int ent) {
-        if (k >= BCAP && off + k < W) nbr[ell_index<TPP>(off + k, i, npad)] = ent;
+      scan_rows([&](int k, int ent, float) {
+        if (k >= BCAP && off + k < W) {
+          nbr[ell_index<TPP>(off + k, i, npad)] = ent;
+          put_code(off + k, ent);
+        }
       });
     if (t == 0) {
       a.ncnt_out[i] = total;
+      a.rcnt_out[i] = rtotal;
       if (a.flags & F_RX_HERE) {  // reaction prefilter of this step (see rx_may_react)
         rec = make_int4(i, (int)mi, total, a.pid[i]);
-        listed = rx_may_react<D>(s, (int)(mi & 0xff), total, rec.w, eff_step(a), nullptr);
-        a.meta_out[i] = mi | ((prep && listed) ? META_PENDING : 0u);
+        listed = rx_may_react<D>(s, (int)(mi & 0xff), rtotal, rec.w, eff_step(a), nullptr);
+        a.meta_out[i] = mi;
       }
+      if (prep) first_records<D>(a, i, mi, listed);
     }
-  }
-  if (prep) {
-    if (listed) atomicOr(&scand[pp >> 5], 1u << (pp & 31));
-    __syncthreads();
-    const int c = (int)blockIdx.x;
-    for (int w = (int)threadIdx.x; w < PMASK_WORDS; w += NTH)
-      a.nbmask[(size_t)c * PMASK_WORDS + w] = sbits[w];
-    for (int w = (int)threadIdx.x; w < CAND_WORDS; w += NTH) a.cand0[c * CAND_WORDS + w] = scand[w];
-    if (threadIdx.x == 0) a.pflag[c * PFLAG_STRIDE] = 0;
   }
   if (a.flags & F_RX_HERE) {  // the candidate list of the per-step kernels
     const unsigned int bal = __ballot_sync(0xffffffffu, listed);
@@ -565,6 +676,32 @@ __global__ void __launch_bounds__((LBLOCK / TPP) * (D == 1 ? 1 : 3)) k_nlist(Arg
       base = __shfl_sync(0xffffffffu, base, leader);
       if (listed) a.rx_list[(size_t)p * a.npad + base + __popc(bal & ((1u << l32) - 1u))] = rec;
     }
+  }
+}
+
+// Adds one listed partner (type tj before the step's reactions, pair words xj,
+// sorted index j()) of particle m (type tm, pair words xm) to the counts of the
+// neighbour-dependent reactions whose radius it is within.
+template <int D, class J>
+__device__ inline void count_partner(const SysDev& s, const RxDev* rx, const Args& a, int m, J&& j,
+                                     int tm, int tj, const uint32_t* xm, const uint32_t* xj,
+                                     uint32_t* cw) {
+  float d[3];
+  const float r2 = pair_geom<D>(s, xj, xm, d);
+  if (!(r2 < s.Rrx2)) return;
+  const unsigned int rmask = s.rxmatch[tm * MAXT + tj];
+  double dexact = -1.0;
+  for (unsigned int b = rmask; b; b &= b - 1u) {
+    const int r = __ffs(b) - 1;
+    const RxDev& R = rx[r];
+    bool inside;
+    if (r2 < R.r02_lo) inside = true;
+    else if (r2 > R.r02_hi) inside = false;
+    else {
+      if (dexact < 0) dexact = exact_dist<D>(s, a, m, j());
+      inside = dexact < R.r0;
+    }
+    if (inside) cw[r >> 1] += 1u << (16 * (r & 1));
   }
 }
 
@@ -589,26 +726,9 @@ __device__ inline int resolve_listed(const SysDev& s, const RxDev* rx, const Arg
     uint32_t xm[3] = {0u, 0u, 0u};
 #pragma unroll
     for (int k = 0; k < D; k++) xm[k] = a.xp[k][m];
-    const float Rrx2 = s.Rrx2;
     auto count = [&](const Nb& nb) {
-      const int j = nb.v & 0x7fffffff;
-      float d[3];
-      const float r2 = pair_geom<D>(s, nb.x, xm, d);
-      if (!(r2 < Rrx2)) return;
-      const unsigned int rmask = s.rxmatch[tm * MAXT + (nb.m & 0xff)];
-      double dexact = -1.0;
-      for (unsigned int b = rmask; b; b &= b - 1u) {
-        const int r = __ffs(b) - 1;
-        const RxDev& R = rx[r];
-        bool inside;
-        if (r2 < R.r02_lo) inside = true;
-        else if (r2 > R.r02_hi) inside = false;
-        else {
-          if (dexact < 0) dexact = exact_dist<D>(s, a, m, j);
-          inside = dexact < R.r0;
-        }
-        if (inside) cw[r >> 1] += 1u << (16 * (r & 1));
-      }
+      count_partner<D>(s, rx, a, m, [&] { return nb.v & 0x7fffffff; }, tm, (int)(nb.m & 0xff), xm,
+                       nb.x, cw);
     };
     if (cnt <= a.W) {
       for (int e = lane; e < cnt; e += 32) count(gather<D>(a, a.nbr[ell_index<TPP>(e, m, a.npad)]));
@@ -623,18 +743,16 @@ __device__ inline int resolve_listed(const SysDev& s, const RxDev* rx, const Arg
                    : tm;
 }
 
-// Phase A of the drift kernels: this lane's share of the pair drift of
-// sorted particle i (type word mi, pair words xo) over its list entries
-// (pyrdsim.pyx:1988-2030), added to acc.
-// One list entry's pair drift on particle i (type ti, pair words xo).
-template <int D>
-__device__ __forceinline__ void pair_term(const ListShared& sh, const Args& a, int i, int ti,
-                                          const uint32_t* xo, const Nb& nb, float* acc) {
+// One listed pair's drift on particle i (type ti, pair words xo) from a
+// partner with pair words xj and type tj (sorted index j(), evaluated where a
+// cutoff is close), added to acc (pyrdsim.pyx:1988-2030).
+template <int D, class J>
+__device__ __forceinline__ void pair_eval(const ListShared& sh, const Args& a, int i, int ti,
+                                          const uint32_t* xo, const uint32_t* xj, int tj, J&& j,
+                                          float* acc) {
   const SysDev& s = sh.sys;
-  if (nb.v < 0) return;  // same molecule: reactions only
   float d[3];
-  const float r2 = pair_geom<D>(s, nb.x, xo, d);
-  const int tj = nb.m & 0xff;
+  const float r2 = pair_geom<D>(s, xj, xo, d);
   if (!(r2 < s.prc2[ti * MAXT + tj])) return;  // beyond every law of the pair
   const unsigned int pp = s.ppair[ti * MAXT + tj];
   const PairLaw& L0 = sh.laws[(pp >> 5) & 0x3ff];
@@ -644,10 +762,142 @@ __device__ __forceinline__ void pair_term(const ListShared& sh, const Args& a, i
     // arithmetic inline
     fr = lj6_over_r(L0.c0, L0.c1, r2, recip(r2));
   } else {
-    fr = pair_force<D>(s, sh.laws, a, i, nb.v, pp, r2);
+    fr = pair_force<D>(s, sh.laws, a, i, j, pp, r2);
   }
 #pragma unroll
   for (int k = 0; k < D; k++) acc[k] = fmaf(fr, d[k], acc[k]);
+}
+
+template <int D>
+__device__ __forceinline__ void pair_term(const ListShared& sh, const Args& a, int i, int ti,
+                                          const uint32_t* xo, const Nb& nb, float* acc) {
+  if (nb.v < 0) return;  // same molecule: reactions only
+  pair_eval<D>(sh, a, i, ti, xo, nb.x, (int)(nb.m & 0xff), [&] { return nb.v; }, acc);
+}
+
+// What the pair loop needs of a type pair in one 16-byte read: the largest
+// guarded rc^2 of its laws and, for a single Lennard-Jones n = 6 law, the lower
+// edge of its guard band and its constants (lo < 0: other laws).
+// {rc2, lo, c0, c1} by [ti * ntypes + tj].  Whole CTA; the tables are staged.
+__device__ inline void fill_rows(float4* rows, const ListShared& sh) {
+  const int nt = sh.sys.ntypes;
+  for (int q = threadIdx.x; q < nt * nt; q += LBLOCK) {
+    const int t = q / nt * MAXT + q % nt;
+    const unsigned int pp = sh.sys.ppair[t];
+    const PairLaw& L = sh.laws[(pp >> 5) & 0x3ff];
+    const bool lj6 = (pp & 0x8000u) != 0u;
+    rows[q] = make_float4(sh.sys.prc2[t], lj6 ? L.rc2_lo : -1.f, lj6 ? L.c0 : 0.f, lj6 ? L.c1 : 0.f);
+  }
+}
+
+// Phase A from the staged records of a period kernel: this lane's share
+// (entries lane, lane + TPP, ...) of the pair drift of sorted particle i.
+// codes: the lane's first word of the chunk's table; g, rec: the table's sorted
+// indices and the records of this step.  A neighbour within range whose draw is
+// pending (RX) is waited for.  The walk holds no call: at a distance in a cutoff's
+// guard band it stops and returns false, and the lane walks its row again in
+// staged_slow, where the float64 distance decides.  Two entries are in flight
+// at a time: the loop is bound by the latency of its shared-memory reads and of
+// the reciprocal.
+//
+// LPC > 1: LPC lanes share a chain (the entries that one lane would walk).
+// Each evaluates every LPC-th entry; then the terms go round by shuffles and
+// every lane adds them in list order, so the sum is that of LPC = 1.  All lanes
+// of the warp call it (cnt = 0: no row), and the result is valid on each.
+template <int D, int TPP, int LPC, bool RX>
+__device__ __forceinline__ bool staged_walk(const ListShared& sh, const Args& a, const float4* rows,
+                                            const uint4* slots, const int* g, const uint4* rec,
+                                            const uint32_t* codes, int chain, int sub, int cnt,
+                                            const uint32_t* xo, int ti, float* acc) {
+  const SysDev& s = sh.sys;
+  const float4* row = rows + ti * s.ntypes;
+  // entries of this lane, and the rounds the lanes of the warp make together
+  const int mine = ((cnt - chain + TPP - 1) / TPP - sub + LPC - 1) / LPC;
+  const int rounds = LPC == 1 ? mine : __reduce_max_sync(0xffffffffu, max(mine, 0));
+  bool ok = true;
+  uint32_t next = mine > 0 ? codes[0] : 0u;
+  for (int q = 0; q < rounds; q += 2) {
+    const uint32_t cw = next;
+    if (q + 2 < mine) next = codes[((q >> 1) + 1) * LBLOCK];
+    const unsigned int code[2] = {q < mine ? cw & 0xffffu : 1u, q + 1 < mine ? cw >> 16 : 1u};
+    uint4 r[2];
+    float d[2][3], r2[2], fr[2];
+    float4 t[2];
+#pragma unroll
+    for (int u = 0; u < 2; u++) r[u] = slots[code[u] >> 4];
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      const uint32_t xj[3] = {r[u].x, r[u].y, r[u].z};
+      t[u] = row[r[u].w & 0xfu];
+      r2[u] = pair_geom<D>(s, xj, xo, d[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < 2; u++) {
+      fr[u] = 0.f;
+      bool in = !(code[u] & 1u);  // not of the same molecule (reactions only) or past the row
+      if (RX && in && (r[u].w & REC_PENDING) && r2[u] <= s.R2) {
+        r[u].w = pending_word(a, &rec[g[code[u] >> 4]].w);
+        t[u] = row[r[u].w & 0xfu];
+      }
+      in = in && r2[u] < t[u].x;  // else beyond every law of the pair
+      if (in) {
+        if (r2[u] < t[u].y) {
+          fr[u] = lj6_over_r(t[u].z, t[u].w, r2[u], recip(r2[u]));
+        } else {
+          bool close = t[u].y >= 0.f;
+          if (!close)
+            fr[u] = laws_over_r(sh.laws, s.ppair[ti * MAXT + (int)(r[u].w & 0xfu)], r2[u], close);
+          if (close) {
+            if (LPC == 1) return false;
+            ok = false;
+          }
+        }
+        if (LPC == 1) {
+#pragma unroll
+          for (int k = 0; k < D; k++) acc[k] = fmaf(fr[u], d[u][k], acc[k]);
+        }
+      }
+    }
+    if (LPC > 1) {
+      // (no term: fr = 0 leaves the sum as it is)
+#pragma unroll
+      for (int u = 0; u < 2; u++) {
+#pragma unroll
+        for (int v = 0; v < LPC; v++) {
+          const float f = __shfl_sync(0xffffffffu, fr[u], v, LPC);
+#pragma unroll
+          for (int k = 0; k < D; k++)
+            acc[k] = fmaf(f, __shfl_sync(0xffffffffu, d[u][k], v, LPC), acc[k]);
+        }
+      }
+    }
+  }
+  if (LPC > 1) {
+    const unsigned int bad = __ballot_sync(0xffffffffu, !ok);
+    ok = ((bad >> ((threadIdx.x & 31u) & ~(unsigned)(LPC - 1))) & ((1u << LPC) - 1u)) == 0u;
+  }
+  return ok;
+}
+
+// The chain of particle p of the chunk by one lane, with whatever calls it needs.
+template <int D, int TPP, int LPC>
+__device__ __noinline__ float3 staged_slow(const ListShared& sh, const Args& a, const uint4* slots,
+                                           const int* g, const uint32_t* codes, int i, int p,
+                                           int chain, int cnt, uint3 x, int ti) {
+  const unsigned short* c16 = reinterpret_cast<const unsigned short*>(codes);
+  const uint32_t xo[3] = {x.x, x.y, x.z};
+  float acc[3] = {0.f, 0.f, 0.f};
+  for (int e = chain; e < cnt; e += TPP) {
+    const unsigned int code = c16[code_at<TPP, LPC>(p, e)];
+    if (code & 1u) continue;  // same molecule: reactions only
+    const uint4 r = slots[code >> 4];
+    const uint32_t xj[3] = {r.x, r.y, r.z};
+    int tj = (int)(r.w & 0xfu);
+    if (r.w & REC_PENDING)
+      tj = (int)(rec_wait(a, a.rec[period_n & 1] + g[code >> 4], REC_TAG, period_n, true).w & 0xfu);
+    pair_eval<D>(sh, a, i, ti, xo, xj, tj, [&] { return g[code >> 4]; }, acc);
+  }
+  return make_float3(acc[0], acc[1], acc[2]);
 }
 
 template <int D, int TPP, bool PEND = false>
@@ -658,13 +908,58 @@ __device__ __forceinline__ void pair_drift(const ListShared& sh, const Args& a, 
                             [&](const Nb& nb) { pair_term<D>(sh, a, i, ti, xo, nb, acc); });
 }
 
+// Phase A of the drift kernel where every pair law is a single Lennard-Jones n
+// = 6 law: pair_drift's sums by a walk that holds no call and reads one row per
+// type pair (fill_rows).  Bound by the latency of the gathers: the neighbour of
+// the next entry and the index of the one after it are in flight while an entry
+// is evaluated (4,860 -> 4,679 us per 40 steps at 1,048,576 particles; two
+// entries at a time 4,679, one 4,630).  False at a distance in a cutoff's guard
+// band (the lane then takes pair_drift).  Rows within the stored width only.
+template <int D, int TPP>
+__device__ __forceinline__ bool lj_walk(const ListShared& sh, const Args& a, const float4* rows,
+                                        int i, int lane, int cnt, const uint32_t* xo, int ti,
+                                        float* acc) {
+  const SysDev& s = sh.sys;
+  const float4* row = rows + ti * s.ntypes;
+  auto entry = [&](int e) {
+    return e < cnt ? a.nbr[ell_index<TPP>(e, i, a.npad)] : (i | LIST_SAME_MOL);
+  };
+  Nb nb = gather<D>(a, entry(lane));
+  int v = entry(lane + TPP);
+  for (int e = lane; e < cnt; e += TPP) {
+    const Nb cur = nb;
+    nb = gather<D>(a, v);
+    v = entry(e + 2 * TPP);
+    if (cur.v < 0) continue;  // same molecule: reactions only
+    float d[3];
+    const float r2 = pair_geom<D>(s, cur.x, xo, d);
+    const float4 t = row[cur.m & 0xffu];
+    if (!(r2 < t.x)) continue;  // beyond the pair's law
+    if (!(r2 < t.y)) return false;
+    const float fr = lj6_over_r(t.z, t.w, r2, recip(r2));
+#pragma unroll
+    for (int k = 0; k < D; k++) acc[k] = fmaf(fr, d[k], acc[k]);
+  }
+  return true;
+}
+
+template <int D, int TPP>
+__device__ __noinline__ float3 lj_slow(const ListShared& sh, const Args& a, int i, int lane,
+                                       int cnt, uint3 x, uint32_t mi) {
+  const uint32_t xo[3] = {x.x, x.y, x.z};
+  float acc[3] = {0.f, 0.f, 0.f};
+  pair_drift<D, TPP>(sh, a, i, lane, cnt, xo, mi, acc);
+  return make_float3(acc[0], acc[1], acc[2]);
+}
+
 // Drift kernel.  Phase A: TPP lanes per particle sum the pair drift over its
 // list entries (pyrdsim.pyx:1988-2030).  Phase B: one thread per particle
 // adds walls and bonded terms and performs the fused Euler-Maruyama update.
-template <int D, int TPP>
-__global__ void __launch_bounds__(LBLOCK, RD_LIST_MIN_BLOCKS) k_force_l(Args a) {
+template <int D, int TPP, bool LJ>
+__global__ void __launch_bounds__(LBLOCK, LJ ? LJ_MIN_BLOCKS : RD_LIST_MIN_BLOCKS) k_force_l(Args a) {
   constexpr int PER = LBLOCK / TPP;
   __shared__ ListShared sh;
+  __shared__ float4 rows[LJ ? MAXT * MAXT : 1];
   __shared__ float sacc[3][PER];
   pdl_trigger();
   const Chunk ch = chunk_of<PER>(a);
@@ -690,7 +985,22 @@ __global__ void __launch_bounds__(LBLOCK, RD_LIST_MIN_BLOCKS) k_force_l(Args a) 
   __syncthreads();
   const SysDev& s = sh.sys;
   float acc[3] = {0.f, 0.f, 0.f};
-  if (active && s.R2 > 0.f) pair_drift<D, TPP>(sh, a, i, lane, cnt, xo, mi, acc);
+  if (LJ) {
+    fill_rows(rows, sh);
+    __syncthreads();
+    if (active) {
+      bool ok = cnt <= a.W;
+      if (ok) ok = lj_walk<D, TPP>(sh, a, rows, i, lane, cnt, xo, (int)(mi & 0xff), acc);
+      if (!ok) {
+        const float3 f = lj_slow<D, TPP>(sh, a, i, lane, cnt, make_uint3(xo[0], xo[1], xo[2]), mi);
+        acc[0] = f.x;
+        acc[1] = f.y;
+        acc[2] = f.z;
+      }
+    }
+  } else if (active && s.R2 > 0.f) {
+    pair_drift<D, TPP>(sh, a, i, lane, cnt, xo, mi, acc);
+  }
 #pragma unroll
   for (int o = TPP >> 1; o > 0; o >>= 1) {
 #pragma unroll
@@ -722,7 +1032,7 @@ __global__ void __launch_bounds__(LBLOCK, RD_LIST_MIN_BLOCKS) k_force_l(Args a) 
     if (a.flags & F_RX_NEXT) {
       a.meta_out[ib] = mb;  // the next step's types, unless its draw succeeds
       rec = make_int4(ib, (int)mb, a.ncnt[ib], pid);
-      listed = rx_may_react<D>(s, (int)(mb & 0xff), rec.z, pid, eff_em_step(a), &w0);
+      listed = rx_may_react<D>(s, (int)(mb & 0xff), a.rcnt[ib], pid, eff_em_step(a), &w0);
     }
   }
   if (a.flags & F_RX_NEXT) {
@@ -909,535 +1219,6 @@ __global__ void __launch_bounds__(LBLOCK) k_react_listed(Args a) {
     const int newt = resolve_listed<D, TPP>(s, rx, a, rec, lane);
     if (lane == 0) a.meta_out[rec.x] = ((uint32_t)rec.y & 0xffffff00u) | (uint32_t)newt;
   }
-}
-
-// ---------------------------------------------------------------------------
-// Period kernel: every step of one rebuild period (the listed reactions of
-// each step, then its drift with the fused update of the next step) in one
-// launch, one CTA per chunk, all CTAs resident.  There is no grid-wide
-// barrier: after its drift of step n a chunk publishes progress n + 1, and
-// a chunk starts step n once every chunk it reads (its list entries' and
-// bonded partners' chunks, from the list builder's bitmap) has progress
-// >= n: their positions of step n and their types are written.  The list
-// relation is symmetric (the same distance and partner tests from both
-// ends), so the chunks that read a chunk are among those it waits for,
-// which also protects the buffers it overwrites.
-// Reactions: the drift of step n - 1 marks the type word of each particle
-// whose draw of step n may succeed with META_PENDING; the particle's own
-// chunk resolves the draw at the start of step n and writes the final word.
-// A neighbour that gathers a pending word waits for that word alone, so
-// only the particles next to a pending draw wait for it (and the symmetric
-// list again orders the resolution's reads of the old types before the
-// neighbour overwrites them).  Every wait ends after wait_ns of the global
-// timer, or as soon as any CTA has recorded an error: RDSIM_ERR_SYNC is
-// recorded and the CTA returns.  The arithmetic per particle is that of
-// k_force_l and k_react_listed (same functions), so the results equal
-// theirs bit for bit.
-
-// Polling: relaxed loads (an acquire load invalidates the SM's L1, which
-// the other CTAs on the SM use for their list rows).  With RD_PERIOD_CG = 0
-// (plain loads of other CTAs' words) one acquire fence follows once every
-// word has reached its target; with the default strong loads none does.
-#ifndef RD_PERIOD_POLL_ACQUIRE
-#define RD_PERIOD_POLL_ACQUIRE 0
-#endif
-#ifndef RD_PERIOD_SLEEP_NS
-#define RD_PERIOD_SLEEP_NS 32
-#endif
-
-__device__ inline int ld_poll(const int* p) {
-  int v;
-#if RD_PERIOD_POLL_ACQUIRE
-  asm volatile("ld.acquire.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-#else
-  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-#endif
-  return v;
-}
-
-// With RD_PERIOD_CG the words written by other CTAs are read from L2 and
-// the relaxed poll that saw a chunk's progress precedes those reads (they
-// issue only after the poll's loop has exited on the value, and the writer
-// fenced its words before publishing): no fence here, and the SM's L1 keeps
-// the list rows.
-__device__ inline void fence_acquire() {
-#if !RD_PERIOD_POLL_ACQUIRE && !RD_PERIOD_CG
-  asm volatile("fence.acq_rel.gpu;" ::: "memory");
-#endif
-}
-
-__device__ inline void st_release(int* p, int v) {
-  asm volatile("st.release.gpu.global.b32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
-}
-
-// Per-particle words of the chunk staged in shared memory by the tail
-// threads: static ones once per period (caller index, high words at the
-// rebuild), the CTA's own positions and the noise of the coming update
-// before each step's wait (they depend on no other chunk).
-template <int PER>
-struct PeriodStage {
-  int pid[PER];
-  uint32_t xr[3][PER];
-  uint32_t xh[3][PER];
-  uint32_t xl[3][PER];
-  uint32_t w[4][PER];               // Philox words of the update (tag 0)
-  float xi[3][PER];                 // their standard normals
-};
-
-// Neighbour staging of a chunk (period kernel).  Built once per period from
-// the chunk's static list rows: per chunk that its entries touch (itself
-// included), the run [lo, hi] of sorted indices touched, laid out back to
-// back (slot -> sorted index in g); every entry of a particle whose row fits
-// (at most LS_MAX entries, none regenerated from the cells) is rewritten as
-// its slot (bit 15: same molecule).  Each step the pair and type words of
-// all slots are loaded once, coalesced, into x / m; the pair loop reads them
-// from shared memory in the list's order, so its sums are those of the
-// gathers.  A chunk whose runs exceed SMAX slots (six per particle of the
-// chunk) or that touches more than STAGE_CH chunks gathers from memory as
-// before.
-constexpr int STAGE_CH = 64;
-constexpr int LS_MAX = 32;
-
-template <int D, int PER>
-struct PeriodNbStage {
-  static constexpr int SMAX = 6 * PER;
-  uint32_t x[D][SMAX];
-  uint32_t m[SMAX];
-  int g[SMAX];
-  unsigned short slot[LS_MAX][PER];
-  int lo[STAGE_CH], hi[STAGE_CH], base[STAGE_CH + 1];
-  unsigned short ch[STAGE_CH];
-  int nch, total, on;
-};
-
-struct PeriodShared {
-  ListShared sh;
-  unsigned short wl[PMAX_CHUNKS];   // chunks waited for (not itself)
-  uint32_t cmask[2][CAND_WORDS];    // listed particles of steps of parity 0/1
-  long long s0;                     // first step of the period
-  int nwl;
-  int ok;
-};
-
-// All threads: true once every listed chunk has published progress >=
-// target; false (after recording the error) if the wait gave up.
-__device__ inline bool period_wait(PeriodShared& ps, const int* pflag, int target,
-                                   const PeriodArgs& p, ErrDev* err, long long step) {
-  if (threadIdx.x < 32) {
-    const int lane = threadIdx.x;
-    bool ok = true;
-    unsigned long long t0 = 0ull;
-    for (int b = 0; b < ps.nwl && ok; b += 32) {
-      const int c = b + lane < ps.nwl ? (int)ps.wl[b + lane] : -1;
-      for (;;) {
-        const int v = c >= 0 ? ld_poll(pflag + c * PFLAG_STRIDE) : target;
-        if (__all_sync(0xffffffffu, v - target >= 0)) break;
-        bool give_up = false;
-        if (lane == 0) {
-          const unsigned long long now = global_timer();
-          if (t0 == 0ull) t0 = now;
-          const int e = *(volatile int*)&err->code;
-          give_up = e != 0 || (long long)(now - t0) > p.wait_ns;
-          if (give_up && e == 0)
-            record_error(err, RDSIM_ERR_SYNC, (long long)blockIdx.x, -1, (double)target, step);
-        }
-        if (__shfl_sync(0xffffffffu, give_up, 0)) {
-          ok = false;
-          break;
-        }
-        if (RD_PERIOD_SLEEP_NS > 0) __nanosleep(RD_PERIOD_SLEEP_NS);
-      }
-    }
-    fence_acquire();
-    if (lane == 0) ps.ok = ok;
-  }
-  __syncthreads();
-  return ps.ok != 0;
-}
-
-// Publishes progress v of the CTA's chunk; the caller has synchronised the
-// CTA after its last write of the phase (the barrier orders the other
-// threads' writes before thread 0's release, which is cumulative).
-// RD_PERIOD_PUBLISH_FENCE adds a full fence before the release.
-#ifndef RD_PERIOD_PUBLISH_FENCE
-#define RD_PERIOD_PUBLISH_FENCE 0
-#endif
-__device__ inline void period_publish(int* pflag, int v, const PeriodArgs& p) {
-  if (threadIdx.x == 0 && (int)blockIdx.x != p.withhold) {
-    if (RD_PERIOD_PUBLISH_FENCE) __threadfence();
-    st_release(pflag + (size_t)blockIdx.x * PFLAG_STRIDE, v);
-  }
-}
-
-// The reaction draw of listed particle m by the calling warp (out of line:
-// rare, and its registers stay out of the drift's budget).
-template <int D, int TPP>
-__device__ __noinline__ void period_resolve(const ListShared& sh, const Args& r, int m, int lane) {
-  const int4 rec = make_int4(m, (int)r.meta[m], r.ncnt[m], r.pid[m]);
-  const int newt = resolve_listed<D, TPP>(sh.sys, sh.rx, r, rec, lane);
-  if (lane == 0) r.meta_out[m] = ((uint32_t)rec.y & 0xffffff00u) | (uint32_t)newt;
-}
-
-// Step n of the period on the CTA's chunk: d / r are the step arguments of
-// the drift and of the reactions (buffers of parity P = n & 1).
-template <int D, int TPP, int P>
-__device__ __forceinline__ bool period_run_step(PeriodShared& ps,
-                                                PeriodStage<LBLOCK / TPP>& st,
-                                                PeriodNbStage<D, LBLOCK / TPP>& ns,
-                                                float (*sacc)[LBLOCK / TPP],
-                                                const Args& d, const Args& r,
-                                                const PeriodArgs& p, const Chunk& ch, int n) {
-  const int tid = threadIdx.x, warp = tid >> 5, l32 = tid & 31;
-  const SysDev& s = ps.sh.sys;
-  const bool rx_next = p.rx && n + 1 < p.nsteps;
-  const bool words = rx_next || !(d.flags & F_NO_NOISE);
-  // the tail thread's own words and noise, while other chunks finish
-  if (tid < ch.cnt) {
-    const int ib = ch.beg + tid;
-#pragma unroll
-    for (int k = 0; k < D; k++) {
-      st.xh[k][tid] = d.xh[k][ib];
-      st.xl[k][tid] = d.xl[k][ib];
-    }
-    if (words) {
-      const U4 w0 = noise_words(s.seed, ps.s0 + n + 1, st.pid[tid], 0u);
-      st.w[0][tid] = w0.x;
-      st.w[1][tid] = w0.y;
-      st.w[2][tid] = w0.z;
-      st.w[3][tid] = w0.w;
-      if (!(d.flags & F_NO_NOISE)) {
-        float xi[3];
-        gaussians<D>(w0, xi);
-#pragma unroll
-        for (int k = 0; k < D; k++) st.xi[k][tid] = xi[k];
-      }
-    }
-  }
-  if (tid == 0) period_step = ps.s0 + n;
-  if (!period_wait(ps, d.pflag, n, p, d.err, ps.s0 + n)) return false;
-  // reactions of step n: the chunk's listed particles, a warp each
-  // (k_react_listed's resolution); their neighbours wait for the words
-  if (p.rx) {
-    uint32_t pend = 0u;
-#pragma unroll
-    for (int w = 0; w < CAND_WORDS; w++) pend |= ps.cmask[P][w];
-    if (pend) {
-      int k = 0;
-#pragma unroll 1
-      for (int w = 0; w < CAND_WORDS; w++) {
-        for (uint32_t b = ps.cmask[P][w]; b; b &= b - 1u, k++) {
-          if ((k & (LBLOCK / 32 - 1)) != warp) continue;
-          period_resolve<D, TPP>(ps.sh, r, ch.beg + w * 32 + __ffs(b) - 1, l32);
-        }
-      }
-      __syncthreads();
-    }
-  }
-  // drift of step n and the update of step n + 1 (k_force_l)
-  const int g = tid / TPP, lane = tid % TPP;
-  const bool active = g < ch.cnt;
-  const int i = ch.beg + (active ? g : 0);
-  const int cnt = d.ncnt[i];
-  uint32_t xo[3] = {0u, 0u, 0u};
-#pragma unroll
-  for (int k = 0; k < D; k++) xo[k] = d.xp[k][i];
-  const uint32_t mi = d.meta[i];
-  // the staged neighbours' words of this step, one coalesced pass
-  if (ns.on) {
-    for (int sl = tid; sl < ns.total; sl += LBLOCK) {
-      const int j = ns.g[sl];
-#pragma unroll
-      for (int k = 0; k < D; k++) ns.x[k][sl] = ldw(d, d.xp[k] + j);
-      ns.m[sl] = ldw(d, d.meta + j);
-    }
-    __syncthreads();
-  }
-  const bool staged = ns.on && active && cnt <= min(d.W, LS_MAX);
-  prefetch_rows<TPP>(d, ch, cnt, active && !staged);
-  float acc[3] = {0.f, 0.f, 0.f};
-  if (active && s.R2 > 0.f) {
-    if (staged) {
-      const int ti = mi & 0xff;
-      for (int e = lane; e < cnt; e += TPP) {
-        const unsigned int code = ns.slot[e][g];
-        const int sl = (int)(code & 0x7fffu);
-        Nb nb;
-#pragma unroll
-        for (int k = 0; k < 3; k++) nb.x[k] = k < D ? ns.x[k][sl] : 0u;
-        nb.m = ns.m[sl];
-        const int j = ns.g[sl];
-        if (nb.m & META_PENDING) nb.m = wait_final_meta(d, j, nb.m);
-        nb.v = (code & 0x8000u) ? (j | LIST_SAME_MOL) : j;
-        pair_term<D>(ps.sh, d, i, ti, xo, nb, acc);
-      }
-    } else {
-      pair_drift<D, TPP, true>(ps.sh, d, i, lane, cnt, xo, mi, acc);
-    }
-  }
-#pragma unroll
-  for (int o = TPP >> 1; o > 0; o >>= 1) {
-#pragma unroll
-    for (int k = 0; k < D; k++) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-  }
-  if (active && lane == 0) {
-#pragma unroll
-    for (int k = 0; k < D; k++) sacc[k][g] = acc[k];
-  }
-  __syncthreads();
-  const int ib = ch.beg + tid;
-  bool listed = false;
-  if (tid < ch.cnt) {
-    TailIn t;
-    float xi[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      t.xh[k] = k < D ? st.xh[k][tid] : 0u;
-      t.xl[k] = k < D ? st.xl[k][tid] : 0u;
-      t.xr[k] = k < D ? st.xr[k][tid] : 0u;
-      if (k < D && !(d.flags & F_NO_NOISE)) xi[k] = st.xi[k][tid];
-    }
-    t.xi = xi;
-    float accb[3] = {0.f, 0.f, 0.f};
-#pragma unroll
-    for (int k = 0; k < D; k++) accb[k] = sacc[k][tid];
-    const uint32_t mb = d.meta[ib];
-    const int pid = st.pid[tid];
-    U4 w0 = {0u, 0u, 0u, 0u};
-    if (words) w0 = U4{st.w[0][tid], st.w[1][tid], st.w[2][tid], st.w[3][tid]};
-    force_tail_in<D>(s, ps.sh.walls, d, ib, pid, t, mb, accb, words ? &w0 : nullptr);
-    if (rx_next) {
-      listed = rx_may_react<D>(s, (int)(mb & 0xff), d.ncnt[ib], pid, ps.s0 + n + 1, &w0);
-      // the next step's type word, marked while its draw is pending
-      d.meta_out[ib] = mb | (listed ? META_PENDING : 0u);
-    }
-  }
-  // the particles whose draw of step n + 1 may succeed: one word per warp
-  const unsigned int bal = __ballot_sync(0xffffffffu, listed);
-  if (l32 == 0 && warp < CAND_WORDS) ps.cmask[P ^ 1][warp] = rx_next ? bal : 0u;
-  __syncthreads();
-  period_publish(d.pflag, n + 1, p);
-  return true;
-}
-
-// Clears the pending marks that a period kernel stopped by an error leaves.
-static __global__ void k_clear_pending(uint32_t* m0, uint32_t* m1, int n) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) {
-    m0[i] &= ~META_PENDING;
-    m1[i] &= ~META_PENDING;
-  }
-}
-
-// Resident CTAs per SM the period kernel is compiled for: 7 x 152 SMs hold
-// the 1,024 chunks of 65,536 particles with 72 registers per thread.
-#ifndef RD_PERIOD_MIN_BLOCKS
-#define RD_PERIOD_MIN_BLOCKS 7
-#endif
-
-template <int D, int TPP>
-__global__ void __launch_bounds__(LBLOCK, RD_PERIOD_MIN_BLOCKS)
-    k_period(const __grid_constant__ Args d0, const __grid_constant__ Args d1,
-             const __grid_constant__ Args r0, const __grid_constant__ Args r1, PeriodArgs p) {
-  constexpr int PER = LBLOCK / TPP;
-  __shared__ PeriodShared ps;
-  __shared__ PeriodStage<PER> st;
-  __shared__ PeriodNbStage<D, PER> ns;
-  __shared__ float sacc[3][PER];
-  // No early launch of the next kernel: its CTAs must not take the SM slots
-  // that CTAs of this kernel still wait for.
-  const Chunk ch = chunk_at<PER>(d0, (int)blockIdx.x);
-  list_tables<true, true, true>(ps.sh, d0, ch);
-  pdl_wait();
-  const int tid = threadIdx.x;
-  const int g = tid / TPP, lane = tid % TPP;
-  const int i = ch.beg + (g < ch.cnt ? g : 0);
-  // every word the set-up reads (written by the list builder), issued
-  // together: one round trip instead of a chain
-  long long s0v = 0;
-  if (tid == 0) s0v = d0.step_base ? *d0.step_base + d0.step : d0.step;
-  uint32_t cw = 0u;
-  if (tid < CAND_WORDS && p.rx && p.first_rx) cw = d0.cand0[blockIdx.x * CAND_WORDS + tid];
-  int pidv = 0;
-  uint32_t xrv[3] = {0u, 0u, 0u};
-  if (tid < ch.cnt) {
-    pidv = d0.pid[ch.beg + tid];
-#pragma unroll
-    for (int k = 0; k < D; k++) xrv[k] = d0.xr[k][ch.beg + tid];
-  }
-  uint32_t bits[2] = {0u, 0u};
-  if (tid < 32) {
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int w = h * 32 + tid;
-      if (w < PMASK_WORDS) bits[h] = d0.nbmask[(size_t)blockIdx.x * PMASK_WORDS + w];
-    }
-  }
-  const int cnt = g < ch.cnt ? d0.ncnt[i] : 0;
-  // this lane's entries of the row (up to the staging width, whatever the
-  // count: the ELL array holds W entries per particle)
-  constexpr int EPL = (LS_MAX + TPP - 1) / TPP;
-  const int wmax = min(d0.W, LS_MAX);
-  int ent[EPL];
-#pragma unroll
-  for (int u = 0; u < EPL; u++) {
-    const int e = lane + u * TPP;
-    ent[u] = (g < ch.cnt && e < wmax) ? d0.nbr[ell_index<TPP>(e, i, d0.npad)] : 0;
-  }
-  if (tid == 0) {
-    ps.s0 = s0v;
-    if (blockIdx.x == 0) {
-      // the candidate lists of the per-step kernels stay empty
-      d0.rx_count[0] = 0;
-      d0.rx_count[1] = 0;
-      d0.rx_count[2] = 0;
-    }
-  }
-  if (tid < CAND_WORDS) {
-    ps.cmask[0][tid] = cw;
-    ps.cmask[1][tid] = 0u;
-  }
-  if (tid < ch.cnt) {  // static for the period
-    st.pid[tid] = pidv;
-#pragma unroll
-    for (int k = 0; k < D; k++) st.xr[k][tid] = xrv[k];
-  }
-  // the wait list: the bitmap's chunks other than this one, in order
-  if (tid < 32) {
-    int base = 0;
-#pragma unroll
-    for (int h = 0; h < 2; h++) {
-      const int w = h * 32 + tid;
-      uint32_t bw = bits[h];
-      if (w == (int)(blockIdx.x >> 5)) bw &= ~(1u << (blockIdx.x & 31));
-      const int cntw = __popc(bw);
-      int incl = cntw;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int v = __shfl_up_sync(0xffffffffu, incl, o);
-        if (tid >= o) incl += v;
-      }
-      int pos = base + incl - cntw;
-      for (uint32_t b = bw; b; b &= b - 1u) ps.wl[pos++] = (unsigned short)(w * 32 + __ffs(b) - 1);
-      base += __shfl_sync(0xffffffffu, incl, 31);
-    }
-    if (tid == 0) ps.nwl = base;
-  }
-  __syncthreads();
-  // the neighbour staging table (PeriodNbStage)
-  {
-    const int self = (int)blockIdx.x;
-    const int nwl = ps.nwl;
-    const int on0 = nwl + 1 <= STAGE_CH ? 1 : 0;
-    // the waited chunks and this one, in order (warp 0; ps.wl is sorted)
-    if (tid < 32) {
-      if (on0) {
-        int below = 0;
-        for (int q = tid; q < nwl; q += 32) {
-          const int c = ps.wl[q];
-          below += c < self ? 1 : 0;
-          ns.ch[q + (c > self ? 1 : 0)] = (unsigned short)c;
-        }
-        below = __reduce_add_sync(0xffffffffu, below);
-        if (tid == 0) ns.ch[below] = (unsigned short)self;
-      }
-      if (tid == 0) {
-        ns.on = on0;
-        ns.nch = on0 ? nwl + 1 : 0;
-        ns.total = 0;
-      }
-    }
-    for (int q = tid; q < STAGE_CH; q += LBLOCK) {
-      ns.lo[q] = 0x7fffffff;
-      ns.hi[q] = -1;
-    }
-    const SysDev& s = ps.sh.sys;
-    const int chunk0 = (int)blockIdx.x - (ch.beg - s.p0) / PER;
-    const bool mine = on0 && g < ch.cnt && cnt <= wmax;
-    __syncthreads();
-    // position of the chunk of sorted particle j in ns.ch (-1: absent)
-    auto pos_of = [&](int j) {
-      const int h = chunk0 + (j - s.p0) / PER;
-      int lo = 0, hi = ns.nch - 1;
-      while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if ((int)ns.ch[mid] < h) lo = mid + 1;
-        else hi = mid;
-      }
-      return (int)ns.ch[lo] == h ? lo : -1;
-    };
-    if (mine) {
-#pragma unroll
-      for (int u = 0; u < EPL; u++) {
-        if (lane + u * TPP >= cnt) break;
-        const int j = ent[u] & 0x7fffffff;
-        const int q = pos_of(j);
-        if (q < 0) {
-          ns.on = 0;
-          continue;
-        }
-        atomicMin(&ns.lo[q], j);
-        atomicMax(&ns.hi[q], j);
-      }
-    }
-    __syncthreads();
-    // run lengths -> bases (warp 0, shuffle scan over at most STAGE_CH runs)
-    if (tid < 32 && ns.on) {
-      const int n = ns.nch;
-      int carry = 0;
-      for (int q0 = 0; q0 < n; q0 += 32) {
-        const int q = q0 + tid;
-        const int len = (q < n && ns.hi[q] >= ns.lo[q]) ? ns.hi[q] - ns.lo[q] + 1 : 0;
-        int incl = len;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, incl, o);
-          if (tid >= o) incl += v;
-        }
-        if (q < n) ns.base[q] = carry + incl - len;
-        carry += __shfl_sync(0xffffffffu, incl, 31);
-      }
-      if (tid == 0) {
-        ns.base[n] = carry;
-        ns.total = carry;
-        if (carry > PeriodNbStage<D, PER>::SMAX) ns.on = 0;
-      }
-    }
-    __syncthreads();
-    if (ns.on) {
-      for (int sl = tid; sl < ns.total; sl += LBLOCK) {
-        int lo = 0, hi = ns.nch - 1;  // the last run starting at or before sl
-        while (lo < hi) {
-          const int mid = (lo + hi + 1) >> 1;
-          if (ns.base[mid] <= sl) lo = mid;
-          else hi = mid - 1;
-        }
-        ns.g[sl] = ns.lo[lo] + (sl - ns.base[lo]);
-      }
-      if (mine) {
-#pragma unroll
-        for (int u = 0; u < EPL; u++) {
-          const int e = lane + u * TPP;
-          if (e >= cnt) break;
-          const int v = ent[u];
-          const int j = v & 0x7fffffff;
-          const int q = pos_of(j);
-          const int sl = ns.base[q] + (j - ns.lo[q]);
-          ns.slot[e][g] = (unsigned short)(sl | (v < 0 ? 0x8000 : 0));
-        }
-      }
-    }
-    __syncthreads();
-  }
-  const long long slot = d0.stamps ? (ps.s0 / p.nsteps) % d0.stamp_ring : 0;
-  if (d0.stamps && tid == 0)
-    d0.stamps[((size_t)slot * gridDim.x + blockIdx.x) * 2] = global_timer();
-  for (int n = 0; n < p.nsteps; n += 2) {
-    if (!period_run_step<D, TPP, 0>(ps, st, ns, sacc, d0, r0, p, ch, n)) return;
-    if (n + 1 < p.nsteps && !period_run_step<D, TPP, 1>(ps, st, ns, sacc, d1, r1, p, ch, n + 1))
-      return;
-  }
-  if (d0.stamps && (tid & 31) == 0)
-    atomicMax(d0.stamps + ((size_t)slot * gridDim.x + blockIdx.x) * 2 + 1, global_timer());
 }
 
 }  // namespace rd

@@ -154,3 +154,54 @@ def test_period_kernel_fallbacks_are_exact():
         np.testing.assert_array_equal(ta, tb)
         np.testing.assert_array_equal(xa, xb)
     np.testing.assert_array_equal(one.drift(), per_step.drift())
+
+
+@pytest.mark.parametrize("n", [2, 15, 17, 1000, 14593, 29191, 30011])
+def test_period_lanes_and_frames(n):
+    """The period kernel's lanes per chain follow the number of particles (4,
+    2 and 1 here); launches also end before trajectory frames and the call's
+    last step.  Positions, types, frames and drifts equal the per-step
+    kernels' bit for bit at every size, with ragged last chunks and calls that
+    start and end inside list periods."""
+    from pyrdsim_gb300 import workloads
+    # (a handful of particles at the fluid's density would fill a box smaller
+    # than the interaction range)
+    sd = workloads.active_wall_fluid(n=n, rho=0.4 if n >= 1000 else 0.02, seed=n, k_on=20.0,
+                                     k_off=50.0)
+    one = _engine([sd])
+    per_step = _engine([sd], period_kernel=False)
+    assert one.info()["period_kernel"] == 1
+    for e in (one, per_step):
+        e.set_trajectory(7, 6)
+    for k in (3, 44, 1, 2, 25):
+        one.step(k)
+        per_step.step(k)
+        for a, b in zip(one.state() + one.trajectory(), per_step.state() + per_step.trajectory()):
+            np.testing.assert_array_equal(a, b)
+    np.testing.assert_array_equal(one.drift(), per_step.drift())
+    np.testing.assert_array_equal(one.reaction_rates(), per_step.reaction_rates())
+
+
+@pytest.mark.parametrize("n", [1, 63, 65, 4099])
+def test_lj_walk_equals_the_general_walk(n):
+    """A system whose pair laws are all Lennard-Jones n = 6 takes the drift
+    kernel's Lennard-Jones walk; adding a law between types that no particle
+    has sends it through the general one.  Drifts and states are the same bit
+    for bit, with rows within and beyond the stored list width."""
+    from pyrdsim_gb300 import model, workloads
+    sd = workloads.inhibited_mixture(n=n, seed=n, rho=0.45 if n >= 1000 else 0.02)
+    m = sd.model
+    p = dict(m.parameters)
+    p["tau_by_taud"] = np.ones(4)
+    p["interactions"] = list(m.interactions) + [
+        {"type": "yukawa", "pair": [3, 3], "u0": 1.0, "r0": 0.5, "rc": 1.1}]
+    general = model.SystemData(model.Model.from_dict(p), sd.x, sd.types, sd.molecule_ids,
+                               sd.first_index)
+    for width in (0, 8):
+        es = [_engine([s], period_kernel=False, list_width=width) for s in (sd, general)]
+        for k in (1, 30):
+            for e in es:
+                e.step(k)
+            for a, b in zip(es[0].state(), es[1].state()):
+                np.testing.assert_array_equal(a, b)
+            np.testing.assert_array_equal(es[0].drift(), es[1].drift())
