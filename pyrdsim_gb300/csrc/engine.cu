@@ -161,6 +161,9 @@ struct rdsim_handle {
   float* drift[3] = {};
   // float64 force mode (force64.cuh)
   bool f64 = false;
+  int fpw = 2;                         // particles per warp of its drift kernel
+  unsigned fchunks = 0;                // its CTAs
+  Chunk* fchunks_d = nullptr;
   double* drift_d[3] = {};
   double* typed_d = nullptr;           // [nsys][2][MAXT]: dt D, sqrt(2 dt D)
   double* rates = nullptr;
@@ -434,8 +437,11 @@ int force(rdsim_handle* h, long long step, int flags, const double* xi_next, boo
   a.xi = xi_next;
   {
     ProfScope ps(h, P_FORCE, 1);
-    if (h->f64) CK(launch_force64(h->D, h->ltpp, (unsigned)h->chunks_h.size(), h->stream, a));
-    else CK(launch_force32(h->D, h->ltpp, h->all_lj6, (unsigned)h->chunks_h.size(), h->stream, a));
+    if (h->f64) {
+      a.chunks = h->fchunks_d;
+      CK(launch_force64(h->D, h->ltpp, h->fpw, h->fchunks, h->stream, a));
+    }
+    if (!h->f64) CK(launch_force32(h->D, h->ltpp, h->all_lj6, (unsigned)h->chunks_h.size(), h->stream, a));
   }
   CK(cudaGetLastError());
   if (flags & F_EM) h->cx = 1 - h->cx;
@@ -687,7 +693,7 @@ void free_all(rdsim_handle* h) {
   F(h->sys_d); F(h->laws_d); F(h->walls_d); F(h->rx_d); F(h->tmpl_d);
   F(h->terms_d); F(h->atomterm_d); F(h->cell_count); F(h->cell_start); F(h->bsum);
   F(h->cell_of); F(h->rank_of); F(h->tmp); F(h->sid); F(h->slot_of);
-  F(h->chunks_d); F(h->pchunks_d); F(h->nbr); F(h->ncnt); F(h->rcnt); F(h->rx_list); F(h->rx_count);
+  F(h->chunks_d); F(h->pchunks_d); F(h->fchunks_d); F(h->nbr); F(h->ncnt); F(h->rcnt); F(h->rx_list); F(h->rx_count);
   F(h->stg_n); F(h->stg_g); F(h->codes);
   for (int b = 0; b < 2; b++) { F(h->rec[b]); F(h->recl[b]); F(h->rech[b]); }
   for (int b = 0; b < 2; b++) {
@@ -1473,6 +1479,13 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
       }
     }
   }
+  std::vector<Chunk> fchunks;
+  if (h->f64) {
+    h->fpw = force64_particles(N);
+    fchunks = make_chunks(h->sys_h, force64_chunk(h->fpw));
+    h->fchunks = (unsigned)fchunks.size();
+    if ((rc = dalloc(&h->fchunks_d, fchunks.size(), &B))) return bail(rc);
+  }
   if ((rc = dalloc(&h->cl_d, (size_t)3 * h->nsys, &B))) return bail(rc);
   auto up = [&](void* d, const void* s, size_t bytes) -> int {
     if (bytes == 0) return 0;
@@ -1485,6 +1498,7 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
   if ((rc = up(h->sys_d, h->sys_h.data(), sizeof(SysDev) * h->sys_h.size()))) return bail(rc);
   if ((rc = up(h->chunks_d, h->chunks_h.data(), sizeof(Chunk) * h->chunks_h.size())))
     return bail(rc);
+  if ((rc = up(h->fchunks_d, fchunks.data(), sizeof(Chunk) * fchunks.size()))) return bail(rc);
   if ((rc = up(h->pchunks_d, h->pchunks_h.data(), sizeof(Chunk) * h->pchunks_h.size())))
     return bail(rc);
   if ((rc = up(h->laws_d, laws.data(), sizeof(PairLaw) * laws.size()))) return bail(rc);

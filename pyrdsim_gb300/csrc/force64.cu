@@ -7,18 +7,28 @@
 
 namespace rd {
 
-template <int D>
-static void launch_force64_d(int tpp, unsigned grid, cudaStream_t st, const Args& a) {
-  if (tpp == 1) launch(k_force_d<D, 1>, grid, LBLOCK, st, a);
-  else if (tpp == 2) launch(k_force_d<D, 2>, grid, LBLOCK, st, a);
-  else if (tpp == 8) launch(k_force_d<D, 8>, grid, LBLOCK, st, a);
-  else launch(k_force_d<D, 4>, grid, LBLOCK, st, a);
+namespace {
+
+typedef void (*ForceKernel)(Args);
+
+template <int D, int TPP>
+ForceKernel kernel_of(int pw) {
+  return pw == 2 ? k_force_d<D, TPP, 2> : pw == 4 ? k_force_d<D, TPP, 4> : k_force_d<D, TPP, 16>;
 }
 
-cudaError_t launch_force64(int D, int tpp, unsigned grid, cudaStream_t st, const Args& a) {
-  if (D == 2) launch_force64_d<2>(tpp, grid, st, a);
-  else if (D == 3) launch_force64_d<3>(tpp, grid, st, a);
-  else launch_force64_d<1>(tpp, grid, st, a);
+template <int D>
+ForceKernel kernel_of(int tpp, int pw) {
+  return tpp == 1   ? kernel_of<D, 1>(pw)
+         : tpp == 2 ? kernel_of<D, 2>(pw)
+         : tpp == 8 ? kernel_of<D, 8>(pw)
+                    : kernel_of<D, 4>(pw);
+}
+
+}  // namespace
+
+cudaError_t launch_force64(int D, int tpp, int pw, unsigned grid, cudaStream_t st, const Args& a) {
+  launch(D == 2 ? kernel_of<2>(tpp, pw) : D == 3 ? kernel_of<3>(tpp, pw) : kernel_of<1>(tpp, pw),
+         grid, LBLOCK, st, a);
   return cudaGetLastError();
 }
 

@@ -2,10 +2,10 @@
 // (pyrdsim.pyx:1941-2067 with the laws of 1068-1145, the EM update of
 // 2225-2250), for the "plain method" that wants float64 forces.
 //
-// Same structure as k_force_l (list.cuh): a CTA per run of particles, TPP
-// lanes per particle walking its Verlet-list row, then one thread per
-// particle for walls, bonded terms, the drift store and the fused
-// Euler-Maruyama update.  Differences: pair displacements are the full 64-bit
+// A CTA per run of particles; its warps sum the pair drift of their particles
+// (k_force_d), then one thread per particle adds walls and bonded terms, stores
+// the drift and performs the fused Euler-Maruyama update.  Differences to
+// k_force_l (list.cuh): pair displacements are the full 64-bit
 // fixed-point differences converted to float64 (exact to the double's 53
 // bits); the laws, walls and bonded terms are evaluated in float64 from the
 // deck's float64 parameters with the reference's formulas (angles by acos
@@ -41,31 +41,6 @@ __device__ inline NbF gather_full(const Args& a, int v) {
   return n;
 }
 
-// for_entries (list.cuh) with full-word gathers.
-template <int D, int TPP, class Fn>
-__device__ inline void for_entries_full(const SysDev& s, const Args& a, int i, int lane, int cnt,
-                                        Fn&& fn) {
-  constexpr int B = RD_LIST_BATCH;
-  if (cnt <= a.W) {
-    for (int e0 = lane; e0 < cnt; e0 += B * TPP) {
-      int v[B];
-#pragma unroll
-      for (int u = 0; u < B; u++) {
-        const int e = e0 + u * TPP;
-        v[u] = e < cnt ? a.nbr[ell_index<TPP>(e, i, a.npad)] : i;
-      }
-      NbF nb[B];
-#pragma unroll
-      for (int u = 0; u < B; u++) nb[u] = gather_full<D>(a, v[u]);
-#pragma unroll
-      for (int u = 0; u < B; u++)
-        if (e0 + u * TPP < cnt) fn(nb[u]);
-    }
-  } else {
-    row_scan<D, TPP>(s, a, i, lane, [&](int, int v) { fn(gather_full<D>(a, v)); });
-  }
-}
-
 __device__ inline unsigned long long fixed_word(uint32_t h, uint32_t l) {
   return ((unsigned long long)h << 32) | l;
 }
@@ -80,24 +55,33 @@ __device__ inline double disp_d(const SysDev& s, const Args& a, int k, int gi, i
 
 // f / r of one law at squared distance r2 in float64 (pyrdsim.pyx:1068-1130).
 __device__ inline double law_over_r_d(const rdsim_interaction& O, double r2) {
-  const double r = sqrt(r2);
   switch (O.law) {
     case RDSIM_LAW_LJ: {  // f = -2 n u0 / r * s (s - 1), s = (r0/r)^n
+      if ((O.n & 1) == 0) {  // even powers: one division, no root
+        const double w = 1.0 / r2, q = O.r0 * O.r0 * w;
+        double sn = q;
+        for (int e = 2; e < O.n; e += 2) sn *= q;
+        return -2.0 * O.n * O.u0 * sn * (sn - 1.0) * w;
+      }
+      const double r = sqrt(r2);
       const double b = O.r0 / r;
       double sn = 1.0;
       for (int e = 0; e < O.n; e++) sn *= b;
       return -2.0 * O.n * O.u0 / r * sn * (sn - 1.0) / r;
     }
     case RDSIM_LAW_TANH: {  // f = u0 (1 - tanh^2((r - r0)/a)) / (2a)
+      const double r = sqrt(r2);
       const double t = tanh((r - O.r0) / O.a);
       return O.u0 * (1.0 - t * t) / O.a / 2.0 / r;
     }
-    case RDSIM_LAW_YUKAWA:  // f = -u0 (1 + r0/r) exp(-r/r0) / (r r0)
+    case RDSIM_LAW_YUKAWA: {  // f = -u0 (1 + r0/r) exp(-r/r0) / (r r0)
+      const double r = sqrt(r2);
       return -O.u0 * (1.0 + O.r0 / r) * exp(-r / O.r0) / (r * O.r0) / r;
+    }
     case RDSIM_LAW_HARMONIC:  // f = u0 r
       return O.u0;
     case RDSIM_LAW_PIECEWISE_LINEAR:  // f = u0/dr for r >= r0 - dr (checked by the caller)
-      return O.u0 / O.dr / r;
+      return O.u0 / O.dr / sqrt(r2);
   }
   return 0.0;
 }
@@ -289,20 +273,58 @@ __device__ inline void force_tail_d(const SysDev& s, const WallLaw* walls,
   if (a.flags & F_EM) em_update_d<D>(s, a, sysi, gi, pid, ti, acc, eff_em_step(a), a.flags, w0);
 }
 
-// Drift kernel in float64.  Phase A: TPP lanes per particle sum the pair
-// drift over its list entries; phase B: one thread per particle.
-template <int D, int TPP>
+// Drift kernel in float64.  The float64 pipe bounds it (16 cycles per warp
+// instruction and SM, whatever the number of active lanes), so its lanes see
+// only pairs that can be in range, side by side: the warp's lanes, 32 / PW per
+// particle, screen the list entries of its PW particles in float32 (pair words
+// against the guarded cutoffs) and queue the survivors; 32 of them at a time
+// are evaluated with every lane busy, and the terms are added in list order,
+// one running sum per chain (entries e = c mod TPP) and dimension, so that the
+// sums do not depend on PW.  PW is small in small systems, which then use more
+// SMs (force64_particles).  LJ fluid, us per step (rebuilds included): 32.4 ->
+// 11.8 at 1,024 particles, 103 -> 39 at 16,384, 201 -> 101 at 65,536, against two
+// lanes per particle walking their rows (at 1,024, 64 of 608 SM partitions at
+// work).
+template <int D, int TPP, int PW>
+struct ForceQueue {
+  static constexpr int CAP = 128 / (PW * TPP) < 32 ? 128 / (PW * TPP) : 32;  // terms per chain
+  static constexpr int SLOTS = PW * TPP * CAP;
+  double fr[SLOTS], dx[D][SLOTS];
+  double acc[PW * TPP][D];
+  int j[SLOTS];
+  unsigned short slot[SLOTS];
+  int n[PW * TPP];
+};
+
+// f / r of the pair (gi, gj) of full words and its displacement.
+template <int D>
+__device__ inline double pair_term_d(const ListShared& sh, const rdsim_interaction* olaw,
+                                     const Args& a, int gi, int ti, int gj, double* dx) {
+  const SysDev& s = sh.sys;
+  double r2 = 0.0;
+#pragma unroll
+  for (int k = 0; k < D; k++) {
+    dx[k] = __ll2double_rn((long long)(fixed_word(a.xh[k][gj], a.xl[k][gj]) -
+                                       fixed_word(a.xh[k][gi], a.xl[k][gi]))) * s.unit_d[k];
+    r2 += dx[k] * dx[k];
+  }
+  const int tj = a.meta[gj] & 0xff;
+  if (!(r2 < (double)s.prc2[ti * MAXT + tj])) return 0.0;  // beyond every law of the pair
+  return pair_force_d<D>(s, sh.laws, olaw, a, gi, gj, s.ppair[ti * MAXT + tj], r2);
+}
+
+template <int D, int TPP, int PW>
 __global__ void __launch_bounds__(LBLOCK) k_force_d(Args a) {
-  constexpr int PER = LBLOCK / TPP;
+  constexpr int PER = LBLOCK / 32 * PW, LPP = 32 / PW;
   constexpr int NO = MAXI * (int)(sizeof(rdsim_interaction) / 4);
+  typedef ForceQueue<D, TPP, PW> Queue;
+  constexpr int CAP = Queue::CAP;
   __shared__ ListShared sh;
   __shared__ rdsim_interaction olaw[MAXI];
-  __shared__ double sacc[3][PER];
+  __shared__ Queue queue[LBLOCK / 32];
   pdl_trigger();
   const Chunk ch = chunk_of<PER>(a);
-  const int tid = threadIdx.x, g = tid / TPP, lane = tid % TPP;
-  const bool active = g < ch.cnt;
-  const int i = ch.beg + (active ? g : 0);
+  const int tid = threadIdx.x, warp = tid >> 5, l32 = tid & 31;
   {
     WordLoad<NO> lo;
     const int no = ch.nlaws * (int)(sizeof(rdsim_interaction) / 4);
@@ -310,42 +332,95 @@ __global__ void __launch_bounds__(LBLOCK) k_force_d(Args a) {
     list_tables<true, true, false>(sh, a, ch);
     lo.store(reinterpret_cast<int*>(olaw), no);
   }
-  pdl_wait();
-  const int cnt = a.ncnt[i];
-  unsigned long long Xo[3] = {0ull, 0ull, 0ull};
+  Queue& fq = queue[warp];
+  for (int q = l32; q < PW * TPP; q += 32) {
+    fq.n[q] = 0;
 #pragma unroll
-  for (int k = 0; k < D; k++) Xo[k] = fixed_word(a.xh[k][i], a.xl[k][i]);
-  const uint32_t mi = a.meta[i];
-  prefetch_rows<TPP>(a, ch, cnt, active);
+    for (int k = 0; k < D; k++) fq.acc[q][k] = 0.0;
+  }
+  pdl_wait();
+  const int p = l32 / LPP, sub = l32 % LPP, g = warp * PW + p;
+  const bool active = g < ch.cnt;
+  const int i = ch.beg + (active ? g : 0), i0 = ch.beg + warp * PW;
+  const int cnt = active ? a.ncnt[i] : 0;
+  uint32_t xo[3] = {0u, 0u, 0u};
+#pragma unroll
+  for (int k = 0; k < D; k++) xo[k] = a.xp[k][i];
+  const int ti = (int)(a.meta[i] & 0xffu);
   __syncthreads();
   const SysDev& s = sh.sys;
-  double acc[3] = {0.0, 0.0, 0.0};
-  if (active && s.R2 > 0.f) {
-    const int ti = mi & 0xff;
-    for_entries_full<D, TPP>(s, a, i, lane, cnt, [&](const NbF& nb) {
-      if (nb.v < 0) return;  // same molecule: reactions only
-      double dx[3], r2 = 0.0;
+  if (s.R2 > 0.f) {
+    int queued = 0;  // the same on every lane
+    auto flush = [&] {
+      __syncwarp();
+      for (int q = l32; q < queued; q += 32) {
+        const int slot = fq.slot[q], gi = i0 + slot / (TPP * CAP);
+        double dx[3];
+        fq.fr[slot] = pair_term_d<D>(sh, olaw, a, gi, (int)(a.meta[gi] & 0xffu), fq.j[q], dx);
 #pragma unroll
-      for (int k = 0; k < D; k++) {
-        dx[k] = __ll2double_rn((long long)(fixed_word(nb.h[k], nb.l[k]) - Xo[k])) * s.unit_d[k];
-        r2 += dx[k] * dx[k];
+        for (int k = 0; k < D; k++) fq.dx[k][slot] = dx[k];
       }
-      const int tj = nb.m & 0xff;
-      if (!(r2 < (double)s.prc2[ti * MAXT + tj])) return;  // beyond every law of the pair
-      const unsigned int pp = s.ppair[ti * MAXT + tj];
-      const double fr = pair_force_d<D>(s, sh.laws, olaw, a, i, nb.v, pp, r2);
+      __syncwarp();
+      for (int q = l32; q < PW * TPP * D; q += 32) {
+        const int c = q / D, k = q % D, n = fq.n[c];
+        double v = fq.acc[c][k];
+        for (int t = 0; t < n; t++) v += fq.fr[c * CAP + t] * fq.dx[k][c * CAP + t];
+        fq.acc[c][k] = v;
+      }
+      __syncwarp();
+      for (int q = l32; q < PW * TPP; q += 32) fq.n[q] = 0;
+      queued = 0;
+      __syncwarp();
+    };
+    const int row = cnt <= a.W ? cnt : 0;
+    const int rounds = (__reduce_max_sync(0xffffffffu, row) + LPP - 1) / LPP;
+    // lanes of this lane's particle that take entries of its chain
+    unsigned int peers = 0u;
 #pragma unroll
-      for (int k = 0; k < D; k++) acc[k] += fr * dx[k];
-    });
-  }
+    for (int q = 0; q < LPP; q++)
+      if (q % TPP == sub % TPP) peers |= 1u << (p * LPP + q);
+    int v = sub < row ? a.nbr[ell_index<TPP>(sub, i, a.npad)] : (i | LIST_SAME_MOL);
+    for (int r = 0; r < rounds; r++) {
+      const int e = r * LPP + sub, next = e + LPP;
+      const Nb nb = gather<D>(a, v);
+      v = next < row ? a.nbr[ell_index<TPP>(next, i, a.npad)] : (i | LIST_SAME_MOL);
+      float d[3];
+      const bool hit = nb.v >= 0 && pair_geom<D>(s, nb.x, xo, d) < s.prc2[ti * MAXT + (nb.m & 0xffu)];
+      const unsigned int m = __ballot_sync(0xffffffffu, hit), mine = m & peers;
+      const unsigned int below = (1u << l32) - 1u;
+      const int c = p * TPP + e % TPP, n = fq.n[c];
+      __syncwarp();
+      if (hit) {
+        const int q = queued + __popc(m & below);
+        fq.j[q] = nb.v;
+        fq.slot[q] = (unsigned short)(c * CAP + n + __popc(mine & below));
+      }
+      // (lanes without peers below them: one per chain)
+      if (!(peers & below)) fq.n[c] = n + __popc(mine);
+      queued += __popc(m);
+      __syncwarp();
+      // room for another round in every chain
+      if (__any_sync(0xffffffffu, fq.n[c] > CAP - (LPP + TPP - 1) / TPP)) flush();
+    }
+    flush();
+    // rows beyond the stored width, regenerated from the cells by TPP lanes
+    for (unsigned int big = __ballot_sync(0xffffffffu, sub == 0 && cnt > a.W); big; big &= big - 1u) {
+      const int pb = (__ffs(big) - 1) / LPP, gi = i0 + pb;
+      if (l32 < TPP) {
+        double acc[3] = {0.0, 0.0, 0.0};
+        const int tb = (int)(a.meta[gi] & 0xffu);
+        row_scan<D, TPP>(s, a, gi, l32, [&](int, int ent) {
+          if (ent < 0) return;
+          double dx[3];
+          const double fr = pair_term_d<D>(sh, olaw, a, gi, tb, ent, dx);
 #pragma unroll
-  for (int o = TPP >> 1; o > 0; o >>= 1) {
+          for (int k = 0; k < D; k++) acc[k] += fr * dx[k];
+        });
 #pragma unroll
-    for (int k = 0; k < D; k++) acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-  }
-  if (active && lane == 0) {
-#pragma unroll
-    for (int k = 0; k < D; k++) sacc[k][g] = acc[k];
+        for (int k = 0; k < D; k++) fq.acc[pb * TPP + l32][k] = acc[k];
+      }
+      __syncwarp();
+    }
   }
   __syncthreads();
   const int ib = ch.beg + tid;
@@ -357,7 +432,16 @@ __global__ void __launch_bounds__(LBLOCK) k_force_d(Args a) {
     for (int k = 0; k < D; k++) xb[k] = a.xh[k][ib];
     double accb[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-    for (int k = 0; k < D; k++) accb[k] = sacc[k][tid];
+    for (int k = 0; k < D; k++) {  // the chains' sums, as a xor tree adds them
+      double c[TPP];
+#pragma unroll
+      for (int q = 0; q < TPP; q++) c[q] = queue[tid / PW].acc[tid % PW * TPP + q][k];
+#pragma unroll
+      for (int o = TPP >> 1; o > 0; o >>= 1)
+#pragma unroll
+        for (int q = 0; q < o; q++) c[q] += c[q + o];
+      accb[k] = c[0];
+    }
     const uint32_t mb = a.meta[ib];
     const int pid = a.pid[ib];
     const bool words = (a.flags & F_RX_NEXT) ||
