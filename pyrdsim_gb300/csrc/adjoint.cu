@@ -6,9 +6,11 @@
 // in index order) and gets a neighbour list: the particles of the 3^D
 // cells around each particle that pass a float32 distance screen, in a fixed
 // order, so all sums run in a fixed order and results are deterministic.
-// The float64 kernels walk the lists with four lanes per particle: float64
-// issue is scarce on this GPU (1/64 of float32), and a compact list keeps
-// the lanes of a warp busy with pairs inside the cutoff.  Forward (k_adj_step): pair drift of pyrdsim.pyx:1941-2067 for
+// Float64 issue is scarce on this GPU (a warp instruction every 16 cycles per
+// SM, however few lanes are active), so the float64 kernels screen the list
+// entries in float32 first, queue the pairs inside a law's cutoff by kind of
+// law, and evaluate 32 of a kind at a time (see PairQueue).  Forward
+// (k_adj_step): pair drift of pyrdsim.pyx:1941-2067 for
 // Lennard-Jones and Yukawa laws (pyrdsim.pyx:1068-1130), the loss terms of
 // the state, and the Euler-Maruyama update with injected noise and periodic
 // wrap (pyrdsim.pyx:2225-2292).  Backward (k_adj_back): for state x_n and
@@ -25,6 +27,7 @@
 #include <cmath>
 #include <cstring>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "../../include/rdsim_adjoint.h"
@@ -55,6 +58,9 @@ struct Law {
   int law, n;
   double u0, r0, rc, ir0;       // ir0 = 1 / r0
   double Uc, dUc_du0, dUc_dr0;  // energy at rc and its parameter derivatives
+  double r02, rc2;              // r0^2, rc^2
+  float screen2;                // float32 screen: above rc^2
+  int pad;
 };
 
 struct AdjArgs {
@@ -62,7 +68,7 @@ struct AdjArgs {
   int nc[3], ncell;
   double L[3], cellinv[3];
   float Lf[3], Linvf[3];
-  double rc2max;                // largest law cutoff^2: list entries beyond skip
+  int exact_image;              // boxes near 2 rc: float64 decides the image
   float cut2f;                  // float32 screen of the list in use
   float move2f;                 // displacement^2 allowed while a list is reused                  // float32 screen: above the largest rc^2
   double c[MAXT], s[MAXT];      // dt D and sqrt(2 dt D) per type
@@ -222,7 +228,7 @@ __global__ void k_cell_sort(int ncell, const double* __restrict__ x,
 // includes twice the allowed displacement).  TPP lanes per particle i: lane l takes the
 // members l, l + TPP, ... of each of the 3^D cells around i's cell (cells in
 // a fixed order, members in index order) that pass the float32 distance
-// screen and keeps them in its own sub-list nbr[(e * TPP + l) * N + i],
+// screen and keeps them in its own sub-list nbr[(i * TPP + l) * W + e],
 // e < min(count, W); ncnt[l * N + i] = count.  maxcnt receives the largest
 // count (the caller enlarges W and repeats when it exceeds W).
 template <int D>
@@ -277,7 +283,7 @@ __global__ void __launch_bounds__(BLK) k_adj_list(AdjArgs g, const double* __res
             if (r2f > g.cut2f) continue;
             const int j = idx[p];
             if (j == i) continue;
-            if (cnt < W) nbr[((size_t)cnt * TPP + lane) * g.N + i] = j;
+            if (cnt < W) nbr[((size_t)i * TPP + lane) * W + cnt] = j;
             cnt++;
           }
         }
@@ -291,38 +297,243 @@ __global__ void __launch_bounds__(BLK) k_adj_list(AdjArgs g, const double* __res
   if ((threadIdx.x & 31) == 0 && m > 0) atomicMax(maxcnt, m);
 }
 
-// Visit, on lane `lane` of the TPP lanes of particle i, the entries of its
-// sub-list, with the float64 minimum-image vector d = x_j - x_i.
-template <int D, class Fn>
-__device__ inline void for_list(const AdjArgs& g, const double* __restrict__ x,
-                                const int* __restrict__ nbr, const int* __restrict__ ncnt, int W,
-                                int i, const double* xi, int lane, Fn&& fn) {
-  const int cnt = min(ncnt[(size_t)lane * g.N + i], W);
-  for (int e = 0; e < cnt; e++) {
-    const int j = nbr[((size_t)e * TPP + lane) * g.N + i];
-    double d[3] = {0.0, 0.0, 0.0};
-#pragma unroll
-    for (int k = 0; k < D; k++) {
-      double v = x[(size_t)j * D + k] - xi[k];
-      // minimum image; rint(v / L) is 0 whenever |v| < 0.49 L
-      if (!(fabs(v) < 0.49 * g.L[k])) v -= g.L[k] * rint(v / g.L[k]);
-      d[k] = v;
-    }
-    fn(j, d);
+// Float32 value of a coordinate from the high word of its float64 (20 bits of
+// the significand; Law::screen2 allows for what that leaves out);
+// coordinates far outside the box are wrapped first.
+__device__ inline float screen_coord(const AdjArgs& g, int k, const double* p) {
+  const uint32_t h = reinterpret_cast<const uint32_t*>(p)[1];
+  const uint32_t m = h & 0x7fffffffu;
+  const float v = __uint_as_float((m < (897u << 20) ? 0u : (m - (896u << 20)) << 3) | (h & 0x80000000u));
+  if (!(fabsf(v) <= 2.f * g.Lf[k])) {
+    const double x = *p;
+    return (float)(x - g.L[k] * floor(x / g.L[k]));
   }
-}
-
-// Sum over the TPP lanes of one particle (xor tree: the same order on every
-// lane, so all lanes hold the same value).
-__device__ inline double lane_sum(double v) {
-#pragma unroll
-  for (int o = 1; o < TPP; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
+// 1 / r2 to within about one ulp: the float32 reciprocal and two Newton steps.
+__device__ inline double recip_d(double r2) {
+  const float f = (float)r2;
+  if (!(f > 1e-30f && f < 1e30f)) return 1.0 / r2;
+  double w = (double)(1.0f / f);
+  w = fma(w, fma(-r2, w, 1.0), w);
+  return fma(w, fma(-r2, w, 1.0), w);
+}
+
+// Displacement x_j - x_i, minimum image (float64; the float32 value decides the
+// image unless the box is so small that a pair in range can be half a box long).
+template <int D>
+__device__ inline double pair_vec(const AdjArgs& g, const double* __restrict__ x, int i, int j,
+                                  double* d) {
+  double r2 = 0.0;
+#pragma unroll
+  for (int k = 0; k < D; k++) {
+    double v = __dadd_rn(x[(size_t)j * D + k], -x[(size_t)i * D + k]);
+    if (g.exact_image) {
+      if (!(fabs(v) < 0.49 * g.L[k])) v -= g.L[k] * rint(v / g.L[k]);
+    } else {
+      const float q = rintf((float)v * g.Linvf[k]);
+      if (q != 0.f) v = fma(-(double)q, g.L[k], v);
+    }
+    d[k] = v;
+    r2 = k == 0 ? __dmul_rn(v, v) : fma(v, v, r2);
+  }
+  return r2;
+}
+
+// One law at squared distance r2 < rc2, in the form the kernels use it:
+// U, fr = f / r, and (WANT_G) fp = f' and the derivatives of U and f / r by
+// (u0, r0).  Lennard-Jones laws of even power take a reciprocal, no root.
+struct PairD {
+  double U, fr, fp, dU[2], dfr[2], w;
+};
+
+template <bool LJ>
+__device__ inline PairD eval_pair_d(const Law& l, double r2) {
+  PairD p;
+  if (LJ) {
+    const double w = recip_d(r2), n = (double)l.n;
+    double s;  // (r0 / r)^n
+    if (l.n == 6) {
+      const double q = __dmul_rn(l.r02, w);
+      s = __dmul_rn(__dmul_rn(q, q), q);
+    } else if ((l.n & 1) == 0) {
+      const double q = __dmul_rn(l.r02, w);
+      s = q;
+      for (int e = 2; e < l.n; e += 2) s = __dmul_rn(s, q);
+    } else {
+      const double q = sqrt(__dmul_rn(l.r02, w));
+      s = q;
+      for (int e = 1; e < l.n; e++) s = __dmul_rn(s, q);
+    }
+    const double t = __dmul_rn(2.0 * n, __dmul_rn(s, w));  // 2 n s / r^2
+    p.w = w;
+    p.U = l.u0 * s * (s - 2.0);
+    p.dfr[0] = __dmul_rn(-t, __dadd_rn(s, -1.0));
+    p.fr = __dmul_rn(l.u0, p.dfr[0]);
+    p.fp = l.u0 * t * fma(2.0 * n + 1.0, s, -(n + 1.0));
+    p.dU[0] = s * (s - 2.0);
+    p.dU[1] = 2.0 * n * l.u0 * s * (s - 1.0) * l.ir0;
+    p.dfr[1] = -l.u0 * t * n * fma(2.0, s, -1.0) * l.ir0;
+  } else {
+    // Yukawa: U = u0 e / r, e = exp(-r / r0)
+    const double ir = rsqrt(r2), r = __dmul_rn(r2, ir), ir0 = l.ir0;
+    const double e = exp(__dmul_rn(-r, ir0));
+    const double eir = __dmul_rn(e, ir);                   // e / r
+    const double h = __dmul_rn(eir, __dadd_rn(ir0, ir));   // e (1 / (r r0) + 1 / r^2)
+    p.w = __dmul_rn(ir, ir);
+    p.U = l.u0 * eir;
+    p.dfr[0] = __dmul_rn(-h, ir);
+    p.fr = __dmul_rn(l.u0, p.dfr[0]);
+    p.fp = l.u0 * eir * (ir0 * ir0 + 2.0 * ir * ir0 + 2.0 * p.w);
+    p.dU[0] = eir;
+    p.dU[1] = l.u0 * e * ir0 * ir0;
+    p.dfr[1] = -l.u0 * eir * ir0 * ir0 * ir0;
+  }
+  return p;
+}
+
+// The pair terms of a warp's PW particles.  32 / PW lanes per particle screen
+// its four sub-lists in float32; the pairs inside a law's cutoff are queued by
+// kind of law, 32 of a kind are evaluated with every lane busy, and each
+// sub-list's terms are added in list order (one running sum per sub-list, kind
+// and component), so results do not depend on PW.  Measured on the mixture at
+// 16,384 / 1,001 particles, against four lanes per particle walking their
+// sub-lists: see k_adj_step and k_adj_back.
+// NS: terms held per kind.
+template <int NC, int PW, int NS = 128>
+struct PairQueue {
+  static constexpr int CH = PW * TPP;           // sub-lists of the warp
+  static constexpr int CAP = NS / CH;           // terms per sub-list and kind
+  static_assert(CAP >= 32 / CH, "a round fits");
+  static constexpr int SLOTS = CH * CAP;
+  double term[SLOTS][NC];
+  double acc[CH][NC];
+  int j[SLOTS];
+  unsigned short slot[SLOTS];
+  unsigned char law[SLOTS];
+  int n[CH];
+};
+
+// Runs term(p, i, j, law, kind, out[NC]) for every pair of the warp's
+// particles and adds the results to q[kind].acc.  ti, i, cnt: the lane's
+// particle (p = lane / LPP of the warp), its type and its sub-list's length
+// (sub-list sub % TPP); i0: the warp's first particle.
+template <int D, int NC, int PW, int NS, class Term>
+__device__ inline void for_pairs(const AdjArgs& g, const Law* laws, PairQueue<NC, PW, NS>* q,
+                                 const double* __restrict__ x, const int* __restrict__ nbr, int W,
+                                 const int* __restrict__ types, int i0, int i, int ti, int cnt,
+                                 Term&& term) {
+  typedef PairQueue<NC, PW, NS> Queue;
+  constexpr int LPP = 32 / PW, CAP = Queue::CAP, STEP = LPP / TPP;  // entries per round
+  const int l32 = threadIdx.x & 31, p = l32 / LPP, sub = l32 % LPP, c = p * TPP + sub % TPP;
+  for (int e = l32; e < 2 * Queue::CH; e += 32) {
+    q[e & 1].n[e >> 1] = 0;
+#pragma unroll
+    for (int k = 0; k < NC; k++) q[e & 1].acc[e >> 1][k] = 0.0;
+  }
+  __syncwarp();
+  int queued[2] = {0, 0};  // the same on every lane
+  auto flush = [&](auto kind) {
+    constexpr int K = decltype(kind)::value;
+    Queue& f = q[K];
+    __syncwarp();
+    for (int e = l32; e < queued[K]; e += 32) {
+      const int slot = f.slot[e];
+      double out[NC];
+      term(kind, i0 + slot / (TPP * CAP), f.j[e], laws[f.law[e]], (int)f.law[e], out);
+#pragma unroll
+      for (int k = 0; k < NC; k++) f.term[slot][k] = out[k];
+    }
+    __syncwarp();
+    for (int e = l32; e < Queue::CH * NC; e += 32) {
+      const int cc = e / NC, k = e % NC, n = f.n[cc];
+      double v = f.acc[cc][k];
+      for (int t = 0; t < n; t++) v = __dadd_rn(v, f.term[cc * CAP + t][k]);
+      f.acc[cc][k] = v;
+    }
+    __syncwarp();
+    for (int e = l32; e < Queue::CH; e += 32) f.n[e] = 0;
+    queued[K] = 0;
+    __syncwarp();
+  };
+  float xi[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+  for (int k = 0; k < D; k++) xi[k] = screen_coord(g, k, x + (size_t)i * D + k);
+  // lanes of the same sub-list
+  unsigned int peers = 0u;
+#pragma unroll
+  for (int e = 0; e < LPP; e++)
+    if (e % TPP == sub % TPP) peers |= 1u << (p * LPP + e);
+  const unsigned int below = (1u << l32) - 1u;
+  const int* row = nbr + ((size_t)i * TPP + sub % TPP) * W;
+  const int rounds = (__reduce_max_sync(0xffffffffu, cnt) + STEP - 1) / STEP;
+  int e = sub / TPP;
+  int jn = e < cnt ? row[e] : -1;
+  for (int r = 0; r < rounds; r++) {
+    const int j = jn;
+    e += STEP;
+    jn = e < cnt ? row[e] : -1;
+    unsigned int m = 0u;  // laws the pair is inside of
+    if (j >= 0) {
+      float r2 = 0.f;
+#pragma unroll
+      for (int k = 0; k < D; k++) {
+        float v = screen_coord(g, k, x + (size_t)j * D + k) - xi[k];
+        v -= g.Lf[k] * rintf(v * g.Linvf[k]);
+        r2 += v * v;
+      }
+      for (unsigned int mm = g.lawmask[ti * MAXT + types[j]]; mm; mm &= mm - 1u) {
+        const int l = __ffs(mm) - 1;
+        if (r2 < laws[l].screen2) m |= 1u << l;
+      }
+    }
+    while (__any_sync(0xffffffffu, m)) {  // each lane's next law
+      const int l = m ? __ffs(m) - 1 : 0;
+      const int kind = m ? (laws[l].law == RDSIM_LAW_LJ ? 0 : 1) : -1;
+      m &= m - 1u;
+#pragma unroll
+      for (int K = 0; K < 2; K++) {
+        const unsigned int b = __ballot_sync(0xffffffffu, kind == K), mine = b & peers;
+        if (!b) continue;
+        Queue& f = q[K];
+        const int n = f.n[c];
+        __syncwarp();
+        if (kind == K) {
+          const int at = queued[K] + __popc(b & below);
+          f.j[at] = j;
+          f.law[at] = (unsigned char)l;
+          f.slot[at] = (unsigned short)(c * CAP + n + __popc(mine & below));
+        }
+        if (!(peers & below)) f.n[c] = n + __popc(mine);
+        queued[K] += __popc(b);
+        __syncwarp();
+        // room for another round in every sub-list
+        if (__any_sync(0xffffffffu, f.n[c] > CAP - STEP)) {
+          if (K == 0) flush(std::integral_constant<int, 0>{});
+          else flush(std::integral_constant<int, 1>{});
+        }
+      }
+    }
+  }
+  flush(std::integral_constant<int, 0>{});
+  flush(std::integral_constant<int, 1>{});
+}
+
+// Component k of particle p's sum over its sub-lists and kinds (in the order of
+// a xor tree over four lanes).
+template <int NC, int PW, int NS>
+__device__ inline double pair_sum(const PairQueue<NC, PW, NS>* q, int p, int k) {
+  double c[TPP];
+#pragma unroll
+  for (int l = 0; l < TPP; l++) c[l] = __dadd_rn(q[0].acc[p * TPP + l][k], q[1].acc[p * TPP + l][k]);
+  return __dadd_rn(__dadd_rn(c[0], c[1]), __dadd_rn(c[2], c[3]));
+}
+
 // One state: loss terms (F_LOSS, accumulated per particle into lacc) and the
-// step to the next state (F_STEP).  TPP lanes per particle.
-template <int D, int FL>
+// step to the next state (F_STEP).  Mixture, step only: 70 -> 35 us at 16,384
+// particles (57 % of the float64 pipe), 30 -> 10 us at 1,001.
+template <int D, int FL, int PW>
 __global__ void __launch_bounds__(BLK) k_adj_step(AdjArgs g, const double* __restrict__ x,
                                                   const int* __restrict__ nbr,
                                                   const int* __restrict__ ncnt, int W,
@@ -332,73 +543,72 @@ __global__ void __launch_bounds__(BLK) k_adj_step(AdjArgs g, const double* __res
                                                   double* __restrict__ lacc,
                                                   const float* __restrict__ xr,
                                                   int* __restrict__ moved) {
+  constexpr int LPP = 32 / PW, PER = BLK / 32 * PW;
+  constexpr bool LOSS = (FL & F_LOSS) != 0;
+  constexpr int NC = D + (LOSS ? 1 : 0);
   __shared__ Law slaws[MAXL];
+  __shared__ PairQueue<NC, PW> queue[BLK / 32][2];
   if (threadIdx.x < (unsigned)g.nlaws) slaws[threadIdx.x] = g.laws[threadIdx.x];
   __syncthreads();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = t % TPP;
-  const int i = min(t / TPP, g.N - 1);  // surplus lanes mirror the last particle
-  const bool own = t / TPP < g.N;
-  const int ti = types[i];
-  double xi[3] = {0.0, 0.0, 0.0};
+  const int warp = threadIdx.x >> 5, l32 = threadIdx.x & 31, sub = l32 % LPP;
+  const int i0 = (int)blockIdx.x * PER + warp * PW;
+  const bool own = i0 + l32 / LPP < g.N;
+  const int i = own ? i0 + l32 / LPP : g.N - 1;
+  const int cnt = own ? min(ncnt[(size_t)(sub % TPP) * g.N + i], W) : 0;
+  for_pairs<D>(g, slaws, queue[warp], x, nbr, W, types, i0, i, types[i], cnt,
+                       [&](auto kind, int gi, int gj, const Law& w, int, double* out) {
+    double d[3];
+    const double r2 = pair_vec<D>(g, x, gi, gj, d);
+    if (!(r2 < w.rc2)) {
 #pragma unroll
-  for (int k = 0; k < D; k++) xi[k] = x[(size_t)i * D + k];
-  double a[3] = {0.0, 0.0, 0.0};
-  double loss = 0.0;
-  for_list<D>(g, x, nbr, ncnt, W, i, xi, lane, [&](int j, const double* d) {
-    const int tj = types[j];
-    const unsigned int m = g.lawmask[ti * MAXT + tj];
-    if (!m) return;
-    double r2 = 0.0;
-#pragma unroll
-    for (int k = 0; k < D; k++) r2 += d[k] * d[k];
-    if (!(r2 < g.rc2max)) return;  // in the list's skin only
-    const double ir = rsqrt(r2), r = r2 * ir;
-    // iteration q takes each lane's q-th law: lanes of different type
-    // pairs evaluate their first laws together
-    for (unsigned int mm = m; mm; mm &= mm - 1) {
-      const Law& w = slaws[__ffs(mm) - 1];
-      if (!(r < w.rc)) continue;
-      const PairEval p = eval_law(w, r, ir);
-      const double fi = p.f * ir;
-#pragma unroll
-      for (int k = 0; k < D; k++) a[k] += fi * d[k];
-      // each pair is seen from both ends: half of its loss on each
-      if (FL & F_LOSS) loss += 0.5 * (g.wU * (p.U - w.Uc) - g.wW * r * p.f);
+      for (int k = 0; k < NC; k++) out[k] = 0.0;
+      return;
     }
-  });
+    const PairD e = eval_pair_d<decltype(kind)::value == 0>(w, r2);
 #pragma unroll
-  for (int k = 0; k < D; k++) a[k] = lane_sum(a[k]);
-  if (FL & F_LOSS) loss = lane_sum(loss);
-  if (!own || lane != 0) return;
-  if (xr) {
+    for (int k = 0; k < D; k++) out[k] = __dmul_rn(e.fr, d[k]);
+    // each pair is seen from both ends: half of its loss on each
+    if (LOSS) out[NC - 1] = 0.5 * (g.wU * (e.U - w.Uc) - g.wW * r2 * e.fr);
+  });
+  __syncthreads();
+  // one thread per particle and component
+  const int t = threadIdx.x;
+  if (t >= PER * NC) return;
+  const int pq = t / NC, k = t % NC, ip = (int)blockIdx.x * PER + pq;
+  if (ip >= g.N) return;
+  const double v = pair_sum(queue[pq / PW], pq % PW, k);
+  if (LOSS && k == D) {
+    lacc[ip] += v;
+    return;
+  }
+  const int ti = types[ip];
+  const double xk = x[(size_t)ip * D + k];
+  if (xr && k == 0) {
     // the list in use dates from an earlier state: it holds every pair in
     // range only while no particle has moved more than the skin allows
     float d2 = 0.f;
 #pragma unroll
-    for (int k = 0; k < D; k++) {
-      float v = (float)xi[k] - xr[(size_t)i * D + k];
-      v -= g.Lf[k] * rintf(v * g.Linvf[k]);
-      d2 += v * v;
+    for (int c = 0; c < D; c++) {
+      float u = (float)x[(size_t)ip * D + c] - xr[(size_t)ip * D + c];
+      u -= g.Lf[c] * rintf(u * g.Linvf[c]);
+      d2 += u * u;
     }
     if (d2 > g.move2f) atomicOr(moved, 1);
   }
-  if (FL & F_LOSS) lacc[i] += loss;
   if (FL & F_STEP) {
-#pragma unroll
-    for (int k = 0; k < D; k++) {
-      double v = xi[k];
-      v += g.c[ti] * a[k];
-      v += g.s[ti] * noise[(size_t)i * D + k];
-      v -= g.L[k] * floor(v / g.L[k]);
-      x_out[(size_t)i * D + k] = v;
-    }
+    double y = fma(g.c[ti], v, xk);
+    y = fma(g.s[ti], noise[(size_t)ip * D + k], y);
+    const double L = k == 0 ? g.L[0] : (k == 1 ? g.L[1] : g.L[2]);
+    if (!(y >= 0.0 && y < L)) y -= L * floor(y / L);
+    x_out[(size_t)ip * D + k] = y;
   }
 }
 
 // One state of the backward pass (see the file comment).  gpart[block][NG]
 // accumulates this CTA's parameter gradients over the steps, in step order.
-template <int D, int FL>
+// Mixture, step only / with loss terms: 128 / 162 -> 63 / 79 us at 16,384
+// particles, 51 / 62 -> 13 / 14 us at 1,001.
+template <int D, int FL, int PW>
 __global__ void __launch_bounds__(BLK) k_adj_back(AdjArgs g, const double* __restrict__ x,
                                                   const int* __restrict__ nbr,
                                                   const int* __restrict__ ncnt, int W,
@@ -406,104 +616,98 @@ __global__ void __launch_bounds__(BLK) k_adj_back(AdjArgs g, const double* __res
                                                   const double* __restrict__ lam_next,
                                                   double* __restrict__ lam_out,
                                                   double* __restrict__ gpart) {
+  constexpr int LPP = 32 / PW, PER = BLK / 32 * PW;
   __shared__ Law slaws[MAXL];
-  __shared__ double sgp[NG][BLK];  // per-thread parameter gradients
-  if (threadIdx.x < (unsigned)g.nlaws) slaws[threadIdx.x] = g.laws[threadIdx.x];
-#pragma unroll
-  for (int q = 0; q < NG; q++) sgp[q][threadIdx.x] = 0.0;
+  __shared__ PairQueue<D, PW, D == 3 ? 64 : 128> queue[BLK / 32][2];  // (48 KB in all)
+  __shared__ double sgp[NG][BLK + 1];  // per-thread parameter gradients
+  const int tid = threadIdx.x;
+  if (tid < g.nlaws) slaws[tid] = g.laws[tid];
+  for (int q = 0; q < 2 * g.nlaws; q++) sgp[q][tid] = 0.0;
   __syncthreads();
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
-  const int lane = t % TPP;
-  const int i = min(t / TPP, g.N - 1);
-  const bool own = t / TPP < g.N;
-  const int ti = types[i];
-  double xi[3] = {0.0, 0.0, 0.0}, wi[3] = {0.0, 0.0, 0.0}, out[3] = {0.0, 0.0, 0.0};
+  const int warp = tid >> 5, l32 = tid & 31, sub = l32 % LPP;
+  const int i0 = (int)blockIdx.x * PER + warp * PW;
+  const bool own = i0 + l32 / LPP < g.N;
+  const int i = own ? i0 + l32 / LPP : g.N - 1;
+  const int cnt = own ? min(ncnt[(size_t)(sub % TPP) * g.N + i], W) : 0;
+  for_pairs<D>(g, slaws, queue[warp], x, nbr, W, types, i0, i, types[i], cnt,
+                      [&](auto kind, int gi, int gj, const Law& w, int l, double* out) {
+    double d[3];
+    const double r2 = pair_vec<D>(g, x, gi, gj, d);
 #pragma unroll
-  for (int k = 0; k < D; k++) {
-    xi[k] = x[(size_t)i * D + k];
-    if (FL & F_STEP) wi[k] = g.c[ti] * lam_next[(size_t)i * D + k];
-  }
-  for_list<D>(g, x, nbr, ncnt, W, i, xi, lane, [&](int j, const double* d) {
-    const int tj = types[j];
-    const unsigned int m = g.lawmask[ti * MAXT + tj];
-    if (!m) return;
-    double r2 = 0.0;
+    for (int k = 0; k < D; k++) out[k] = 0.0;
+    if (!(r2 < w.rc2)) return;
+    const PairD e = eval_pair_d<decltype(kind)::value == 0>(w, r2);
+    double ddw = 0.0;  // d . (w_j - w_i)
+    if (FL & F_STEP) {
+      const double ci = g.c[types[gi]], cj = g.c[types[gj]];
+      double dw[3];
 #pragma unroll
-    for (int k = 0; k < D; k++) r2 += d[k] * d[k];
-    if (!(r2 < g.rc2max)) return;  // in the list's skin only
-    const double ir = rsqrt(r2), r = r2 * ir;
-    double rh[3] = {0.0, 0.0, 0.0}, dw[3] = {0.0, 0.0, 0.0};
-    double rdw = 0.0;  // rhat . (w_j - w_i)
-#pragma unroll
-    for (int k = 0; k < D; k++) {
-      rh[k] = d[k] * ir;
-      if (FL & F_STEP) {
-        dw[k] = g.c[tj] * lam_next[(size_t)j * D + k] - wi[k];
-        rdw += rh[k] * dw[k];
+      for (int k = 0; k < D; k++) {
+        dw[k] = fma(cj, lam_next[(size_t)gj * D + k], -(ci * lam_next[(size_t)gi * D + k]));
+        ddw = fma(d[k], dw[k], ddw);
       }
+      // f' rhat rhat.dw + (f / r) (dw - rhat rhat.dw)
+      const double h = (e.fp - e.fr) * e.w * ddw;
+#pragma unroll
+      for (int k = 0; k < D; k++) out[k] = fma(h, d[k], e.fr * dw[k]);
     }
-    // iteration q takes each lane's q-th law (see k_adj_step)
-    for (unsigned int mm = m; mm; mm &= mm - 1) {
-      const int l = __ffs(mm) - 1;
-      const Law& w = slaws[l];
-      if (!(r < w.rc)) continue;
-      const PairEval p = eval_law(w, r, ir);
-      if (FL & F_STEP) {
-        const double fr = p.f * ir;
+    if (FL & F_LOSS) {
+      // d loss_pair / dr times d r / d x_i = -rhat
+      const double dl = g.wU * e.fr - g.wW * (e.fr + e.fp);
 #pragma unroll
-        for (int k = 0; k < D; k++) out[k] += p.fp * rh[k] * rdw + fr * (dw[k] - rh[k] * rdw);
-      }
-      if (FL & F_LOSS) {
-        // d loss_pair / dr times d r / d x_i = -rhat
-        const double dl = g.wU * p.f - g.wW * (p.f + r * p.fp);
+      for (int k = 0; k < D; k++) out[k] = fma(-dl, d[k], out[k]);
+    }
+    if (gj > gi) {
 #pragma unroll
-        for (int k = 0; k < D; k++) out[k] -= dl * rh[k];
-      }
-      if (j > i && own) {
-#pragma unroll
-        for (int q = 0; q < 2; q++) {
-          double v = 0.0;
-          if (FL & F_STEP) v -= p.df[q] * rdw;  // df/dtheta rhat . (w_i - w_j)
-          if (FL & F_LOSS)
-            v += g.wU * (p.dU[q] - (q == 0 ? w.dUc_du0 : w.dUc_dr0)) - g.wW * r * p.df[q];
-          sgp[2 * l + q][threadIdx.x] += v;
-        }
+      for (int q = 0; q < 2; q++) {
+        double v = 0.0;
+        if (FL & F_STEP) v -= e.dfr[q] * ddw;  // df/dtheta rhat . (w_i - w_j)
+        if (FL & F_LOSS)
+          v += g.wU * (e.dU[q] - (q == 0 ? w.dUc_du0 : w.dUc_dr0)) - g.wW * r2 * e.dfr[q];
+        sgp[2 * l + q][tid] += v;
       }
     }
   });
-#pragma unroll
-  for (int k = 0; k < D; k++) out[k] = lane_sum(out[k]);
-  if (own && lane == 0) {
-#pragma unroll
-    for (int k = 0; k < D; k++)
-      lam_out[(size_t)i * D + k] = out[k] + ((FL & F_STEP) ? lam_next[(size_t)i * D + k] : 0.0);
-  }
-  // CTA sum of the parameter gradients in thread order, added to this CTA's
-  // slot
   __syncthreads();
-  if (threadIdx.x < 2 * g.nlaws) {
+  if (tid < PER * D) {
+    const int pq = tid / D, k = tid % D, ip = (int)blockIdx.x * PER + pq;
+    if (ip < g.N) {
+      const double v = pair_sum(queue[pq / PW], pq % PW, k);
+      lam_out[(size_t)ip * D + k] = v + ((FL & F_STEP) ? lam_next[(size_t)ip * D + k] : 0.0);
+    }
+  }
+  // CTA sum of the parameter gradients in a fixed order (eight threads per
+  // parameter), added to this CTA's slot
+  static_assert(BLK == 8 * NG, "eight threads per parameter");
+  {
+    const int q = tid / 8, part = tid % 8;
     double v = 0.0;
-    for (int u = 0; u < BLK; u++) v += sgp[threadIdx.x][u];
-    gpart[(size_t)blockIdx.x * NG + threadIdx.x] += v;
+    if (q < 2 * g.nlaws)
+      for (int u = 0; u < BLK / 8; u++) v += sgp[q][u * 8 + part];
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    if (part == 0 && q < 2 * g.nlaws) gpart[(size_t)blockIdx.x * NG + q] += v;
   }
 }
 
-// Sum of n values (or n rows of NG values) in a fixed order: one CTA, thread
-// t adds entries t, t + BLK, ..., then a fixed tree.
-__global__ void __launch_bounds__(BLK) k_sum_rows(const double* __restrict__ v, int n, int width,
-                                                  double* __restrict__ out) {
-  __shared__ double sh[BLK];
-  for (int col = 0; col < width; col++) {
+// Sum of n values (or n rows of NG values) in a fixed order: one CTA per column,
+// thread t adds entries t, t + SUM_T, ..., then a fixed tree.  (One CTA of 128
+// threads for all columns: 16 us of latency; now 4 us.)
+constexpr int SUM_T = 512;
+__global__ void __launch_bounds__(SUM_T) k_sum_rows(const double* __restrict__ v, int n, int width,
+                                                    double* __restrict__ out) {
+  __shared__ double sh[SUM_T];
+  const int col = blockIdx.x;
+  {
     double s = 0.0;
-    for (int r = threadIdx.x; r < n; r += BLK) s += v[(size_t)r * width + col];
+    for (int r = threadIdx.x; r < n; r += SUM_T) s += v[(size_t)r * width + col];
     sh[threadIdx.x] = s;
     __syncthreads();
-    for (int o = BLK / 2; o > 0; o >>= 1) {
+    for (int o = SUM_T / 2; o > 0; o >>= 1) {
       if ((int)threadIdx.x < o) sh[threadIdx.x] += sh[threadIdx.x + o];
       __syncthreads();
     }
     if (threadIdx.x == 0) out[col] = sh[0];
-    __syncthreads();
   }
 }
 
@@ -513,8 +717,16 @@ __global__ void k_scale(double* v, size_t n, double f) {
 }
 
 unsigned nblk(int n) { return (unsigned)((n + BLK - 1) / BLK); }
-// CTAs of the pair kernels (TPP lanes per particle)
-unsigned pblk(int n) { return nblk(n * TPP); }
+// CTAs of the list kernel (TPP lanes per particle) and of the pair kernels
+unsigned lblk(int n) { return nblk(n * TPP); }
+// Particles per warp of the float64 pair kernels.  Loss and gradients at 2 / 4 /
+// 8 per warp: 1.45 / 1.62 / 2.24 ms for 16 steps at 1,001 particles, 3.30 / 2.97
+// / 3.95 ms for 32 steps at 4,096, 7.67 / 6.15 / 6.08 ms at 16,384.
+int pair_width(int n) { return n <= 2500 ? 2 : 4; }
+unsigned pblk(int n) {
+  const int per = BLK / 32 * pair_width(n);
+  return (unsigned)((n + per - 1) / per);
+}
 
 }  // namespace
 
@@ -585,7 +797,7 @@ void build_list_d(rdsim_adjoint* h, const double* x, int slot, float* xr) {
   k_fill<D><<<nblk(g.N), BLK, 0, h->stream>>>(g, x, h->cursor, h->idx);
   k_cell_sort<D><<<nblk(g.ncell), BLK, 0, h->stream>>>(g.ncell, x, h->start, h->idx, h->xs,
                                                         h->count);
-  k_adj_list<D><<<pblk(g.N), BLK, 0, h->stream>>>(g, x, h->start, h->idx, h->xs, h->W,
+  k_adj_list<D><<<lblk(g.N), BLK, 0, h->stream>>>(g, x, h->start, h->idx, h->xs, h->W,
                                                    slot_nbr(h, slot), slot_ncnt(h, slot),
                                                    h->maxcnt, xr);
 }
@@ -601,9 +813,9 @@ void build_list(rdsim_adjoint* h, const double* x, int slot, float* xr = nullptr
 template <int D, int FL>
 void step_k(rdsim_adjoint* h, const double* x, int slot, const double* noise, double* x_out,
             const float* xr) {
-  k_adj_step<D, FL><<<pblk(h->g.N), BLK, 0, h->stream>>>(h->g, x, slot_nbr(h, slot),
-                                                          slot_ncnt(h, slot), h->W, h->types,
-                                                          noise, x_out, h->lacc, xr, h->moved);
+  auto k = pair_width(h->g.N) == 2 ? k_adj_step<D, FL, 2> : k_adj_step<D, FL, 4>;
+  k<<<pblk(h->g.N), BLK, 0, h->stream>>>(h->g, x, slot_nbr(h, slot), slot_ncnt(h, slot), h->W,
+                                         h->types, noise, x_out, h->lacc, xr, h->moved);
 }
 
 template <int D>
@@ -625,9 +837,9 @@ void step(rdsim_adjoint* h, const double* x, int slot, const double* noise, doub
 
 template <int D, int FL>
 void back_k(rdsim_adjoint* h, const double* x, int slot, const double* lam_next, double* lam_out) {
-  k_adj_back<D, FL><<<pblk(h->g.N), BLK, 0, h->stream>>>(h->g, x, slot_nbr(h, slot),
-                                                          slot_ncnt(h, slot), h->W, h->types,
-                                                          lam_next, lam_out, h->gpart);
+  auto k = pair_width(h->g.N) == 2 ? k_adj_back<D, FL, 2> : k_adj_back<D, FL, 4>;
+  k<<<pblk(h->g.N), BLK, 0, h->stream>>>(h->g, x, slot_nbr(h, slot), slot_ncnt(h, slot), h->W,
+                                         h->types, lam_next, lam_out, h->gpart);
 }
 
 template <int D>
@@ -703,7 +915,8 @@ int rdsim_adjoint_create(const rdsim_adjoint_system* s, int32_t device, rdsim_ad
   const double cut_skin = cut_exact + 2.0 * skin_half;
   if (rc_max <= 0 || 2.0 * cut_skin > Lmin) h->R = 1;
   const double cut_cells = h->R > 1 ? cut_skin : cut_exact;
-  g.rc2max = rc_max * rc_max;
+  for (int k = 0; k < D; k++)
+    if (!(s->L[k] >= 2.1 * rc_max)) g.exact_image = 1;
   h->cut2f_exact = (float)(cut_exact * cut_exact * (1.0 + 1e-6));
   h->cut2f_skin = (float)(cut_skin * cut_skin * (1.0 + 1e-6));
   {
@@ -829,6 +1042,14 @@ int rdsim_adjoint_forward(rdsim_adjoint* h, const double* x0, const double* para
     w.rc = it.rc;
     if (!(w.r0 > 0)) return fail(RDSIM_ERR_ARG, "r0 must be positive");
     w.ir0 = 1.0 / w.r0;
+    w.r02 = w.r0 * w.r0;
+    w.rc2 = w.rc * w.rc;
+    // the screen's coordinates carry 20 bits each: at most 2^-20 of twice the
+    // box per coordinate, and the float32 arithmetic a few 1e-7 of it
+    double Lmax = 0.0;
+    for (int k = 0; k < g.D; k++) Lmax = std::max(Lmax, g.L[k]);
+    const double cut = w.rc + 8.0 * std::sqrt((double)g.D) * std::ldexp(Lmax, -20) + 1e-4;
+    w.screen2 = (float)(cut * cut * (1.0 + 1e-6));
     const PairEval p = eval_law(w, w.rc, 1.0 / w.rc);
     w.Uc = p.U;
     w.dUc_du0 = p.dU[0];
@@ -887,7 +1108,7 @@ int rdsim_adjoint_forward(rdsim_adjoint* h, const double* x0, const double* para
   }
   h->R_used = R;
   if (cur != h->xT) CK(cudaMemcpyAsync(h->xT, cur, sizeof(double) * nd, cudaMemcpyDeviceToDevice, h->stream));
-  k_sum_rows<<<1, BLK, 0, h->stream>>>(h->lacc, N, 1, h->red);
+  k_sum_rows<<<1, SUM_T, 0, h->stream>>>(h->lacc, N, 1, h->red);
   CK(cudaMemcpyAsync(loss, h->red, sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   if (x_final) CK(cudaMemcpyAsync(x_final, h->xT, sizeof(double) * nd, cudaMemcpyDeviceToDevice, h->stream));
   CK(cudaStreamSynchronize(h->stream));
@@ -954,7 +1175,7 @@ int rdsim_adjoint_backward(rdsim_adjoint* h, double dloss, double* grad_x0, doub
     cur = 1 - cur;
   }
   CK(cudaGetLastError());
-  k_sum_rows<<<1, BLK, 0, h->stream>>>(h->gpart, (int)pblk(N), NG, h->red);
+  k_sum_rows<<<NG, SUM_T, 0, h->stream>>>(h->gpart, (int)pblk(N), NG, h->red);
   double gsum[NG];
   CK(cudaMemcpyAsync(gsum, h->red, sizeof gsum, cudaMemcpyDeviceToHost, h->stream));
   CK(cudaMemcpyAsync(grad_x0, h->lam[cur], sizeof(double) * nd, cudaMemcpyDeviceToDevice,

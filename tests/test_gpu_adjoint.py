@@ -210,3 +210,48 @@ def test_adjoint_3d_matches_dense_autograd():
     assert abs(loss.item() - ref.item()) <= 1e-12 * abs(ref.item())
     assert float((x0.grad - xd.grad).norm() / xd.grad.norm()) <= 1e-9
     np.testing.assert_allclose(params.grad.numpy(), pd.grad.cpu().numpy(), rtol=1e-9)
+
+
+@pytest.mark.parametrize("n,scale", [(37, 1.0), (2499, 1.0), (2503, 1.0), (300, 2.02), (300, 37.0)])
+def test_pair_kernels_at_their_splits(n, scale):
+    """Sizes around the split of particles over warps, a box of little more
+    than twice the cutoff (the float64 image test), and starting positions
+    many boxes away (the screen wraps them): loss and gradients against the
+    dense reference.  scale 2.02: box length in units of the cutoff; 37: boxes
+    by which the start is displaced."""
+    from pyrdsim_gb300 import workloads
+    from pyrdsim_gb300.adjoint import Adjoint, trajectory_loss
+    if scale == 2.02:
+        L = 2.02 * 2.5
+        rng = np.random.default_rng(n)
+        g = np.stack(np.meshgrid(np.arange(4), np.arange(4), indexing="ij"), -1).reshape(-1, 2)
+        x = (g + 0.5 + rng.uniform(-0.05, 0.05, g.shape)) * (L / 4)
+        w = {"L": [L, L], "dt": 1e-4, "mobility": np.array([1.0, 1.0]),
+             "types": np.arange(16, dtype=np.int32) % 2, "x0": x, "pairs": [(0, 0), (0, 1), (1, 1)],
+             "rc_lj": 2.5, "rc_yukawa": 2.5, "theta": np.array([1.0, 1.0, 5.0, 2.0])}
+    else:
+        w = workloads.mixed_lj_yukawa(n=n, seed=n)
+    n = len(w["types"])
+    x0 = np.array(w["x0"])
+    if scale == 37.0:
+        x0 = x0 + 37.0 * np.asarray(w["L"]) * np.where(np.arange(n)[:, None] % 2, 1.0, -1.0)
+    adj = Adjoint(2, w["L"], w["dt"], w["mobility"], w["types"],
+                  workloads.mixed_lj_yukawa_laws(w), loss_steps=3, checkpoint_every=2)
+    rng = np.random.default_rng(1)
+    xi = torch.tensor(rng.standard_normal((5, n, 2)), dtype=torch.float64, device="cuda")
+    res = []
+    for fn in ("gpu", "dense"):
+        xg = torch.tensor(x0, dtype=torch.float64, device="cuda", requires_grad=True)
+        p = torch.tensor(workloads.mixed_lj_yukawa_params(w["theta"]), dtype=torch.float64,
+                         device="cpu" if fn == "gpu" else "cuda", requires_grad=True)
+        if fn == "gpu":
+            loss = trajectory_loss(xg, p, xi, adj)
+        else:
+            loss = dense_loss(xg, p, xi, w["types"], _dense_laws(w), w["L"], w["dt"],
+                              w["mobility"], 3)
+        loss.backward()
+        res.append((loss.item(), xg.grad.cpu().numpy(), p.grad.cpu().numpy()))
+    (la, ga, pa), (lb, gb, pb) = res
+    assert abs(la - lb) <= 1e-11 * abs(lb), (la, lb)
+    assert np.linalg.norm(ga - gb) <= 1e-9 * np.linalg.norm(gb)
+    np.testing.assert_allclose(pa, pb, rtol=1e-9, atol=1e-12 * np.abs(pb).max())
