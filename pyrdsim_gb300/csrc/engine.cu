@@ -352,8 +352,12 @@ void launch_listed(rdsim_handle* h, unsigned g, const Args& a) {
 
 template <int D, int TPP, int LPC>
 void launch_nlist_v(rdsim_handle* h, const Args& a) {
-  const unsigned per = (unsigned)(LBLOCK / TPP / LPC * (D == 1 ? 1 : 3));
-  launch(k_nlist<D, TPP, LPC>, (unsigned)h->pchunks_h.size(), per, h->stream, a);
+  constexpr int per = LBLOCK / TPP / LPC;
+  const unsigned g = (unsigned)h->pchunks_h.size();
+  if constexpr (nlist_by_lanes(D, LPC))
+    launch(k_nlist_lanes<D, TPP, LPC>, g, nlist_lane_threads(per), h->stream, a);
+  else
+    launch(k_nlist<D, TPP, LPC>, g, nlist_threads(D, per), h->stream, a);
 }
 
 template <int D>

@@ -414,18 +414,12 @@ __global__ void k_first_records(Args a) {
   if (i < a.n_total) first_records<D>(a, i, a.meta[i], false);
 }
 
-// Rebuild: every particle's list row and entry count.  NT threads per
-// particle (3 for D >= 2: one per row of cells in 2D, one per three rows in
-// 3D) scan their rows' runs in candidate order, four candidates per batch of
-// loads, into shared-memory buffers; the buffers are then concatenated in row
-// order (the order row_scan uses), so the row does not depend on NT.  A
-// thread whose rows hold more than BCAP listed pairs rescans them to write
-// the rest.  With F_RX_HERE the first thread of each particle also runs the
-// reaction prefilter of its step with the fresh entry count.  With
-// F_PERIOD_PREP it also writes the period kernel's records of its particles:
-// of step 0 (candidates of the rebuild step marked pending), and "no step yet"
-// for the other parity.  Chunks' staging tables and slot codes: see the top of
-// this file.
+// Rebuild: every particle's list row and entry count.  With F_RX_HERE one thread
+// per particle also runs the reaction prefilter of its step with the fresh
+// counts, and with F_PERIOD_PREP it writes the period kernel's records of its
+// particle: of step 0 (candidates of the rebuild step marked pending), and "no
+// step yet" for the other parity.  Chunks' staging tables and slot codes: see
+// the top of this file.
 // Position, in 16-bit codes, of entry e of particle p of a chunk: chain e % TPP of
 // its row is shared by LPC lanes, which take its entries in turn.
 template <int TPP, int LPC>
@@ -441,10 +435,31 @@ struct StageHash {
   int total, on;
 };
 
+// Two forms.  k_nlist: NT threads per particle (3 in 2D, one per row of cells)
+// scan their rows' runs in candidate order, four candidates per batch of loads,
+// into shared-memory buffers; the buffers are then concatenated in row order (the
+// order row_scan uses).  A thread whose rows hold more than BCAP listed pairs
+// scans again to write the rest.  k_nlist_lanes: 16 lanes per particle walk one
+// run after the other, 16 consecutive candidates at a time; hits are numbered by
+// ballots and written where they belong; lane q finds the run bounds of row q of
+// cells for the others.  The rows are the same.  The lanes form is the faster one
+// where rows of cells hold many candidates (in 3D the thread with a particle's
+// own row outgrows its buffer: 107 us with threads, 55 with lanes at 13,824
+// particles) and where few particles leave threads to spare (11.2 -> 9.2 us at
+// 1,024); its set-up, done by 16 lanes for 3 rows, loses in large 2D systems (21 /
+// 43 us at 65,536, 127 / 409 at 1,048,576).
+__host__ __device__ constexpr bool nlist_by_lanes(int D, int lpc) { return D == 3 || lpc == 4; }
+constexpr int NL_LANES = 16;
+// Threads per CTA (chunks of `per` particles).
+__host__ __device__ constexpr int nlist_threads(int D, int per) { return per * (D == 1 ? 1 : 3); }
+__host__ __device__ constexpr int nlist_lane_threads(int per) {
+  return per * NL_LANES < 512 ? per * NL_LANES : 512;
+}
+
 // LPC: see period.cuh (the period kernel's lanes per chain of a row; its chunks
 // are this kernel's).
 template <int D, int TPP, int LPC>
-__global__ void __launch_bounds__((LBLOCK / TPP / LPC) * (D == 1 ? 1 : 3)) k_nlist(Args a) {
+__global__ void __launch_bounds__(nlist_threads(D, LBLOCK / TPP / LPC)) k_nlist(Args a) {
   constexpr int PER = LBLOCK / TPP / LPC;
   constexpr int NT = D == 1 ? 1 : 3;
   constexpr int NTH = PER * NT;
@@ -670,6 +685,204 @@ __global__ void __launch_bounds__((LBLOCK / TPP / LPC) * (D == 1 ? 1 : 3)) k_nli
     const unsigned int bal = __ballot_sync(0xffffffffu, listed);
     if (bal) {
       const int l32 = threadIdx.x & 31, leader = __ffs(bal) - 1;
+      const int p = rx_slot(eff_step(a));
+      int base = 0;
+      if (l32 == leader) base = atomicAdd(a.rx_count + p, __popc(bal));
+      base = __shfl_sync(0xffffffffu, base, leader);
+      if (listed) a.rx_list[(size_t)p * a.npad + base + __popc(bal & ((1u << l32) - 1u))] = rec;
+    }
+  }
+}
+
+template <int D, int TPP, int LPC>
+__global__ void __launch_bounds__(nlist_lane_threads(LBLOCK / TPP / LPC)) k_nlist_lanes(Args a) {
+  constexpr int PER = LBLOCK / TPP / LPC;
+  constexpr int NTH = nlist_lane_threads(PER), NPASS = PER * NL_LANES / NTH;
+  constexpr int NROW = D == 3 ? 9 : (D == 2 ? 3 : 1);
+  static_assert(NROW <= NL_LANES, "a lane per row of cells");
+  __shared__ SysDev sys;
+  __shared__ StageHash sth;
+  __shared__ int2 scnt[PER];  // entries, and those within the reactions' reach
+  pdl_trigger();
+  const Chunk ch = chunk_at<PER>(a, (int)blockIdx.x);
+  {
+    constexpr int NS = (int)(sizeof(SysDev) / 4);
+    WordLoad<NS, NTH> ls;
+    ls.load(reinterpret_cast<const int*>(&a.sys[ch.sys]), NS);
+    ls.store(reinterpret_cast<int*>(&sys), NS);
+  }
+  const bool prep = (a.flags & F_PERIOD_PREP) != 0;
+  const bool stage = a.codes != nullptr;
+  const int tid = (int)threadIdx.x, l32 = tid & 31, sub = tid % NL_LANES;
+  if (stage) {
+    for (int q = tid; q < STG_HASH; q += NTH) {
+      sth.key[q] = 0;
+      sth.lo[q] = 0x7fffffff;
+      sth.hi[q] = -1;
+    }
+    if (tid == 0) {
+      sth.total = 0;
+      sth.on = 1;
+    }
+  }
+  pdl_wait();
+  __syncthreads();
+  const SysDev& s = sys;
+  // slot of chunk key - 1 (of this system) in the hash, -1 if absent
+  auto find = [&](int key, bool insert) {
+    for (int q = 0, h = key & (STG_HASH - 1); q < STG_HASH; q++, h = (h + 1) & (STG_HASH - 1)) {
+      const int k = insert ? atomicCAS(&sth.key[h], 0, key) : sth.key[h];
+      if (k == key || (insert && k == 0)) return h;
+      if (k == 0) return -1;
+    }
+    return -1;
+  };
+  // the runs of row `sub` of the cells around the particle of each pass
+  int rb[NPASS][2], re[NPASS][2];
+#pragma unroll
+  for (int ps = 0; ps < NPASS; ps++) {
+    const int pp = ps * (NTH / NL_LANES) + tid / NL_LANES;
+    const bool valid = pp < ch.cnt;
+    const int i = ch.beg + (valid ? pp : 0);
+    int c[3] = {0, 0, 0};
+    bool first = pp == 0;
+#pragma unroll
+    for (int k = 0; k < D; k++) {
+      c[k] = cell_coord(s, k, a.xr[k][i]);
+      if (pp > 0 && valid) first = first || cell_coord(s, k, a.xr[k][i - 1]) != c[k];
+    }
+    const int dz = D == 3 ? sub / 3 - 1 : 0, dy = D >= 2 ? sub % 3 - 1 : 0;
+    const int h1 = D > 1 ? s.halo[1] : 0, h2 = D > 2 ? s.halo[2] : 0;
+    int row = 0, lo0 = 0, hi0 = 0, lo1 = 0, hi1 = 0;
+    const bool ok = valid && sub < NROW && dy >= -h1 && dy <= h1 && dz >= -h2 && dz <= h2 &&
+                    row_runs<D>(s, c, dy, dz, row, lo0, hi0, lo1, hi1);
+    const int* cs = a.cell_start + s.c0 + row;
+    const bool two = ok && hi1 >= lo1;
+    rb[ps][0] = ok ? cs[lo0] : 0;
+    re[ps][0] = ok ? cs[hi0 + 1] : 0;
+    rb[ps][1] = two ? cs[lo1] : 0;
+    re[ps][1] = two ? cs[hi1 + 1] : 0;
+    // the chunks they touch (the runs of the first particle of each cell are
+    // those of the others too)
+    if (stage && valid && first)
+#pragma unroll
+      for (int q = 0; q < 2; q++)
+        for (int b = rb[ps][q]; b < re[ps][q];) {
+          const int cc = (b - s.p0) / PER, e = min(re[ps][q], s.p0 + (cc + 1) * PER);
+          const int h = find(cc + 1, true);
+          if (h < 0) {
+            sth.on = 0;
+          } else {
+            atomicMin(&sth.lo[h], b);
+            atomicMax(&sth.hi[h], e - 1);
+          }
+          b = e;
+        }
+  }
+  bool staged = false;
+  if (stage) {
+    __syncthreads();
+    // table positions, in whatever order the counter hands them out
+    for (int q = tid; q < STG_HASH; q += NTH)
+      if (sth.key[q]) {
+        const int len = sth.hi[q] - sth.lo[q] + 1;
+        sth.off[q] = atomicAdd(&sth.total, len) - sth.lo[q];
+      }
+    __syncthreads();
+    staged = sth.on && sth.total <= a.stg_max;
+    if (tid == 0) a.stg_n[blockIdx.x] = staged ? sth.total : -1;
+    if (staged) {
+      int* g = a.stg_g + (size_t)blockIdx.x * a.stg_max;
+      for (int q = tid / 16; q < STG_HASH; q += NTH / 16)
+        if (sth.key[q])
+          for (int j = sth.lo[q] + tid % 16; j <= sth.hi[q]; j += 16) g[sth.off[q] + j] = j;
+    }
+  }
+  unsigned short* codes = reinterpret_cast<unsigned short*>(a.codes) +
+                          (size_t)blockIdx.x * a.kw * LBLOCK * 2;
+  const int coded = staged ? min(a.W, a.kw * 2 * TPP * LPC) : 0;  // entries with a code
+  const float Rl2 = s.Rl2, Rrl2 = s.Rrl2;
+  const unsigned int below = (1u << sub) - 1u;
+  const int shift = l32 & ~(NL_LANES - 1);
+#pragma unroll
+  for (int ps = 0; ps < NPASS; ps++) {
+    const int pp = ps * (NTH / NL_LANES) + tid / NL_LANES;
+    const bool valid = pp < ch.cnt;
+    const int i = ch.beg + (valid ? pp : 0);
+    uint32_t xi[3] = {0u, 0u, 0u};
+#pragma unroll
+    for (int k = 0; k < D; k++) xi[k] = a.xr[k][i];
+    const uint32_t mi = a.meta[i];
+    const int moli = a.mol[i];
+    const int trbi = (mi >> 8) & 0xff, loci = (mi >> 16) & 0xff, tmi = mi >> 24;
+    const unsigned int pmask = s.partner[trbi];
+    const uint32_t bmask = tmi != 0xff ? a.tmpl[tmi].bondmask[loci] : 0u;
+    int cnt = 0, rcnt = 0, lastc = -1, lasto = 0;
+#pragma unroll 1
+    for (int q = 0; q < 2 * NROW; q++) {
+      const int b = __shfl_sync(0xffffffffu, (q & 1) ? rb[ps][1] : rb[ps][0], q >> 1, NL_LANES);
+      const int e = __shfl_sync(0xffffffffu, (q & 1) ? re[ps][1] : re[ps][0], q >> 1, NL_LANES);
+      // (the particles of a warp go round together)
+      const int most = __reduce_max_sync(0xffffffffu, max(e - b, 0));
+      for (int t = sub; t < most + sub; t += NL_LANES) {
+        const int j = b + t;
+        const bool in = j < e;
+        const int jl = in ? j : i;
+        uint32_t xj[3] = {0u, 0u, 0u};
+#pragma unroll
+        for (int d = 0; d < D; d++) xj[d] = a.xr[d][jl];
+        const uint32_t mj = a.meta[jl];
+        const bool own = a.mol[jl] == moli;
+        float r2 = 0.f;
+#pragma unroll
+        for (int d = 0; d < D; d++) {
+          const float dd = (float)(int)(xj[d] - xi[d]) * s.unit_hi[d];
+          r2 += dd * dd;
+        }
+        const bool hit = in && j != i && r2 < Rl2 &&
+                         ((own ? bmask >> ((mj >> 16) & 31) : pmask >> ((mj >> 8) & 0xff)) & 1u);
+        const unsigned int m = (__ballot_sync(0xffffffffu, hit) >> shift) & ((1u << NL_LANES) - 1u);
+        const unsigned int mr = (__ballot_sync(0xffffffffu, hit && r2 < Rrl2) >> shift) &
+                                ((1u << NL_LANES) - 1u);
+        if (hit) {
+          const int k = cnt + __popc(m & below);
+          if (k < a.W) a.nbr_out[ell_index<TPP>(k, i, a.npad)] = own ? (j | LIST_SAME_MOL) : j;
+          if (k < coded) {
+            const int cc = (j - s.p0) / PER;
+            if (cc != lastc) {
+              lastc = cc;
+              lasto = sth.off[find(cc + 1, false)];
+            }
+            codes[code_at<TPP, LPC>(pp, k)] = (unsigned short)(((j + lasto) << 4) | (own ? 1 : 0));
+          }
+        }
+        cnt += __popc(m);
+        rcnt += __popc(mr);
+      }
+    }
+    if (valid && sub == 0) scnt[pp] = make_int2(cnt, rcnt);
+  }
+  __syncthreads();
+  if (tid >= (PER + 31) / 32 * 32) return;
+  int4 rec = make_int4(0, 0, 0, 0);
+  bool listed = false;
+  if (tid < ch.cnt) {
+    const int i = ch.beg + tid;
+    const uint32_t mi = a.meta[i];
+    const int2 n = scnt[tid];
+    a.ncnt_out[i] = n.x;
+    a.rcnt_out[i] = n.y;
+    if (a.flags & F_RX_HERE) {  // reaction prefilter of this step (see rx_may_react)
+      rec = make_int4(i, (int)mi, n.x, a.pid[i]);
+      listed = rx_may_react<D>(s, (int)(mi & 0xff), n.y, rec.w, eff_step(a), nullptr);
+      a.meta_out[i] = mi;
+    }
+    if (prep) first_records<D>(a, i, mi, listed);
+  }
+  if (a.flags & F_RX_HERE) {  // the candidate list of the per-step kernels
+    const unsigned int bal = __ballot_sync(0xffffffffu, listed);
+    if (bal) {
+      const int leader = __ffs(bal) - 1;
       const int p = rx_slot(eff_step(a));
       int base = 0;
       if (l32 == leader) base = atomicAdd(a.rx_count + p, __popc(bal));

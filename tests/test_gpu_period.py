@@ -205,3 +205,23 @@ def test_lj_walk_equals_the_general_walk(n):
             for a, b in zip(es[0].state(), es[1].state()):
                 np.testing.assert_array_equal(a, b)
             np.testing.assert_array_equal(es[0].drift(), es[1].drift())
+
+
+@pytest.mark.parametrize("n,D,width", [(1, 2, 0), (16, 2, 0), (17, 2, 8), (65, 2, 0), (1100, 2, 0),
+                                       (2049, 3, 0), (2060, 3, 8), (70, 1, 0)])
+def test_list_builder_of_small_and_3d_systems(n, D, width):
+    """Rows built by 16 lanes per particle, at remainders of a chunk and with rows
+    beyond the stored width: the drift from them against float64 (the suite's
+    bounds), and the period kernel's states from the codes written with them
+    against the per-step kernels' from the rows."""
+    from test_gpu_force64 import _system
+    from test_gpu_parity import _oracle, drift_errors
+    sd = _system(n, D, "lj")
+    one = _engine([sd], list_width=width)
+    norm, per = drift_errors(one.drift(), _oracle(sd).drift())
+    assert norm < 1e-5 and per < 1e-4, (norm, per)
+    steps = _engine([sd], list_width=width, period_kernel=False)
+    for k in (23, 12):
+        one.step(k)
+        steps.step(k)
+        np.testing.assert_array_equal(one.state()[0], steps.state()[0])
