@@ -379,17 +379,10 @@ void launch_react(rdsim_handle* h, const Args& a) {
 
 unsigned nblk(int n, int b = 256) { return (unsigned)((n + b - 1) / b); }
 
-// `prefilter`: the list builder also runs the reaction prefilter of `step`
-// (then the reaction kernel of that step visits the listed particles only);
-// `rel`: step numbers are offsets from the device counter (graph capture).
-int rebuild(rdsim_handle* h, long long step = 0, bool prefilter = false, bool rel = false,
-            bool period_prep = false) {
+// Every particle into the order of its cell (k_bin, the scan, k_scatter, k_order).
+void sort_cells(rdsim_handle* h, const Args& a, const OrderOut& o, long long* ctr, long long add) {
   const int n = h->N;
-  ProfScope ps(h, P_REBUILD, h->ncells <= SCAN1_T * SCAN1_I ? 5 : 6);
   uint32_t* const* x = h->xh[h->cx];
-  // a captured period advances the step counter by one period in k_bin
-  long long* ctr = rel ? h->step_dev : nullptr;
-  const long long add = h->freq;
   if (h->D == 2)
     launch(k_bin<2>, nblk(n), 256, h->stream, h->sys_d, h->sid, x[0], x[1], x[2], n, h->cell_of, h->rank_of, h->cell_count, ctr, add);
   else if (h->D == 3)
@@ -404,15 +397,36 @@ int rebuild(rdsim_handle* h, long long step = 0, bool prefilter = false, bool re
   }
   launch(k_scatter, nblk(n), 256, h->stream, h->cell_of, h->rank_of, h->cell_start, n, h->tmp,
          h->cell_count, h->ncells);
+  if (h->D == 2) launch(k_order<2>, nblk(n), 256, h->stream, a, o, h->tmp, h->cell_of, h->cell_start, n);
+  else if (h->D == 3) launch(k_order<3>, nblk(n), 256, h->stream, a, o, h->tmp, h->cell_of, h->cell_start, n);
+  else launch(k_order<1>, nblk(n), 256, h->stream, a, o, h->tmp, h->cell_of, h->cell_start, n);
+}
+
+// `prefilter`: the list builder also runs the reaction prefilter of `step`
+// (then the reaction kernel of that step visits the listed particles only);
+// `rel`: step numbers are offsets from the device counter (graph capture).
+int rebuild(rdsim_handle* h, long long step = 0, bool prefilter = false, bool rel = false,
+            bool period_prep = false) {
+  const int n = h->N;
+  // sort_one: see k_sort_one
+  const bool sort_one = n <= SORT1_MAX && h->ncells <= SORT1_MAX;
+  ProfScope ps(h, P_REBUILD, sort_one ? 2 : (h->ncells <= SCAN1_T * SCAN1_I ? 5 : 6));
+  // a captured period advances the step counter by one period
+  long long* ctr = rel ? h->step_dev : nullptr;
+  const long long add = h->freq;
   Args a = make_args(h);
   OrderOut o;
   o.mol = h->mol[1 - h->co];
   o.pid = h->pid[1 - h->co];
   for (int k = 0; k < 3; k++) o.xr[k] = h->xr[k];
   o.slot_of = h->slot_of;
-  if (h->D == 2) launch(k_order<2>, nblk(n), 256, h->stream, a, o, h->tmp, h->cell_of, h->cell_start, n);
-  else if (h->D == 3) launch(k_order<3>, nblk(n), 256, h->stream, a, o, h->tmp, h->cell_of, h->cell_start, n);
-  else launch(k_order<1>, nblk(n), 256, h->stream, a, o, h->tmp, h->cell_of, h->cell_start, n);
+  if (sort_one) {
+    const size_t mem = sizeof(int) * ((size_t)h->ncells + n);
+    auto k = h->D == 2 ? k_sort_one<2> : h->D == 3 ? k_sort_one<3> : k_sort_one<1>;
+    launch_dyn(k, 1, SORT1_T, mem, h->stream, a, o, h->sid, n, h->ncells, h->cell_start, ctr, add);
+  } else {
+    sort_cells(h, a, o, ctr, add);
+  }
   h->cx = 1 - h->cx;
   h->cm = 1 - h->cm;
   h->co = 1 - h->co;

@@ -225,3 +225,35 @@ def test_list_builder_of_small_and_3d_systems(n, D, width):
         one.step(k)
         steps.step(k)
         np.testing.assert_array_equal(one.state()[0], steps.state()[0])
+
+
+@pytest.mark.parametrize("n,D", [(2048, 2), (2049, 2), (1331, 3), (1100, 1)])
+def test_small_sort_equals_the_general_one(n, D):
+    """Up to 2,048 particles one CTA sorts the cells; a batch with a second
+    system takes the four kernels for both.  A system's rows, states and drift
+    are the same bit for bit, with list builders of either form."""
+    from pyrdsim_gb300 import model
+    rng = np.random.default_rng(n)
+    side = int(np.ceil(n ** (1.0 / D)))
+    L = 1.5 * side
+    g = np.stack(np.meshgrid(*[np.arange(side)] * D, indexing="ij"), -1).reshape(-1, D)
+    x = (g[rng.permutation(len(g))[:n]] + 0.5 + rng.uniform(-0.1, 0.1, (n, D))) * 1.5
+    m = model.Model.from_dict({
+        "n_dim": D, "l": np.full(D, L), "periodic": np.array([1.0] * (D - 1) + [-1.0]),
+        "dt": 1e-4, "n_steps": 10, "n_out": 1000, "tau_by_taud": np.ones(2), "seed": 3,
+        "interactions": [{"type": "lj", "pair": [a, b], "u0": 1.0, "r0": 1.1, "rc": 2.5, "n": 6}
+                         for a, b in ((0, 0), (0, 1), (1, 1))],
+        "reactions": [{"type": "linear", "reactant": 0, "product": 1, "rate": 20.0},
+                      {"type": "locally_catalyzed", "reactant": 1, "catalyst": 0, "product": 0,
+                       "rate": 20.0, "r0": 1.6}]})
+    mol = np.stack([np.arange(n), np.zeros(n, int), np.zeros(n, int)], 1).astype(np.int32)
+    sd = model.SystemData(m, x, rng.integers(0, 2, n).astype(np.int32), mol,
+                          np.arange(n, dtype=np.int32))
+    alone, batch = _engine([sd]), _engine([sd, sd])
+    for k in (25, 8, 13):
+        alone.step(k)
+        batch.step(k)
+        (xa, ta), (xb, tb) = alone.state(), batch.state()
+        np.testing.assert_array_equal(xa, xb[:n])
+        np.testing.assert_array_equal(ta, tb[:n])
+    np.testing.assert_array_equal(alone.drift(), batch.drift()[:n])
