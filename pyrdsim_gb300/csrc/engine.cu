@@ -172,6 +172,11 @@ struct rdsim_handle {
   ErrDev* err = nullptr;
   double* cl_d = nullptr;
   int cx = 0, cm = 0, co = 0;
+  // device memory of the arrays above, in a few blocks (a cudaMalloc costs 10 to
+  // 20 us, and a handle has about 60 arrays)
+  std::vector<void*> blocks;
+  char* block_at = nullptr;
+  size_t block_left = 0;
   // static per-particle data (caller order): host copies and device copies
   std::vector<uint32_t> meta_static;  // local << 16 | template << 24
   std::vector<int> mol_h;
@@ -213,6 +218,34 @@ struct rdsim_handle {
 };
 
 namespace {
+
+// n elements for the handle's lifetime: small arrays share blocks.
+template <class T>
+int salloc(rdsim_handle* h, T** p, size_t n) {
+  constexpr size_t BLOCK_BYTES = (size_t)2 << 20;
+  const size_t bytes = (std::max<size_t>(n, 1) * sizeof(T) + 255) / 256 * 256;
+  h->device_bytes += (int64_t)(std::max<size_t>(n, 1) * sizeof(T));
+  if (bytes > h->block_left) {
+    const size_t take = std::max(bytes, BLOCK_BYTES);
+    void* b = nullptr;
+    cudaError_t e = cudaMalloc(&b, take);
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // clear the non-sticky allocation error
+      return fail(RDSIM_ERR_NOMEM, std::string("cudaMalloc: ") + cudaGetErrorString(e));
+    }
+    h->blocks.push_back(b);
+    if (bytes > BLOCK_BYTES / 2) {  // a block of its own; the shared one stays in use
+      *p = reinterpret_cast<T*>(b);
+      return 0;
+    }
+    h->block_at = reinterpret_cast<char*>(b);
+    h->block_left = take;
+  }
+  *p = reinterpret_cast<T*>(h->block_at);
+  h->block_at += bytes;
+  h->block_left -= bytes;
+  return 0;
+}
 
 enum { P_FORCE = 0, P_REACT = 1, P_EM = 2, P_REBUILD = 3, P_HOOK = 4 };
 
@@ -708,25 +741,10 @@ void free_all(rdsim_handle* h) {
   auto F = [](void* p) {
     if (p) cudaFree(p);
   };
-  F(h->sys_d); F(h->laws_d); F(h->walls_d); F(h->rx_d); F(h->tmpl_d);
-  F(h->terms_d); F(h->atomterm_d); F(h->cell_count); F(h->cell_start); F(h->bsum);
-  F(h->cell_of); F(h->rank_of); F(h->tmp); F(h->sid); F(h->slot_of);
-  F(h->chunks_d); F(h->pchunks_d); F(h->fchunks_d); F(h->nbr); F(h->ncnt); F(h->rcnt); F(h->rx_list); F(h->rx_count);
-  F(h->stg_n); F(h->stg_g); F(h->codes);
-  for (int b = 0; b < 2; b++) { F(h->rec[b]); F(h->recl[b]); F(h->rech[b]); }
-  for (int b = 0; b < 2; b++) {
-    for (int k = 0; k < 3; k++) { F(h->xh[b][k]); F(h->xl[b][k]); F(h->xp[b][k]); }
-    F(h->meta[b]); F(h->mol[b]); F(h->pid[b]);
-  }
-  for (int k = 0; k < 3; k++) { F(h->xr[k]); F(h->drift[k]); F(h->drift_d[k]); }
-  F(h->typed_d);
-  F(h->rates); F(h->xbuf); F(h->tbuf); F(h->err); F(h->cl_d);
-  F(h->meta_static_d); F(h->mol_static_d); F(h->flag_d);
+  for (void* b : h->blocks) F(b);
   F(h->inj_xi); F(h->inj_u1); F(h->inj_u2); F(h->traj_x); F(h->traj_t);
-  F(h->olaws_d); F(h->owalls_d); F(h->oterms_d); F(h->obs_part); F(h->obs_counts);
-  F(h->rdf_counts); F(h->pair_total);
-  F(h->stamps);
-  F(h->stamp_sum);
+  F(h->obs_part); F(h->obs_counts); F(h->rdf_counts);
+  F(h->stamps); F(h->stamp_sum);
   for (auto& p : h->pending) {
     cudaEventDestroy(p.a);
     cudaEventDestroy(p.b);
@@ -734,7 +752,6 @@ void free_all(rdsim_handle* h) {
   for (auto e : h->ev_pool) cudaEventDestroy(e);
   for (auto& g : h->graph_cache) cudaGraphExecDestroy(g.second.exec);
   h->graph_cache.clear();
-  F(h->step_dev);
   if (h->stream) cudaStreamDestroy(h->stream);
 }
 
@@ -1380,61 +1397,60 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
       return bail(fail(RDSIM_ERR_UNSUPPORTED, "too many particles for the list kernels"));
   }
   // device memory
-  int64_t& B = h->device_bytes;
   const int N = h->N;
-  if ((rc = dalloc(&h->sys_d, h->sys_h.size(), &B))) return bail(rc);
-  if ((rc = dalloc(&h->laws_d, laws.size(), &B))) return bail(rc);
-  if ((rc = dalloc(&h->walls_d, walls.size(), &B))) return bail(rc);
-  if ((rc = dalloc(&h->rx_d, rxs.size(), &B))) return bail(rc);
-  if ((rc = dalloc(&h->tmpl_d, tmpls.size(), &B))) return bail(rc);
-  if ((rc = dalloc(&h->terms_d, terms.size(), &B))) return bail(rc);
-  if ((rc = dalloc(&h->atomterm_d, atomterm.size(), &B))) return bail(rc);
-  if ((rc = dalloc(&h->olaws_d, olaws.size(), &B))) return bail(rc);
-  if ((rc = dalloc(&h->owalls_d, owalls.size(), &B))) return bail(rc);
-  if ((rc = dalloc(&h->oterms_d, oterms.size(), &B))) return bail(rc);
-  if ((rc = dalloc(&h->cell_count, (size_t)h->ncells, &B))) return bail(rc);
+  if ((rc = salloc(h, &h->sys_d, h->sys_h.size()))) return bail(rc);
+  if ((rc = salloc(h, &h->laws_d, laws.size()))) return bail(rc);
+  if ((rc = salloc(h, &h->walls_d, walls.size()))) return bail(rc);
+  if ((rc = salloc(h, &h->rx_d, rxs.size()))) return bail(rc);
+  if ((rc = salloc(h, &h->tmpl_d, tmpls.size()))) return bail(rc);
+  if ((rc = salloc(h, &h->terms_d, terms.size()))) return bail(rc);
+  if ((rc = salloc(h, &h->atomterm_d, atomterm.size()))) return bail(rc);
+  if ((rc = salloc(h, &h->olaws_d, olaws.size()))) return bail(rc);
+  if ((rc = salloc(h, &h->owalls_d, owalls.size()))) return bail(rc);
+  if ((rc = salloc(h, &h->oterms_d, oterms.size()))) return bail(rc);
+  if ((rc = salloc(h, &h->cell_count, (size_t)h->ncells))) return bail(rc);
   // zero once; every rebuild leaves them zero for the next (k_scatter)
   if (cudaMemsetAsync(h->cell_count, 0, sizeof(int) * (size_t)h->ncells, h->stream) != cudaSuccess)
     return bail(fail(RDSIM_ERR_CUDA, "memset"));
-  if ((rc = dalloc(&h->cell_start, (size_t)h->ncells + 1, &B))) return bail(rc);
-  if ((rc = dalloc(&h->bsum, (size_t)h->nscan, &B))) return bail(rc);
-  if ((rc = dalloc(&h->cell_of, N, &B))) return bail(rc);
-  if ((rc = dalloc(&h->rank_of, N, &B))) return bail(rc);
-  if ((rc = dalloc(&h->tmp, N, &B))) return bail(rc);
-  if ((rc = dalloc(&h->sid, N, &B))) return bail(rc);
-  if ((rc = dalloc(&h->slot_of, N, &B))) return bail(rc);
+  if ((rc = salloc(h, &h->cell_start, (size_t)h->ncells + 1))) return bail(rc);
+  if ((rc = salloc(h, &h->bsum, (size_t)h->nscan))) return bail(rc);
+  if ((rc = salloc(h, &h->cell_of, N))) return bail(rc);
+  if ((rc = salloc(h, &h->rank_of, N))) return bail(rc);
+  if ((rc = salloc(h, &h->tmp, N))) return bail(rc);
+  if ((rc = salloc(h, &h->sid, N))) return bail(rc);
+  if ((rc = salloc(h, &h->slot_of, N))) return bail(rc);
   for (int b = 0; b < 2; b++) {
     for (int k = 0; k < D; k++) {
-      if ((rc = dalloc(&h->xh[b][k], N, &B))) return bail(rc);
-      if ((rc = dalloc(&h->xl[b][k], N, &B))) return bail(rc);
-      if ((rc = dalloc(&h->xp[b][k], N, &B))) return bail(rc);
+      if ((rc = salloc(h, &h->xh[b][k], N))) return bail(rc);
+      if ((rc = salloc(h, &h->xl[b][k], N))) return bail(rc);
+      if ((rc = salloc(h, &h->xp[b][k], N))) return bail(rc);
     }
-    if ((rc = dalloc(&h->meta[b], N, &B))) return bail(rc);
-    if ((rc = dalloc(&h->mol[b], N, &B))) return bail(rc);
-    if ((rc = dalloc(&h->pid[b], N, &B))) return bail(rc);
+    if ((rc = salloc(h, &h->meta[b], N))) return bail(rc);
+    if ((rc = salloc(h, &h->mol[b], N))) return bail(rc);
+    if ((rc = salloc(h, &h->pid[b], N))) return bail(rc);
   }
   for (int k = 0; k < D; k++) {
-    if ((rc = dalloc(&h->xr[k], N, &B))) return bail(rc);
-    if ((rc = dalloc(&h->drift[k], N, &B))) return bail(rc);
-    if (h->f64 && (rc = dalloc(&h->drift_d[k], N, &B))) return bail(rc);
+    if ((rc = salloc(h, &h->xr[k], N))) return bail(rc);
+    if ((rc = salloc(h, &h->drift[k], N))) return bail(rc);
+    if (h->f64 && (rc = salloc(h, &h->drift_d[k], N))) return bail(rc);
   }
-  if ((rc = dalloc(&h->typed_d, typed.size(), &B))) return bail(rc);
-  if ((rc = dalloc(&h->rates, N, &B))) return bail(rc);
-  if ((rc = dalloc(&h->xbuf, (size_t)N * D, &B))) return bail(rc);
-  if ((rc = dalloc(&h->tbuf, N, &B))) return bail(rc);
-  if ((rc = dalloc(&h->meta_static_d, N, &B))) return bail(rc);
-  if ((rc = dalloc(&h->mol_static_d, N, &B))) return bail(rc);
-  if ((rc = dalloc(&h->flag_d, 1, &B))) return bail(rc);
-  if ((rc = dalloc(&h->err, 1, &B))) return bail(rc);
-  if ((rc = dalloc(&h->step_dev, 1, &B))) return bail(rc);
-  if ((rc = dalloc(&h->pair_total, 2, &B))) return bail(rc);
+  if ((rc = salloc(h, &h->typed_d, typed.size()))) return bail(rc);
+  if ((rc = salloc(h, &h->rates, N))) return bail(rc);
+  if ((rc = salloc(h, &h->xbuf, (size_t)N * D))) return bail(rc);
+  if ((rc = salloc(h, &h->tbuf, N))) return bail(rc);
+  if ((rc = salloc(h, &h->meta_static_d, N))) return bail(rc);
+  if ((rc = salloc(h, &h->mol_static_d, N))) return bail(rc);
+  if ((rc = salloc(h, &h->flag_d, 1))) return bail(rc);
+  if ((rc = salloc(h, &h->err, 1))) return bail(rc);
+  if ((rc = salloc(h, &h->step_dev, 1))) return bail(rc);
+  if ((rc = salloc(h, &h->pair_total, 2))) return bail(rc);
   {
-    if ((rc = dalloc(&h->chunks_d, h->chunks_h.size(), &B))) return bail(rc);
-    if ((rc = dalloc(&h->nbr, (size_t)h->W * h->npad, &B))) return bail(rc);
-    if ((rc = dalloc(&h->ncnt, N, &B))) return bail(rc);
-    if ((rc = dalloc(&h->rcnt, N, &B))) return bail(rc);
-    if ((rc = dalloc(&h->rx_list, 3 * (size_t)h->npad, &B))) return bail(rc);
-    if ((rc = dalloc(&h->rx_count, 3, &B))) return bail(rc);
+    if ((rc = salloc(h, &h->chunks_d, h->chunks_h.size()))) return bail(rc);
+    if ((rc = salloc(h, &h->nbr, (size_t)h->W * h->npad))) return bail(rc);
+    if ((rc = salloc(h, &h->ncnt, N))) return bail(rc);
+    if ((rc = salloc(h, &h->rcnt, N))) return bail(rc);
+    if ((rc = salloc(h, &h->rx_list, 3 * (size_t)h->npad))) return bail(rc);
+    if ((rc = salloc(h, &h->rx_count, 3))) return bail(rc);
     if (cudaMemsetAsync(h->rx_count, 0, 3 * sizeof(int), h->stream) != cudaSuccess)
       return bail(fail(RDSIM_ERR_CUDA, "memset"));
   }
@@ -1485,15 +1501,15 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
   h->pchunks_h = make_chunks(h->sys_h, LBLOCK / h->ltpp / h->lpc);
   {
     const size_t nch = h->pchunks_h.size();
-    if ((rc = dalloc(&h->pchunks_d, nch, &B))) return bail(rc);
+    if ((rc = salloc(h, &h->pchunks_d, nch))) return bail(rc);
     if (h->period_on) {
-      if ((rc = dalloc(&h->stg_n, nch, &B))) return bail(rc);
-      if ((rc = dalloc(&h->stg_g, nch * h->stg_max, &B))) return bail(rc);
-      if ((rc = dalloc(&h->codes, nch * h->kw * LBLOCK, &B))) return bail(rc);
+      if ((rc = salloc(h, &h->stg_n, nch))) return bail(rc);
+      if ((rc = salloc(h, &h->stg_g, nch * h->stg_max))) return bail(rc);
+      if ((rc = salloc(h, &h->codes, nch * h->kw * LBLOCK))) return bail(rc);
       for (int b = 0; b < 2; b++) {
-        if ((rc = dalloc(&h->rec[b], N, &B))) return bail(rc);
-        if ((rc = dalloc(&h->recl[b], N, &B))) return bail(rc);
-        if ((rc = dalloc(&h->rech[b], N, &B))) return bail(rc);
+        if ((rc = salloc(h, &h->rec[b], N))) return bail(rc);
+        if ((rc = salloc(h, &h->recl[b], N))) return bail(rc);
+        if ((rc = salloc(h, &h->rech[b], N))) return bail(rc);
       }
     }
   }
@@ -1502,9 +1518,9 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
     h->fpw = force64_particles(N);
     fchunks = make_chunks(h->sys_h, force64_chunk(h->fpw));
     h->fchunks = (unsigned)fchunks.size();
-    if ((rc = dalloc(&h->fchunks_d, fchunks.size(), &B))) return bail(rc);
+    if ((rc = salloc(h, &h->fchunks_d, fchunks.size()))) return bail(rc);
   }
-  if ((rc = dalloc(&h->cl_d, (size_t)3 * h->nsys, &B))) return bail(rc);
+  if ((rc = salloc(h, &h->cl_d, (size_t)3 * h->nsys))) return bail(rc);
   auto up = [&](void* d, const void* s, size_t bytes) -> int {
     if (bytes == 0) return 0;
     CK(cudaMemcpyAsync(d, s, bytes, cudaMemcpyHostToDevice, h->stream));
