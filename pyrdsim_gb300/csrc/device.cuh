@@ -275,8 +275,13 @@ enum : int {
   F_RX_HERE = 128,                // list builder: the same for its own step
   F_PERIOD = 256,                 // step functions inside k_period: the step
                                   // number is the CTA's current step
-  F_PERIOD_PREP = 512             // list builder: write the records of the
+  F_PERIOD_PREP = 512,            // list builder: write the records of the
                                   // period kernel's first step
+  F_PERIOD_FULL = 1024            // list builder: the period kernel behind it
+                                  // needs most of the GPU, so no early launch:
+                                  // its CTAs among the builder's leave holes in
+                                  // an SM's shared memory that the last one does
+                                  // not fit in, and the others wait for it
 };
 
 // Slot of the candidate list of a step: three slots, so that a drift kernel

@@ -136,7 +136,7 @@ struct rdsim_handle {
   uint32_t* codes = nullptr;         // [chunks][kw][LBLOCK]
   // period kernel (period.cuh): the steps between two rebuilds in one launch
   bool all_lj6 = true;               // every pair law is a single Lennard-Jones n = 6
-  bool period_on = false;
+  bool period_on = false, period_full = false;  // period_full: see F_PERIOD_FULL
   int lpc = 1;                       // its lanes per chain (period.cuh)
   std::vector<Chunk> pchunks_h;      // its chunks
   Chunk* pchunks_d = nullptr;
@@ -466,7 +466,8 @@ int rebuild(rdsim_handle* h, long long step = 0, bool prefilter = false, bool re
   Args b = make_args(h);
   b.step = step;
   b.step_base = rel ? h->step_dev : nullptr;
-  b.flags = (prefilter ? F_RX_HERE : 0) | (period_prep ? F_PERIOD_PREP : 0);
+  b.flags = (prefilter ? F_RX_HERE : 0) | (period_prep ? F_PERIOD_PREP : 0) |
+            (period_prep && h->period_full ? F_PERIOD_FULL : 0);
   if (h->D == 2) launch_nlist<2>(h, b);
   else if (h->D == 3) launch_nlist<3>(h, b);
   else launch_nlist<1>(h, b);
@@ -1471,14 +1472,17 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
     const int nch = (int)make_chunks(h->sys_h, per).size();
     // neighbour staging: a chunk of P particles touches about its own run and
     // three cells more in every row of cells around it; a third more for
-    // denser places (a chunk that touches more gathers from memory)
+    // denser places, half more in 3D (a chunk that touches more gathers from
+    // memory, and the others wait for it: 13,824 particles in 3D 13.4 us per step
+    // with a third, 11.9 with half, 12.4 with twice; 65,536 in 2D 19.4 with a
+    // tenth, 16.0 with a third or half)
     double want = 64;
     int largest = 1;
     for (const SysDev& sd : h->sys_h) {
       double cells = 1;
       for (int k = 0; k < D; k++) cells *= sd.nc[k];
       const double rows = D == 3 ? 9 : (D == 2 ? 3 : 1);
-      want = std::max(want, rows * (per + 3.0 * sd.n / cells) * 1.3 + 64);
+      want = std::max(want, rows * (per + 3.0 * sd.n / cells) * (D == 3 ? 1.5 : 1.3) + 64);
       largest = std::max(largest, sd.n);
       h->rows = std::max(h->rows, sd.ntypes * sd.ntypes);
     }
@@ -1491,11 +1495,18 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
     // every chunk resident at once (its CTAs wait for each other), with less
     // room for staging if need be
     const PeriodVariant v{D, h->ltpp, h->lpc, h->has_rx};
-    for (int m = h->stg_max; m >= 64 && m >= h->stg_max / 4 && !h->period_on; m = m / 128 * 64)
-      if ((long long)period_blocks_per_sm(v, m, h->kw, h->rows) * sms >= nch) {
+    for (int m = h->stg_max; m >= 64 && m >= h->stg_max / 4 && !h->period_on; m = m / 128 * 64) {
+      const long long room = (long long)period_blocks_per_sm(v, m, h->kw, h->rows) * sms;
+      if (room >= nch) {
         h->period_on = true;
         h->stg_max = m;
+        // a third of the room is always left between another kernel's CTAs; there
+        // the early launch is worth 2 % (1,024 and 5,003 particles), above it
+        // costs (13,824 in 3D: 12.0 -> 11.7 us per step without it; 65,536: the
+        // last chunks did not fit, 27.6 -> 19.6)
+        h->period_full = nch > room / 3;
       }
+    }
     if (!h->period_on) h->lpc = 1;
   }
   h->pchunks_h = make_chunks(h->sys_h, LBLOCK / h->ltpp / h->lpc);

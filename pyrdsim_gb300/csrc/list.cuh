@@ -408,8 +408,7 @@ __device__ inline void first_records(const Args& a, int i, uint32_t mi, bool pen
 // The same for a launch of the period kernel that no list builder precedes.
 template <int D>
 __global__ void k_first_records(Args a) {
-  pdl_trigger();
-  pdl_wait();
+  pdl_wait();  // (no early launch of the period kernel: see F_PERIOD_FULL)
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < a.n_total) first_records<D>(a, i, a.meta[i], false);
 }
@@ -472,7 +471,7 @@ __global__ void __launch_bounds__(nlist_threads(D, LBLOCK / TPP / LPC)) k_nlist(
   __shared__ int sbuf[NTH][BCAP];
   __shared__ int2 scnt[NTH];
   __shared__ StageHash sth;
-  pdl_trigger();
+  if (!(a.flags & F_PERIOD_FULL)) pdl_trigger();
   const Chunk ch = chunk_at<PER>(a, (int)blockIdx.x);
   {
     constexpr int NS = (int)(sizeof(SysDev) / 4);
@@ -703,7 +702,7 @@ __global__ void __launch_bounds__(nlist_lane_threads(LBLOCK / TPP / LPC)) k_nlis
   __shared__ SysDev sys;
   __shared__ StageHash sth;
   __shared__ int2 scnt[PER];  // entries, and those within the reactions' reach
-  pdl_trigger();
+  if (!(a.flags & F_PERIOD_FULL)) pdl_trigger();
   const Chunk ch = chunk_at<PER>(a, (int)blockIdx.x);
   {
     constexpr int NS = (int)(sizeof(SysDev) / 4);

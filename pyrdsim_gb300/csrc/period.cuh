@@ -61,16 +61,35 @@ namespace rd {
 
 // Per-particle words of the chunk, kept for the launch.  The noise of the
 // update of a step is computed by the threads that have no particle tail of
-// their own while the tails of the step before run.
+// their own while the tails of the step before run.  Kept small (no pair words,
+// counts in 16 bits): seven chunks of a 2D system then need 164 KB of an SM and
+// not 196, which leaves the L1 92 KB and not 60 for spills, bonded partners and
+// the loads of the draws (65,536 particles, 10-step launch of the patchy system:
+// 111 -> 100 us; 160 / 153 us per rebuild period).
+constexpr unsigned int CNT_MANY = 0xffffu;  // this many or more: read it from memory
 template <int D, int PER>
 struct PeriodStage {
-  int pid[PER], cnt[PER], rcnt[PER];
+  int pid[PER];
+  uint32_t cnts[PER];               // entries of the row | those in the reactions' reach << 16
   uint32_t meta[PER];
   uint32_t xr[D][PER];              // high words at the rebuild
-  uint32_t xh[D][PER], xl[D][PER], xp[D][PER];
+  uint32_t xh[D][PER], xl[D][PER];
   uint32_t w[2][2][PER];            // Philox words (tag 0) the reaction draw uses, by
                                     // parity of the step
   float xi[2][D][PER];              // their standard normals
+
+  __device__ int cnt(const Args& a, int p, int i) const {
+    const unsigned int c = cnts[p] & 0xffffu;
+    return c < CNT_MANY ? (int)c : a.ncnt[i];
+  }
+  __device__ int rcnt(const Args& a, int p, int i) const {
+    const unsigned int c = cnts[p] >> 16;
+    return c < CNT_MANY ? (int)c : a.rcnt[i];
+  }
+  // pair word of dimension k
+  __device__ uint32_t xp(const SysDev& s, int k, int p) const {
+    return (uint32_t)((((unsigned long long)xh[k][p] << 32) | xl[k][p]) >> s.ps[k]);
+  }
 };
 
 struct PeriodShared {
@@ -250,9 +269,10 @@ __device__ __forceinline__ bool period_run_step(PeriodShared& ps,
       const int q = q0 + __ffs(b) - 1;
       uint32_t xo[3] = {0u, 0u, 0u};
 #pragma unroll
-      for (int d = 0; d < D; d++) xo[d] = st.xp[d][q];
-      period_resolve<D, TPP, LPC>(ps.sh, a, slots, codes, nstg >= 0 && st.cnt[q] <= lsmax, ch.beg + q, q,
-                             st.cnt[q], st.pid[q], &st.meta[q], xo, n, l32);
+      for (int d = 0; d < D; d++) xo[d] = st.xp(s, d, q);
+      const int cnt = st.cnt(a, q, ch.beg + q);
+      period_resolve<D, TPP, LPC>(ps.sh, a, slots, codes, nstg >= 0 && cnt <= lsmax, ch.beg + q, q,
+                             cnt, st.pid[q], &st.meta[q], xo, n, l32);
       __syncwarp();
     }
   }
@@ -263,10 +283,10 @@ __device__ __forceinline__ bool period_run_step(PeriodShared& ps,
   const int i = ch.beg + gq;
   float acc[3] = {0.f, 0.f, 0.f};
   if (s.R2 > 0.f) {
-    const int cnt = st.cnt[gq];
+    const int cnt = st.cnt(a, gq, i);
     uint32_t xo[3] = {0u, 0u, 0u};
 #pragma unroll
-    for (int k = 0; k < D; k++) xo[k] = st.xp[k][gq];
+    for (int k = 0; k < D; k++) xo[k] = st.xp(s, k, gq);
     const int ti = (int)(st.meta[gq] & 0xffu);
     const bool staged = nstg >= 0 && active && cnt <= lsmax;
     const bool ok = staged_walk<D, TPP, LPC, RX>(ps.sh, a, tb.rows, slots, sg, rec, codes + tid,
@@ -326,7 +346,7 @@ __device__ __forceinline__ bool period_run_step(PeriodShared& ps,
       U4 w0 = {0u, 0u, 0u, 0u};
       if (rx_next) w0 = U4{0u, 0u, st.w[P][0][tid], st.w[P][1][tid]};
       if (rx_next)
-        listed = rx_may_react<D>(s, (int)(mb & 0xff), st.rcnt[tid], pid, ps.s0 + n + 1, &w0);
+        listed = rx_may_react<D>(s, (int)(mb & 0xff), st.rcnt(a, tid, ib), pid, ps.s0 + n + 1, &w0);
       uint32_t h[3] = {0u, 0u, 0u}, l[3] = {0u, 0u, 0u}, q[3] = {0u, 0u, 0u};
 #pragma unroll
       for (int k = 0; k < D; k++) {
@@ -345,7 +365,6 @@ __device__ __forceinline__ bool period_run_step(PeriodShared& ps,
         for (int k = 0; k < D; k++) {
           st.xh[k][tid] = h[k];
           st.xl[k][tid] = l[k];
-          st.xp[k][tid] = q[k];
         }
       } else {
 #pragma unroll
@@ -379,7 +398,7 @@ __global__ void __launch_bounds__(LBLOCK, RD_PERIOD_MIN_BLOCKS)
   const PeriodTables tb = period_tables(a0, dyn);
   __shared__ PeriodShared ps;
   __shared__ PeriodStage<D, PER> st;
-  __shared__ float sacc[3][PER];
+  __shared__ float sacc[D][PER];
   // No early launch of the next kernel: its CTAs must not take the SM slots
   // that CTAs of this kernel still wait for.
   const Chunk ch = chunk_at<PER>(a0, (int)blockIdx.x);
@@ -411,15 +430,14 @@ __global__ void __launch_bounds__(LBLOCK, RD_PERIOD_MIN_BLOCKS)
   if (tid < ch.cnt) {
     const int ib = ch.beg + tid;
     st.pid[tid] = a0.pid[ib];
-    st.cnt[tid] = a0.ncnt[ib];
-    st.rcnt[tid] = a0.rcnt[ib];
+    st.cnts[tid] = min((unsigned int)a0.ncnt[ib], CNT_MANY) |
+                   min((unsigned int)a0.rcnt[ib], CNT_MANY) << 16;
     st.meta[tid] = a0.meta[ib];
 #pragma unroll
     for (int k = 0; k < D; k++) {
       st.xr[k][tid] = a0.xr[k][ib];
       st.xh[k][tid] = a0.xh[k][ib];
       st.xl[k][tid] = a0.xl[k][ib];
-      st.xp[k][tid] = a0.xp[k][ib];
     }
     listed = RX && p.first_rx && (a0.rec[0][ib].w & REC_PENDING);
   }
