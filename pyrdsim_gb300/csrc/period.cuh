@@ -28,9 +28,9 @@
 // the pair loop may call or spill: the spills of calls in it went to L2 (the
 // L1 is small beside the shared memory) and made the step 25 % slower.
 // Measured at 65,536 particles (wall fluid, 20-step launches, ncu): 201 us with
-// progress flags, an acquire per step and one polling warp, 150 us now; the LJ
-// fluid at 1,024 particles 70 -> 37 us per 10-step launch, 28 us with 4 lanes
-// per chain.
+// progress flags, an acquire per step and one polling warp, 150 us with records
+// and 139 with the L1 that PeriodStage leaves; the LJ fluid at 1,024 particles 70 ->
+// 37 us per 10-step launch, 28 us with 4 lanes per chain.
 //
 // LPC lanes share a chain (the entries of a row that one lane of the per-step
 // kernels walks), so that small systems, whose few chunks leave most of the
@@ -330,7 +330,7 @@ __device__ __forceinline__ bool period_run_step(PeriodShared& ps,
       const uint32_t mb = st.meta[tid];
       const int pid = st.pid[tid];
       wall_terms<D>(s, ps.sh.walls, t.xh, t.xl, (int)(mb & 0xff), accb);
-      add_bonded<D>(s, a, t.xh, t.xl, pid, mb, n, accb);
+      add_bonded<D, true>(s, a, t.xh, t.xl, pid, mb, n, accb);
       // (loaded here: nothing of it lives across the bonded terms' call)
 #pragma unroll
       for (int k = 0; k < D; k++) t.xr[k] = st.xr[k][tid];

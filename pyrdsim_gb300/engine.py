@@ -319,7 +319,7 @@ class Engine:
 
     def test_withhold(self, chunk):
         """Test hook: chunk ``chunk`` of the period kernel stops publishing
-        its progress (its neighbours' waits run out); -1 restores."""
+        its records (its neighbours' waits run out); -1 restores."""
         _check(self.lib.rdsim_test_withhold(self.h, int(chunk)))
 
     def set_profiling(self, on=True, stamps=False):

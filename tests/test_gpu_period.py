@@ -182,9 +182,9 @@ def test_period_lanes_and_frames(n):
     np.testing.assert_array_equal(one.reaction_rates(), per_step.reaction_rates())
 
 
-@pytest.mark.parametrize("n", [1, 63, 65, 4099])
+@pytest.mark.parametrize("n", [1, 63, 65, 4099, 250001])
 def test_lj_walk_equals_the_general_walk(n):
-    """A system whose pair laws are all Lennard-Jones n = 6 takes the drift
+    """A large system whose pair laws are all Lennard-Jones n = 6 takes the drift
     kernel's Lennard-Jones walk; adding a law between types that no particle
     has sends it through the general one.  Drifts and states are the same bit
     for bit, with rows within and beyond the stored list width."""
