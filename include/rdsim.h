@@ -49,7 +49,7 @@ enum {
                                  (Euclidean; dim = -1) between two rebuilds */
   RDSIM_ERR_NONFINITE = 19,   /* non-finite or larger-than-box displacement  */
   RDSIM_ERR_CAPACITY = 20,    /* a per-call buffer was too small             */
-  RDSIM_ERR_SYNC = 21         /* a wait of the period kernel on the progress
+  RDSIM_ERR_SYNC = 21         /* a wait of the period kernel on the records
                                  of neighbouring chunks ran out (no GPU hang:
                                  every CTA gives up and returns)           */
 };
@@ -159,7 +159,7 @@ typedef struct {
                                      may succeed (same results).  0: when few
                                      draws are expected to pass the bound;
                                      > 0: whenever the rates allow; < 0: off  */
-  int32_t period_kernel;          /* >= 0: graph-replayed rebuild periods run
+  int32_t period_kernel;          /* >= 0: rebuild periods (and parts of them) run
                                      as one launch of the period kernel when
                                      every chunk of particles fits on the GPU
                                      at once (same results); < 0: one drift
@@ -335,7 +335,7 @@ int rdsim_get_info(rdsim_handle* h, rdsim_info* info);
  * bracketed by CUDA events on the handle's stream and its device time summed
  * per class: 0 = drift (k_force_l), 1 = reactions (k_react_l,
  * k_react_listed), 2 = stand-alone Euler-Maruyama (k_em), 3 = cell-list and
- * Verlet-list rebuild (6 kernels), 4 = hooks and observables (the events
+ * Verlet-list rebuild (2, 5 or 6 kernels), 4 = hooks and observables (the events
  * serialise launches and keep graphs from replaying).  With bit 1 the drift
  * kernel itself (the period kernel alone, when rdsim_get_info reports it)
  * records the global timer when each CTA starts its work (after waiting for
@@ -355,7 +355,7 @@ int rdsim_set_profiling(rdsim_handle* h, int32_t enable);
 int rdsim_get_profile(rdsim_handle* h, rdsim_profile* p);
 
 /* Test hook, no counterpart in the reference: chunk `chunk` (a CTA of the
- * period kernel) stops publishing its progress, so that the waits of its
+ * period kernel) stops publishing its records, so that the waits of its
  * neighbours run out after sync_wait_ms and the next rdsim_step returns
  * RDSIM_ERR_SYNC.  -1 restores normal operation. */
 int rdsim_test_withhold(rdsim_handle* h, int32_t chunk);
