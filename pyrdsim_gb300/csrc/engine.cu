@@ -2058,6 +2058,27 @@ int rdsim_test_withhold(rdsim_handle* h, int32_t chunk) {
   return 0;
 }
 
+int rdsim_test_lists(rdsim_handle* h, int64_t* out) {
+  if (!h || !out) return fail(RDSIM_ERR_ARG, "null argument");
+  CK(cudaSetDevice(h->device));
+  std::vector<int> cnt(h->N), stg(h->period_on ? h->pchunks_h.size() : 0);
+  CK(cudaMemcpyAsync(cnt.data(), h->ncnt, sizeof(int) * cnt.size(), cudaMemcpyDeviceToHost, h->stream));
+  if (!stg.empty())
+    CK(cudaMemcpyAsync(stg.data(), h->stg_n, sizeof(int) * stg.size(), cudaMemcpyDeviceToHost, h->stream));
+  CK(cudaStreamSynchronize(h->stream));
+  const int coded = h->kw * 2 * h->ltpp * h->lpc;
+  std::memset(out, 0, 6 * sizeof *out);
+  out[0] = h->period_on ? h->lpc : 0;
+  out[1] = (int64_t)stg.size();
+  for (int n : stg) out[2] += n < 0;
+  for (int c : cnt) {
+    out[3] = std::max<int64_t>(out[3], c);
+    out[4] += c > h->W;
+    out[5] += c <= h->W && c > coded;
+  }
+  return 0;
+}
+
 }  // extern "C"
 
 // ---------------------------------------------------------------------------

@@ -17,7 +17,9 @@
 // that reads a particle is waited for by that particle's chunk: before a
 // particle's record of step n is overwritten (at the end of step n + 1) its
 // chunk has seen the step n + 1 record of a particle of every chunk that lists
-// it, and that chunk wrote it after it had read all records of step n.  A
+// it, and that chunk wrote it after it had read all records of step n.  (A chunk
+// that stages nothing waits for what it lists by gathering it, in every step
+// whose reactions read records, whatever the laws.)  A
 // staged run also holds particles that no row lists; their records may be one
 // buffer ahead, which the tag test accepts (they are not used).  Bonded
 // partners read each other's records and so order each other in the same way.
@@ -282,7 +284,10 @@ __device__ __forceinline__ bool period_run_step(PeriodShared& ps,
   const int gq = active ? g : 0;
   const int i = ch.beg + gq;
   float acc[3] = {0.f, 0.f, 0.f};
-  if (s.R2 > 0.f) {
+  // (an unstaged chunk walks its rows in a system without pair laws too: the
+  // gathers are its wait for the particles it lists, whose draws read its
+  // records)
+  if (s.R2 > 0.f || (RX && nstg < 0)) {
     const int cnt = st.cnt(a, gq, i);
     uint32_t xo[3] = {0u, 0u, 0u};
 #pragma unroll

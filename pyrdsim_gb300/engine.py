@@ -24,6 +24,7 @@ EXPORTS = [
     "rdsim_get_error", "rdsim_get_stream", "rdsim_get_info", "rdsim_last_error",
     "rdsim_set_profiling", "rdsim_get_profile", "rdsim_get_pairs_static",
     "rdsim_get_observables", "rdsim_get_rdf", "rdsim_test_withhold",
+    "rdsim_test_lists",
 ]
 
 
@@ -70,6 +71,7 @@ def load_library(path=None):
     L.rdsim_set_profiling.argtypes = [vp, C.c_int32]
     L.rdsim_get_profile.argtypes = [vp, C.POINTER(abi.Profile)]
     L.rdsim_test_withhold.argtypes = [vp, C.c_int32]
+    L.rdsim_test_lists.argtypes = [vp, C.POINTER(C.c_int64)]
     L.rdsim_last_error.restype = C.c_char_p
     if path is None:
         _lib = L
@@ -321,6 +323,14 @@ class Engine:
         """Test hook: chunk ``chunk`` of the period kernel stops publishing
         its records (its neighbours' waits run out); -1 restores."""
         _check(self.lib.rdsim_test_withhold(self.h, int(chunk)))
+
+    def test_lists(self):
+        """Test hook: the paths of the current list's rows in the period kernel
+        (counts; see rdsim_test_lists in include/rdsim.h)."""
+        out = (C.c_int64 * 6)()
+        _check(self.lib.rdsim_test_lists(self.h, out))
+        return dict(zip(("lanes", "chunks", "unstaged", "longest", "beyond_width",
+                         "beyond_codes"), out))
 
     def set_profiling(self, on=True, stamps=False):
         """``on``: CUDA events around every launch (serialised, no graphs);

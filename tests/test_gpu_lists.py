@@ -1,0 +1,68 @@
+"""Paths of the period kernel that only crowded places reach: chunks that touch
+more particles than they stage, rows longer than the slot codes, rows beyond
+the stored width.  States equal the per-step kernels' bit for bit."""
+import numpy as np
+import pytest
+
+from test_gpu_parity import _engine
+
+pytestmark = pytest.mark.gpu
+
+# particles, box, lanes per chain of the period kernel at that size
+SIZES = [(6001, 60.0, 4), (20011, 110.0, 2), (40009, 155.0, 1)]
+
+
+def _crowded(n, L, law, seed=1):
+    """3,000 particles in one corner of the box (a few hundred neighbours each),
+    ten clusters of 60, the others anywhere; three species that react."""
+    from pyrdsim_gb300 import model
+    rng = np.random.default_rng(seed)
+    x = rng.uniform(0.0, L, (n, 2))
+    x[:3000] = rng.uniform(1.0, 7.0, (3000, 2))
+    for q in range(10):
+        x[3000 + 60 * q:3060 + 60 * q] = [L - 4.0, 4.0 + 5.0 * q] + rng.uniform(-0.4, 0.4, (60, 2))
+    inter = [{"type": "tanh", "pair": [a, b], "u0": 0.02, "r0": 0.5, "a": 0.3, "rc": 1.0}
+             for a in range(3) for b in range(a, 3)] if law else []
+    m = model.Model.from_dict({
+        "n_dim": 2, "l": np.array([L, L]), "periodic": np.array([1.0, 1.0]), "dt": 1e-4,
+        "n_steps": 10, "n_out": 1000000, "tau_by_taud": np.ones(3), "seed": seed, "rs": 2.5,
+        "interactions": inter,
+        "reactions": [{"type": "locally_catalyzed", "reactant": 0, "product": 1, "catalyst": 1,
+                       "rate": 5.0, "r0": 1.0},
+                      {"type": "locally_inhibited", "reactant": 1, "product": 2, "rate": 60.0,
+                       "rate_decrease": 0.5, "inhibitor": 0, "inhibitor2": 2, "r0": 1.0},
+                      {"type": "linear", "reactant": 2, "product": 0, "rate": 30.0}]})
+    mol = np.stack([np.arange(n), np.zeros(n, int), np.zeros(n, int)], 1).astype(np.int32)
+    return model.SystemData(m, x, rng.integers(0, 3, n).astype(np.int32), mol,
+                            np.arange(n, dtype=np.int32))
+
+
+def _same_as_per_step(sd, calls, **kw):
+    """Steps the period kernel and the per-step kernels; returns the counts of
+    the start's list and the number of type changes."""
+    one, per_step = _engine([sd], **kw), _engine([sd], period_kernel=False, **kw)
+    lists = one.test_lists()
+    changed, prev = 0, one.state()[1]
+    for k in calls:
+        one.step(k)
+        per_step.step(k)
+        (xa, ta), (xb, tb) = one.state(), per_step.state()
+        np.testing.assert_array_equal(ta, tb)
+        np.testing.assert_array_equal(xa, xb)
+        changed += int((ta != prev).sum())
+        prev = ta
+    np.testing.assert_array_equal(one.drift(), per_step.drift())
+    one.close()
+    per_step.close()
+    return lists, changed
+
+
+@pytest.mark.parametrize("n,L,lanes", SIZES)
+def test_crowded_reactions_without_pair_laws(n, L, lanes):
+    """Reactions that count neighbours in a system without pair laws: a chunk that
+    stages nothing has no pair walk to hold it back, and must not run ahead of
+    the particles it lists."""
+    for _ in range(2):  # (the second run shows the same from run to run)
+        lists, changed = _same_as_per_step(_crowded(n, L, law=False), (7, 64, 130, 99))
+        assert lists["lanes"] == lanes and 0 < lists["unstaged"] < lists["chunks"], lists
+        assert changed > 500, changed
