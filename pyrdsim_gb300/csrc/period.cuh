@@ -167,13 +167,23 @@ __device__ __forceinline__ void period_noise(PeriodStage<D, PER>& st, const SysD
   }
 }
 
-// Phase A of a particle whose row or chunk is not staged.
-template <int D, int TPP>
-__device__ __noinline__ float3 period_gather(const ListShared& sh, const Args& a, int i, int lane,
+// Phase A of a particle whose row or chunk is not staged.  A row beyond the
+// stored width, where LPC lanes share a chain: each lane generates the whole row
+// and takes its chain's entries (row_scan's lanes are adjacent threads, the
+// chains here are not), so that the sums stay those of LPC = 1.
+template <int D, int TPP, int LPC>
+__device__ __noinline__ float3 period_gather(const ListShared& sh, const Args& a, int i, int chain,
                                              int cnt, uint3 x, uint32_t mi) {
   const uint32_t xo[3] = {x.x, x.y, x.z};
   float acc[3] = {0.f, 0.f, 0.f};
-  pair_drift<D, TPP, true>(sh, a, i, lane, cnt, xo, mi, acc);
+  if (LPC > 1 && cnt > a.W) {
+    row_scan<D, 1>(sh.sys, a, i, 0, [&](int k, int v) {
+      if (k % TPP == chain)
+        pair_term<D>(sh, a, i, (int)(mi & 0xff), xo, gather<D, true>(a, v), acc);
+    });
+  } else {
+    pair_drift<D, TPP, true>(sh, a, i, chain, cnt, xo, mi, acc);
+  }
   return make_float3(acc[0], acc[1], acc[2]);
 }
 
@@ -300,7 +310,7 @@ __device__ __forceinline__ bool period_run_step(PeriodShared& ps,
       const uint3 x = make_uint3(xo[0], xo[1], xo[2]);
       const float3 f =
           staged ? staged_slow<D, TPP, LPC>(ps.sh, a, slots, sg, codes, i, g, chain, cnt, x, ti)
-                 : period_gather<D, TPP>(ps.sh, a, i, chain, cnt, x, (uint32_t)ti);
+                 : period_gather<D, TPP, LPC>(ps.sh, a, i, chain, cnt, x, (uint32_t)ti);
       acc[0] = f.x;
       acc[1] = f.y;
       acc[2] = f.z;

@@ -66,3 +66,22 @@ def test_crowded_reactions_without_pair_laws(n, L, lanes):
         lists, changed = _same_as_per_step(_crowded(n, L, law=False), (7, 64, 130, 99))
         assert lists["lanes"] == lanes and 0 < lists["unstaged"] < lists["chunks"], lists
         assert changed > 500, changed
+
+
+@pytest.mark.parametrize("width,path", [(8, "beyond_width"), (200, "beyond_codes")])
+@pytest.mark.parametrize("n,L,lanes", SIZES)
+def test_long_rows_are_summed_in_list_order(n, L, lanes, width, path):
+    """Rows that the codes or the stored width do not hold, with 1, 2 and 4 lanes per
+    chain, in staged and unstaged chunks: the float32 sums in list order."""
+    lists, changed = _same_as_per_step(_crowded(n, L, law=True), (5, 44, 31), list_width=width)
+    assert lists["lanes"] == lanes and lists[path] > 0, lists
+    assert 0 < lists["unstaged"] < lists["chunks"] and changed > 100, (lists, changed)
+
+
+@pytest.mark.parametrize("n", [1009, 14593, 30011])
+def test_rows_beyond_the_width_of_a_fluid(n):
+    """The same in an even fluid, whose chunks are all staged."""
+    from pyrdsim_gb300 import workloads
+    sd = workloads.active_wall_fluid(n=n, seed=n, k_on=20.0, k_off=50.0)
+    lists, _ = _same_as_per_step(sd, (3, 58, 24), list_width=8)
+    assert lists["beyond_width"] > 100 and lists["unstaged"] == 0, lists
