@@ -168,6 +168,13 @@ __device__ inline void wait_failed(const Args& a, int n) {
   period_failed = 1;
 }
 
+// A drift summed from records, or NaN once a wait of this CTA ran out (the sum
+// may hold records of other steps): its update then leaves the particle in place.
+__device__ inline float3 unless_failed(float3 f) {
+  const float q = nanf("");
+  return *(volatile int*)&period_failed ? make_float3(q, q, q) : f;
+}
+
 // Polls a record until it is of step n (and, with `pend`, its draw is
 // resolved); after a failed wait the last value is used.  Out of line, for the
 // rare readers; the staging loop polls inline.
@@ -800,7 +807,7 @@ __device__ inline void wall_terms(const SysDev& s, const WallLaw* walls, const u
 template <int D>
 __device__ __noinline__ float3 bonded_call(const SysDev& s, const Args& a, Words own, int pid,
                                            uint32_t mi, int n, float3 acc0) {
-  return bonded_terms<D>(s, a, own, pid, mi, n, acc0);
+  return unless_failed(bonded_terms<D>(s, a, own, pid, mi, n, acc0));
 }
 
 // A particle's bonded terms, if it has any, added to acc.

@@ -184,7 +184,21 @@ __device__ __noinline__ float3 period_gather(const ListShared& sh, const Args& a
   } else {
     pair_drift<D, TPP, true>(sh, a, i, chain, cnt, xo, mi, acc);
   }
-  return make_float3(acc[0], acc[1], acc[2]);
+  return unless_failed(make_float3(acc[0], acc[1], acc[2]));
+}
+
+// A wait ran out, or another chunk recorded an error: the particles stay where
+// this chunk's last step left them.
+template <int D, int PER, bool RX>
+__device__ __noinline__ void leave_state(const SysDev& s, const PeriodStage<D, PER>& st,
+                                         const Args& a, int i, int p) {
+#pragma unroll
+  for (int k = 0; k < D; k++) {
+    a.xh_out[k][i] = st.xh[k][p];
+    a.xl_out[k][i] = st.xl[k][p];
+    a.xp_out[k][i] = st.xp(s, k, p);
+  }
+  if (RX) a.meta_out[i] = st.meta[p];
 }
 
 // Records a thread loads before it looks at their tags (1, 2, 4: 2,794 / 2,789
@@ -471,7 +485,10 @@ __global__ void __launch_bounds__(LBLOCK, RD_PERIOD_MIN_BLOCKS)
     a0.stamps[((size_t)slot * gridDim.x + blockIdx.x) * 2] = global_timer();
 #pragma unroll 1
   for (int n = 0; n < p.nsteps; n++)
-    if (!period_run_step<D, TPP, LPC, RX>(ps, st, tb, sacc, a0, p, ch, nstg, n)) return;
+    if (!period_run_step<D, TPP, LPC, RX>(ps, st, tb, sacc, a0, p, ch, nstg, n)) {
+      if (tid < ch.cnt) leave_state<D, PER, RX>(s, st, a0, ch.beg + tid, tid);
+      return;
+    }
   if (a0.stamps && (tid & 31) == 0)
     atomicMax(a0.stamps + ((size_t)slot * gridDim.x + blockIdx.x) * 2 + 1, global_timer());
 }

@@ -1,0 +1,41 @@
+"""What a handle holds after a call that failed: every particle its own last
+valid position, type and caller index."""
+import numpy as np
+import pytest
+
+from test_gpu_parity import _engine
+
+pytestmark = pytest.mark.gpu
+
+
+def _far(x, y, L):
+    d = x - y
+    d -= L * np.round(d / L)
+    return np.abs(d).max()
+
+
+@pytest.mark.parametrize("case", ["fluid", "patchy"])
+def test_state_after_a_period_that_gave_up(case):
+    """Chunks that give up inside a period (a neighbour's records never come)
+    leave their particles where their last step put them, not the words of a
+    buffer from before the last sort."""
+    from pyrdsim_gb300 import abi, workloads
+    from pyrdsim_gb300.engine import EngineError
+    sd = (workloads.active_wall_fluid(n=8192, seed=3) if case == "fluid"
+          else workloads.patchy_colloids(n_molecules=2048, seed=3))
+    # (launches of an odd number of steps end in the other buffer)
+    e = _engine([sd], sync_wait_ms=20, list_period=11)
+    L = np.asarray(sd.model.L, dtype=float)
+    e.step(10)
+    x0, t0 = e.state()
+    e.test_withhold(5)
+    for steps in (13, 8):  # steps 11 to 21, a whole period; 24 to 30, part of one
+        with pytest.raises(EngineError) as ei:
+            e.step(steps)
+        assert ei.value.code == abi.ERR_SYNC, str(ei.value)
+        x, t = e.state()
+        # at most the allowed displacement (half the skin) per period begun
+        assert _far(x, x0, L) < 2 * 0.5 * e.info()["skin"], _far(x, x0, L)
+        assert (t != t0).mean() < 0.01
+        x0, t0 = x, t
+    e.close()
