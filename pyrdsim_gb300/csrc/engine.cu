@@ -586,11 +586,10 @@ int check_device_error(rdsim_handle* h) {
 
 // Caller-order float64 positions and types in xbuf / tbuf (device) -> the
 // engine's state (fixed point, slot = caller index), converted exactly on
-// the device (fixed_from_double).
+// the device (fixed_from_double).  A state that is refused leaves the current
+// one, its cells and its lists as they are.
 int upload_state(rdsim_handle* h) {
   const int N = h->N;
-  h->cx = h->cm = h->co = 0;
-  CK(cudaMemsetAsync(h->flag_d, 0, sizeof(int), h->stream));
   StateOut a;
   std::memset(&a, 0, sizeof a);
   for (int k = 0; k < 3; k++) {
@@ -603,22 +602,20 @@ int upload_state(rdsim_handle* h) {
   a.pid = h->pid[0];
   a.n = N;
   const unsigned g = nblk(N);
-  if (h->D == 2)
-    k_from_double<2><<<g, 256, 0, h->stream>>>(h->sys_d, h->sid, h->xbuf, h->tbuf, h->meta_static_d,
-                                               h->mol_static_d, a, h->flag_d);
-  else if (h->D == 3)
-    k_from_double<3><<<g, 256, 0, h->stream>>>(h->sys_d, h->sid, h->xbuf, h->tbuf, h->meta_static_d,
-                                               h->mol_static_d, a, h->flag_d);
-  else
-    k_from_double<1><<<g, 256, 0, h->stream>>>(h->sys_d, h->sid, h->xbuf, h->tbuf, h->meta_static_d,
-                                               h->mol_static_d, a, h->flag_d);
+  auto check = h->D == 2 ? k_check_state<2> : h->D == 3 ? k_check_state<3> : k_check_state<1>;
+  auto convert = h->D == 2 ? k_from_double<2> : h->D == 3 ? k_from_double<3> : k_from_double<1>;
+  check<<<g, 256, 0, h->stream>>>(h->sys_d, h->sid, h->xbuf, h->tbuf, N, h->flag_d);
+  convert<<<g, 256, 0, h->stream>>>(h->sys_d, h->sid, h->xbuf, h->tbuf, h->meta_static_d,
+                                    h->mol_static_d, a, h->flag_d);
   CK(cudaGetLastError());
   int bad = 0;
   CK(cudaMemcpyAsync(&bad, h->flag_d, sizeof(int), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
+  if (bad) CK(cudaMemsetAsync(h->flag_d, 0, sizeof(int), h->stream));
   if (bad == 1) return fail(RDSIM_ERR_ARG, "initial position outside the reflecting box");
   if (bad == 2) return fail(RDSIM_ERR_ARG, "non-finite initial position");
   if (bad == 3) return fail(RDSIM_ERR_ARG, "particle type without tau_by_tauD entry");
+  h->cx = h->cm = h->co = 0;
   return 0;
 }
 
@@ -1442,6 +1439,9 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
   if ((rc = salloc(h, &h->meta_static_d, N))) return bail(rc);
   if ((rc = salloc(h, &h->mol_static_d, N))) return bail(rc);
   if ((rc = salloc(h, &h->flag_d, 1))) return bail(rc);
+  // zero between calls (upload_state)
+  if (cudaMemsetAsync(h->flag_d, 0, sizeof(int), h->stream) != cudaSuccess)
+    return bail(fail(RDSIM_ERR_CUDA, "memset"));
   if ((rc = salloc(h, &h->err, 1))) return bail(rc);
   if ((rc = salloc(h, &h->step_dev, 1))) return bail(rc);
   if ((rc = salloc(h, &h->pair_total, 2))) return bail(rc);

@@ -1370,9 +1370,7 @@ __global__ void k_to_double(const SysDev* sysv, const int* sid, Args a, double* 
 }
 
 // State upload: caller-order float64 positions x and types -> the fixed-point
-// arrays (slot = caller index), meta and molecule words.  bad receives the
-// first problem: 1 reflecting position outside [-L, L], 2 non-finite
-// position, 3 type without a tau_by_tauD entry.
+// arrays (slot = caller index), meta and molecule words.
 struct StateOut {
   uint32_t* xh[3];
   uint32_t* xl[3];
@@ -1383,37 +1381,44 @@ struct StateOut {
   int n;
 };
 
+// bad receives the first problem of a state: 1 reflecting position outside
+// [-L, L], 2 non-finite position, 3 type without a tau_by_tauD entry.  A kernel of
+// its own before k_from_double, so that a state that is refused leaves the
+// current one as it is.
+template <int D>
+__global__ void k_check_state(const SysDev* sysv, const int* sid, const double* x,
+                              const int* types, int n, int* bad) {
+  const int gi = blockIdx.x * blockDim.x + threadIdx.x;
+  if (gi >= n) return;
+  const SysDev& s = sysv[sid[gi]];
+  const int t = types[gi];
+  int code = t < 0 || t >= s.ntypes ? 3 : 0;
+#pragma unroll
+  for (int k = D - 1; k >= 0; k--) {
+    const double v = x[(size_t)gi * D + k];
+    if (!isfinite(v)) code = 2;
+    if (!((s.periodic >> k) & 1) && !(v >= -s.L[k] && v <= s.L[k] * (1.0 + 1e-9))) code = 1;
+  }
+  if (code) atomicCAS(bad, 0, code);
+}
+
+// Writes nothing if the check found a problem.
 template <int D>
 __global__ void k_from_double(const SysDev* sysv, const int* sid, const double* x,
                               const int* types, const uint32_t* meta_static,
-                              const int* mol_static, StateOut a, int* bad) {
-  pdl_trigger();
-  pdl_wait();
+                              const int* mol_static, StateOut a, const int* bad) {
   const int gi = blockIdx.x * blockDim.x + threadIdx.x;
-  if (gi >= a.n) return;
+  if (gi >= a.n || *bad) return;
   const SysDev& s = sysv[sid[gi]];
 #pragma unroll
   for (int k = 0; k < D; k++) {
-    const double v = x[(size_t)gi * D + k];
-    const bool per = (s.periodic >> k) & 1;
-    if (!per && !(v >= -s.L[k] && v <= s.L[k] * (1.0 + 1e-9))) {
-      atomicCAS(bad, 0, 1);
-      return;
-    }
     unsigned long long X = 0;
-    if (!fixed_from_double(v, s.L[k], per, s.Si[k], &X)) {
-      atomicCAS(bad, 0, 2);
-      return;
-    }
+    fixed_from_double(x[(size_t)gi * D + k], s.L[k], (s.periodic >> k) & 1, s.Si[k], &X);
     a.xh[k][gi] = (uint32_t)(X >> 32);
     a.xl[k][gi] = (uint32_t)X;
     a.xp[k][gi] = (uint32_t)(X >> s.ps[k]);
   }
   const int t = types[gi];
-  if (t < 0 || t >= s.ntypes) {
-    atomicCAS(bad, 0, 3);
-    return;
-  }
   a.meta[gi] = meta_static[gi] | (uint32_t)t | ((uint32_t)t << 8);
   a.mol[gi] = mol_static[gi];
   a.pid[gi] = gi;

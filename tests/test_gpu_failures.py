@@ -39,3 +39,37 @@ def test_state_after_a_period_that_gave_up(case):
         assert (t != t0).mean() < 0.01
         x0, t0 = x, t
     e.close()
+
+
+@pytest.mark.parametrize("bad", ["nan", "outside", "type"])
+def test_refused_state_changes_nothing(bad):
+    """set_state with one bad entry is refused; state, neighbour pairs, g(r),
+    observables and the steps after it are those of a handle that never saw it."""
+    from pyrdsim_gb300.engine import EngineError
+    from test_gpu_pairs import _fluid
+    sd = _fluid(1501, 40.0, 2, (1, -1), 3.0, seed=5, types=2)
+    e, ref = _engine([sd]), _engine([sd])
+    for h in (e, ref):
+        h.step(33)
+    x, t = e.state()
+    xb, tb = x[::-1].copy(), t[::-1].copy()  # other particles' places
+    if bad == "nan":
+        xb[700, 0] = np.nan
+    elif bad == "outside":
+        xb[700, 1] = 41.0
+    else:
+        tb[700] = 2
+    with pytest.raises(EngineError):
+        e.set_state(xb, tb)
+    for steps in (0, 14):
+        if steps:
+            for h in (e, ref):
+                h.step(steps)
+        for a, b in zip(e.state(), ref.state()):
+            np.testing.assert_array_equal(a, b)
+        np.testing.assert_array_equal(e.pairs(), ref.pairs())
+        np.testing.assert_array_equal(e.rdf_counts(9.0, 50), ref.rdf_counts(9.0, 50))
+        np.testing.assert_array_equal(e.drift(), ref.drift())
+        np.testing.assert_equal(e.observables(), ref.observables())
+    e.close()
+    ref.close()
