@@ -360,10 +360,11 @@ int rdsim_get_profile(rdsim_handle* h, rdsim_profile* p);
  * RDSIM_ERR_SYNC.  -1 restores normal operation. */
 int rdsim_test_withhold(rdsim_handle* h, int32_t chunk);
 /* Test hook, no counterpart in the reference: which paths the rows of the
- * current neighbour list take in the period kernel.  out[0..5]: lanes per chain
+ * current neighbour list take in the period kernel.  out[0..6]: lanes per chain
  * (0: the handle has no period kernel), chunks, chunks that touch more particles
  * than they stage, longest row, rows longer than the stored width, rows within
- * it that are longer than the slot codes. */
+ * it that are longer than the slot codes; 1 if neighbour pairs and g(r) look
+ * through every cell (after a call that ended with a device error). */
 int rdsim_test_lists(rdsim_handle* h, int64_t* out);
 
 /* Message of the last failing call on this thread. */

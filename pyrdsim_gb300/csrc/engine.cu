@@ -116,8 +116,8 @@ struct rdsim_handle {
   int obs_cap = 0;
   unsigned long long* rdf_counts = nullptr;  // [RDF_MAX_BINS]
   unsigned long long* pair_total = nullptr;  // [2]: neighbour pairs, longest row
-  // the last call ended with a device error: particles may be farther from
-  // their cells than the displacement check allows
+  // a call ended with a device error and none since then rebuilt the cells without
+  // one: particles may be farther from them than the displacement check allows
   bool moved_too_far = false;
   int ncells = 0, nscan = 0;
   int *cell_count = nullptr, *cell_start = nullptr, *bsum = nullptr;
@@ -1634,6 +1634,7 @@ int rdsim_step(rdsim_handle* h, int32_t n_steps, int32_t flags, const double* xi
   // reaction prefilter: needs the counter-based draws (not injected ones)
   const bool pre = h->rx_pre && h->has_rx && !inj;
   bool flagged = false;  // the last drift kernel flagged this step's draws
+  bool rebuilt = false;  // the call put the particles into their cells
   for (int q = 0; q < n_steps;) {
     const long long s = h->step + 1;
     const int left = n_steps - q;
@@ -1642,10 +1643,12 @@ int rdsim_step(rdsim_handle* h, int32_t n_steps, int32_t flags, const double* xi
       h->step = s + h->freq - 1;
       q += h->freq;
       flagged = false;
+      rebuilt = true;
       continue;
     }
     if (s % h->freq == 0) {
       if ((rc = rebuild(h, s, pre))) return rc;
+      rebuilt = true;
       flagged = pre;  // the builder listed this step's candidates
     }
     if (h->has_rx) {
@@ -1681,7 +1684,9 @@ int rdsim_step(rdsim_handle* h, int32_t n_steps, int32_t flags, const double* xi
     h->step = s;
     q++;
   }
-  return check_device_error(h);
+  rc = check_device_error(h);
+  if (!rc && rebuilt) h->moved_too_far = false;
+  return rc;
 }
 
 int rdsim_set_state(rdsim_handle* h, const double* x, const int32_t* types) {
@@ -2067,9 +2072,10 @@ int rdsim_test_lists(rdsim_handle* h, int64_t* out) {
     CK(cudaMemcpyAsync(stg.data(), h->stg_n, sizeof(int) * stg.size(), cudaMemcpyDeviceToHost, h->stream));
   CK(cudaStreamSynchronize(h->stream));
   const int coded = h->kw * 2 * h->ltpp * h->lpc;
-  std::memset(out, 0, 6 * sizeof *out);
+  std::memset(out, 0, 7 * sizeof *out);
   out[0] = h->period_on ? h->lpc : 0;
   out[1] = (int64_t)stg.size();
+  out[6] = h->moved_too_far;
   for (int n : stg) out[2] += n < 0;
   for (int c : cnt) {
     out[3] = std::max<int64_t>(out[3], c);

@@ -327,10 +327,10 @@ class Engine:
     def test_lists(self):
         """Test hook: the paths of the current list's rows in the period kernel
         (counts; see rdsim_test_lists in include/rdsim.h)."""
-        out = (C.c_int64 * 6)()
+        out = (C.c_int64 * 7)()
         _check(self.lib.rdsim_test_lists(self.h, out))
         return dict(zip(("lanes", "chunks", "unstaged", "longest", "beyond_width",
-                         "beyond_codes"), out))
+                         "beyond_codes", "every_cell"), out))
 
     def set_profiling(self, on=True, stamps=False):
         """``on``: CUDA events around every launch (serialised, no graphs);

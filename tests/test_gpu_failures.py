@@ -73,3 +73,31 @@ def test_refused_state_changes_nothing(bad):
         np.testing.assert_equal(e.observables(), ref.observables())
     e.close()
     ref.close()
+
+
+@pytest.mark.parametrize("graphs", [True, False])
+def test_pairs_use_their_cells_again_after_a_good_call(graphs):
+    """After a device error pairs are looked for in every cell; a later call that
+    rebuilds the cells and ends well makes that needless."""
+    from pyrdsim_gb300.engine import EngineError
+    from test_gpu_pairs import _distances, _fluid
+    sd = _fluid(1024, 40.0, 2, (1, 1), 3.0, seed=6)
+    e = _engine([sd], use_graphs=graphs, skin=0.04)
+    xi = np.zeros((3, 1024, 2))
+    xi[:, 5] = 10.0  # one particle moved by more than half the skin
+    # (steps 4 to 13 fail too, up to the rebuild of step 10; 14 to 18 have none)
+    for steps, every in ((0, 1), (10, 1), (5, 1), (20, 0)):
+        if steps == 0:
+            with pytest.raises(EngineError):
+                e.step(3, xi=xi, u1=np.ones((3, 1024)), u2=np.ones((3, 1024)))
+        elif steps == 10:
+            with pytest.raises(EngineError):
+                e.step(steps, noise=False)
+        else:
+            e.step(steps, noise=False)
+        r = _distances(e.state()[0], 40.0, (1, 1))
+        i, j = np.nonzero(np.triu(r <= 3.0, 1))
+        np.testing.assert_array_equal(e.pairs(),
+                                      np.stack([i, j], 1).astype(np.int32).reshape(-1, 2))
+        assert e.test_lists()["every_cell"] == every, steps
+    e.close()
