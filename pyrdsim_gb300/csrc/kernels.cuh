@@ -222,8 +222,9 @@ struct Words {
 // High and low words of particle j: in a period kernel from its records of
 // step n of the launch (other CTAs write them), else from the arrays.
 template <int D>
-__device__ inline void load_full(const Args& a, int j, int n, uint32_t* h, uint32_t* l) {
-  if (a.flags & F_PERIOD) {
+__device__ inline void load_full(const Args& a, bool period, int j, int n, uint32_t* h,
+                                 uint32_t* l) {
+  if (period) {
     const uint4 vl = get_rec(a, a.recl[n & 1] + j, 0, n);
     const uint4 vh = get_rec(a, a.rech[n & 1] + j, 0, n);
     const uint32_t hh[3] = {vh.x, vh.y, vh.z}, ll[3] = {vl.x, vl.y, vl.z};
@@ -241,27 +242,18 @@ __device__ inline void load_full(const Args& a, int j, int n, uint32_t* h, uint3
   }
 }
 
-// The loads of load_full (j < 0: none) without the wait: the tags still have to
-// be looked at in a period kernel.
+// The records of load_full (j < 0: none) without the wait: the tags still have to
+// be looked at.
 struct RawWords {
   uint4 h, l;
 };
 
-template <int D>
 __device__ inline RawWords load_raw(const Args& a, int j, int n) {
   RawWords r;
   r.h = r.l = make_uint4(0u, 0u, 0u, (uint32_t)n);
-  if (j < 0) return r;
-  if (a.flags & F_PERIOD) {
+  if (j >= 0) {
     r.h = ld_rec(a.rech[n & 1] + j);
     r.l = ld_rec(a.recl[n & 1] + j);
-  } else {
-    r.h.x = a.xh[0][j];
-    r.l.x = a.xl[0][j];
-    if (D > 1) r.h.y = a.xh[1][j];
-    if (D > 1) r.l.y = a.xl[1][j];
-    if (D > 2) r.h.z = a.xh[2][j];
-    if (D > 2) r.l.z = a.xl[2][j];
   }
   return r;
 }
@@ -274,8 +266,8 @@ __device__ __noinline__ double exact_dist(const SysDev& s, const Args& a, int gi
   double d2 = 0.0;
   uint32_t hi[3], li[3], hj[3], lj[3];
   const int n = (a.flags & F_PERIOD) ? period_n : 0;
-  load_full<D>(a, gi, n, hi, li);
-  load_full<D>(a, gj, n, hj, lj);
+  load_full<D>(a, (a.flags & F_PERIOD) != 0, gi, n, hi, li);
+  load_full<D>(a, (a.flags & F_PERIOD) != 0, gj, n, hj, lj);
 #pragma unroll
   for (int k = 0; k < D; k++) {
     double xi = fixed_to_double(s, k, hi[k], li[k]);
@@ -623,9 +615,16 @@ __device__ inline void em_update(const SysDev& s, const Args& a, int gi, int pid
 // Bonded terms of one particle (pyrdsim.pyx:2037-2066), gathered: the
 // particle evaluates every bond and angle it takes part in, reading its
 // partners' positions through slot_of (caller index -> sorted slot).  own: its
-// words; n: a period kernel's step within the launch.  Returns acc0 plus the
-// terms.
-template <int D>
+// words; PERIOD: in a period kernel, at step n of the launch.  Returns acc0 plus
+// the terms.
+//
+// In the period kernel the bond partners' records are loaded three terms ahead
+// (one round trip for a particle of up to three bonds instead of one per bond).
+// Not in the per-step kernels, where other warps hide the loads and the words of
+// three partners went to local memory (k_force_l in 2D, bytes of spills stored /
+// loaded: 164 / 216 with it, 72 / 112 without; 80,000 bonded particles 24.7 us per
+// step with it, 21.9 without; wall fluid at 1,048,576 112 and 105).
+template <int D, bool PERIOD>
 __device__ __forceinline__ float3 bonded_terms(const SysDev& s, const Args& a, Words own, int pid,
                                             uint32_t mi, int n, float3 acc0) {
   float acc[3] = {acc0.x, acc0.y, acc0.z};
@@ -636,33 +635,44 @@ __device__ __forceinline__ float3 bonded_terms(const SysDev& s, const Args& a, W
   const int mbase = pid - loc;
   float xo[3];
   const int eb = a.atomterm[T.atom0 + loc], ee = a.atomterm[T.atom0 + loc + 1];
-  // the bond partners' words are loaded three terms ahead (one round trip for a
-  // particle of up to three bonds instead of one per bond)
   auto partner = [&](int e) {
     if (e >= ee) return -1;
     const int code = a.atomterm[e];
     const TermDev& tr = a.terms[code >> 2];
     return tr.kind == RDSIM_TERM_BOND ? a.slot_of[mbase + ((code & 3) == 0 ? tr.j : tr.i)] : -1;
   };
-  int j0 = partner(eb), j1 = partner(eb + 1), j2 = partner(eb + 2);
-  RawWords r0 = load_raw<D>(a, j0, n), r1 = load_raw<D>(a, j1, n), r2 = load_raw<D>(a, j2, n);
+  int j0 = 0, j1 = 0, j2 = 0;
+  RawWords r0, r1, r2;
+  if (PERIOD) {
+    j0 = partner(eb);
+    j1 = partner(eb + 1);
+    j2 = partner(eb + 2);
+    r0 = load_raw(a, j0, n);
+    r1 = load_raw(a, j1, n);
+    r2 = load_raw(a, j2, n);
+  }
 #pragma unroll 1
   for (int e = eb; e < ee; e++) {
     const int code = a.atomterm[e];
     const TermDev& tr = a.terms[code >> 2];
     const int role = code & 3;
-    const int other = j0;
-    RawWords cur = r0;
-    r0 = r1;
-    j0 = j1;
-    r1 = r2;
-    j1 = j2;
-    j2 = partner(e + 3);
-    r2 = load_raw<D>(a, j2, n);
-    if (tr.kind == RDSIM_TERM_BOND) {
+    uint32_t oh[3] = {0u, 0u, 0u}, ol[3] = {0u, 0u, 0u};
+    if (PERIOD) {
+      const int other = j0;
+      RawWords cur = r0;
+      r0 = r1;
+      j0 = j1;
+      r1 = r2;
+      j1 = j2;
+      j2 = partner(e + 3);
+      r2 = load_raw(a, j2, n);
       if (!rec_ready(cur.l.w, 0, n)) cur.l = rec_wait(a, a.recl[n & 1] + other, 0, n, false);
       if (!rec_ready(cur.h.w, 0, n)) cur.h = rec_wait(a, a.rech[n & 1] + other, 0, n, false);
-      const uint32_t oh[3] = {cur.h.x, cur.h.y, cur.h.z}, ol[3] = {cur.l.x, cur.l.y, cur.l.z};
+      oh[0] = cur.h.x, oh[1] = cur.h.y, oh[2] = cur.h.z;
+      ol[0] = cur.l.x, ol[1] = cur.l.y, ol[2] = cur.l.z;
+    }
+    if (tr.kind == RDSIM_TERM_BOND) {
+      if (!PERIOD) load_full<D>(a, false, partner(e), n, oh, ol);
       // f = k (d - r0) / d (pyrdsim.pyx:2037-2047).  A stiff bond near rest
       // cancels in d - r0: where every dimension has the same fixed unit,
       // d^2 - r0^2 is formed exactly in 128-bit integers (units unit^2) and
@@ -701,9 +711,9 @@ __device__ __forceinline__ float3 bonded_terms(const SysDev& s, const Args& a, W
                 s3 = a.slot_of[mbase + tr.k];
       float v1[3], v2[3], n1 = 0.f, n2 = 0.f;
       uint32_t h1[3], l1[3], h2[3], l2[3], h3[3], l3[3];
-      load_full<D>(a, s1, n, h1, l1);
-      load_full<D>(a, s2, n, h2, l2);
-      load_full<D>(a, s3, n, h3, l3);
+      load_full<D>(a, PERIOD, s1, n, h1, l1);
+      load_full<D>(a, PERIOD, s2, n, h2, l2);
+      load_full<D>(a, PERIOD, s3, n, h3, l3);
 #pragma unroll
       for (int k = 0; k < D; k++) {
         v1[k] = disp_full(s, k, h2[k], l2[k], h1[k], l1[k]);
@@ -807,7 +817,7 @@ __device__ inline void wall_terms(const SysDev& s, const WallLaw* walls, const u
 template <int D>
 __device__ __noinline__ float3 bonded_call(const SysDev& s, const Args& a, Words own, int pid,
                                            uint32_t mi, int n, float3 acc0) {
-  return unless_failed(bonded_terms<D>(s, a, own, pid, mi, n, acc0));
+  return unless_failed(bonded_terms<D, true>(s, a, own, pid, mi, n, acc0));
 }
 
 // A particle's bonded terms, if it has any, added to acc.
@@ -818,7 +828,7 @@ __device__ inline void add_bonded(const SysDev& s, const Args& a, const uint32_t
     const Words own = {{xh[0], xh[1], xh[2]}, {xl[0], xl[1], xl[2]}};
     const float3 a0 = make_float3(acc[0], D > 1 ? acc[1] : 0.f, D > 2 ? acc[2] : 0.f);
     const float3 b = CALL ? bonded_call<D>(s, a, own, pid, mi, n, a0)
-                          : bonded_terms<D>(s, a, own, pid, mi, n, a0);
+                          : bonded_terms<D, false>(s, a, own, pid, mi, n, a0);
     acc[0] = b.x;
     if (D > 1) acc[1] = b.y;
     if (D > 2) acc[2] = b.z;
