@@ -367,6 +367,11 @@ int rdsim_test_withhold(rdsim_handle* h, int32_t chunk);
  * through every cell (after a call that ended with a device error). */
 int rdsim_test_lists(rdsim_handle* h, int64_t* out);
 
+/* Test hook, no counterpart in the reference: the per-step drift kernel's
+ * Lennard-Jones walk wherever the laws allow it (1), never (-1), or by the
+ * system's size (0, the default). */
+int rdsim_test_lj_walk(rdsim_handle* h, int32_t mode);
+
 /* Message of the last failing call on this thread. */
 const char* rdsim_last_error(void);
 

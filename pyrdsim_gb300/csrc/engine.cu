@@ -144,6 +144,7 @@ struct rdsim_handle {
   uint4* recl[2] = {};
   uint4* rech[2] = {};
   int withhold = -1;                 // test hook (rdsim_test_withhold)
+  int lj_walk = 0;                   // test hook (rdsim_test_lj_walk)
   long long wait_ns = 1000000000LL;
   std::vector<Chunk> chunks_h;
   Chunk* chunks_d = nullptr;
@@ -493,7 +494,11 @@ int force(rdsim_handle* h, long long step, int flags, const double* xi_next, boo
       a.chunks = h->fchunks_d;
       CK(launch_force64(h->D, h->ltpp, h->fpw, h->fchunks, h->stream, a));
     }
-    if (!h->f64) CK(launch_force32(h->D, h->ltpp, h->all_lj6, (unsigned)h->chunks_h.size(), h->stream, a));
+    if (!h->f64) {
+      const unsigned g = (unsigned)h->chunks_h.size();
+      const bool lj = h->all_lj6 && (h->lj_walk > 0 || (h->lj_walk == 0 && g > LJ_MIN_CHUNKS));
+      CK(launch_force32(h->D, h->ltpp, lj, g, h->stream, a));
+    }
   }
   CK(cudaGetLastError());
   if (flags & F_EM) h->cx = 1 - h->cx;
@@ -2058,6 +2063,16 @@ int rdsim_test_withhold(rdsim_handle* h, int32_t chunk) {
   CK(cudaStreamSynchronize(h->stream));
   h->withhold = chunk;
   // periods are captured with the hook's value: recapture
+  for (auto& g : h->graph_cache) cudaGraphExecDestroy(g.second.exec);
+  h->graph_cache.clear();
+  return 0;
+}
+
+int rdsim_test_lj_walk(rdsim_handle* h, int32_t mode) {
+  if (!h) return fail(RDSIM_ERR_ARG, "null handle");
+  CK(cudaSetDevice(h->device));
+  CK(cudaStreamSynchronize(h->stream));
+  h->lj_walk = mode;
   for (auto& g : h->graph_cache) cudaGraphExecDestroy(g.second.exec);
   h->graph_cache.clear();
   return 0;

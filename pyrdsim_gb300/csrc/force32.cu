@@ -23,17 +23,10 @@ ForceKernel kernel_of(int tpp, bool lj6) {
   return lj6 ? kernel_of<D, true>(tpp) : kernel_of<D, false>(tpp);
 }
 
-// Chunks from which the Lennard-Jones walk's 12 CTAs per SM pay: two rounds of
-// the GPU.  With fewer, the next launch finds no free slot to stage its tables
-// in (100,000 particles: 19.1 us per step with the general walk, 21.4 with it;
-// 250,000: 35 either way; 1,048,576: 133, 114).
-constexpr unsigned LJ_MIN_CHUNKS = 2 * 12 * 152;
-
 }  // namespace
 
 cudaError_t launch_force32(int D, int tpp, bool lj6, unsigned chunks, cudaStream_t st,
                            const Args& a) {
-  lj6 = lj6 && chunks > LJ_MIN_CHUNKS;
   launch(D == 2 ? kernel_of<2>(tpp, lj6) : D == 3 ? kernel_of<3>(tpp, lj6) : kernel_of<1>(tpp, lj6),
          chunks, LBLOCK, st, a);
   return cudaGetLastError();

@@ -7,7 +7,14 @@
 
 namespace rd {
 
-// lj6: every pair law of every system is a single Lennard-Jones n = 6 law.
+// Chunks from which the Lennard-Jones walk's 12 CTAs per SM pay: two rounds of
+// the GPU.  With fewer, the next launch finds no free slot to stage its tables
+// in (100,000 particles: 19.1 us per step with the general walk, 21.4 with it;
+// 250,000: 35 either way; 1,048,576: 133, 114).
+constexpr unsigned LJ_MIN_CHUNKS = 2 * 12 * 152;
+
+// lj6: the Lennard-Jones walk (every pair law of every system is then a single
+// Lennard-Jones n = 6 law).
 cudaError_t launch_force32(int D, int tpp, bool lj6, unsigned chunks, cudaStream_t st,
                            const Args& a);
 

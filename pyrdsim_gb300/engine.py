@@ -24,7 +24,7 @@ EXPORTS = [
     "rdsim_get_error", "rdsim_get_stream", "rdsim_get_info", "rdsim_last_error",
     "rdsim_set_profiling", "rdsim_get_profile", "rdsim_get_pairs_static",
     "rdsim_get_observables", "rdsim_get_rdf", "rdsim_test_withhold",
-    "rdsim_test_lists",
+    "rdsim_test_lists", "rdsim_test_lj_walk",
 ]
 
 
@@ -71,6 +71,7 @@ def load_library(path=None):
     L.rdsim_set_profiling.argtypes = [vp, C.c_int32]
     L.rdsim_get_profile.argtypes = [vp, C.POINTER(abi.Profile)]
     L.rdsim_test_withhold.argtypes = [vp, C.c_int32]
+    L.rdsim_test_lj_walk.argtypes = [vp, C.c_int32]
     L.rdsim_test_lists.argtypes = [vp, C.POINTER(C.c_int64)]
     L.rdsim_last_error.restype = C.c_char_p
     if path is None:
@@ -323,6 +324,11 @@ class Engine:
         """Test hook: chunk ``chunk`` of the period kernel stops publishing
         its records (its neighbours' waits run out); -1 restores."""
         _check(self.lib.rdsim_test_withhold(self.h, int(chunk)))
+
+    def test_lj_walk(self, mode):
+        """Test hook: the per-step Lennard-Jones walk wherever the laws allow
+        it (1), never (-1), by size (0)."""
+        _check(self.lib.rdsim_test_lj_walk(self.h, int(mode)))
 
     def test_lists(self):
         """Test hook: the paths of the current list's rows in the period kernel
