@@ -1481,13 +1481,14 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
     // memory, and the others wait for it: 13,824 particles in 3D 13.4 us per step
     // with a third, 11.9 with half, 12.4 with twice; 65,536 in 2D 19.4 with a
     // tenth, 16.0 with a third or half)
-    double want = 64;
+    double touch = 0, want = 64;
     int largest = 1;
     for (const SysDev& sd : h->sys_h) {
       double cells = 1;
       for (int k = 0; k < D; k++) cells *= sd.nc[k];
       const double rows = D == 3 ? 9 : (D == 2 ? 3 : 1);
-      want = std::max(want, rows * (per + 3.0 * sd.n / cells) * (D == 3 ? 1.5 : 1.3) + 64);
+      touch = std::max(touch, rows * (per + 3.0 * sd.n / cells));
+      want = std::max(want, touch * (D == 3 ? 1.5 : 1.3) + 64);
       largest = std::max(largest, sd.n);
       h->rows = std::max(h->rows, sd.ntypes * sd.ntypes);
     }
@@ -1498,9 +1499,15 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
     const int row = std::min(h->W, (int)(1.5 * list_expect) + 12), lanes = 2 * h->ltpp * h->lpc;
     h->kw = std::min((row + lanes - 1) / lanes, KW_LIMIT);
     // every chunk resident at once (its CTAs wait for each other), with less
-    // room for staging if need be
+    // room for staging if need be, but for a tenth more than the chunks touch:
+    // where they do not fit their tables the per-step kernels are faster (3D,
+    // 39,304 and 46,656 particles, us per step: 47.3 and 49.1 with tables too
+    // small, 43.4 and 43.9 with the per-step kernels; at 32,768 40.9 with the
+    // latter, 39.8 with the largest table that fits, 1.4 times the touched; 2D,
+    // cutoff 5, 60,000: 33.7 with the latter, 32.6 with 1.2 times)
     const PeriodVariant v{D, h->ltpp, h->lpc, h->has_rx};
-    for (int m = h->stg_max; m >= 64 && m >= h->stg_max / 4 && !h->period_on; m = m / 128 * 64) {
+    const int least = std::min(h->stg_max, slots(1.1 * touch));
+    for (int m = h->stg_max; m >= least && !h->period_on; m -= 64) {
       const long long room = (long long)period_blocks_per_sm(v, m, h->kw, h->rows) * sms;
       if (room >= nch) {
         h->period_on = true;

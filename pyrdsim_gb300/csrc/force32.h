@@ -9,8 +9,8 @@ namespace rd {
 
 // Chunks from which the Lennard-Jones walk's 12 CTAs per SM pay: two rounds of
 // the GPU.  With fewer, the next launch finds no free slot to stage its tables
-// in (100,000 particles: 19.1 us per step with the general walk, 21.4 with it;
-// 250,000: 35 either way; 1,048,576: 133, 114).
+// in (us per step with the general walk / with it: 18.9 / 20.0 at 100,000
+// particles, 28.5 / 28.8 at 200,000, 33.9 / 32.9 at 250,000, 130 / 105 at 1,048,576).
 constexpr unsigned LJ_MIN_CHUNKS = 2 * 12 * 152;
 
 // lj6: the Lennard-Jones walk (every pair law of every system is then a single

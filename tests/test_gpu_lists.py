@@ -85,3 +85,25 @@ def test_rows_beyond_the_width_of_a_fluid(n):
     sd = workloads.active_wall_fluid(n=n, seed=n, k_on=20.0, k_off=50.0)
     lists, _ = _same_as_per_step(sd, (3, 58, 24), list_width=8)
     assert lists["beyond_width"] > 100 and lists["unstaged"] == 0, lists
+
+
+@pytest.mark.parametrize("n,D,rc,period", [(13824, 3, 2.5, 1), (35937, 3, 2.5, 1),
+                                           (46656, 3, 2.5, 0), (60000, 2, 5.0, 1)])
+def test_period_kernel_only_where_its_tables_hold_a_chunk(n, D, rc, period):
+    """Large tables are cut to make every chunk resident; a system whose chunks would
+    no longer fit them takes the per-step kernels."""
+    from pyrdsim_gb300 import model
+    rng = np.random.default_rng(1)
+    L = np.full(D, (n / 0.5) ** (1.0 / D))
+    side = int(np.ceil(n ** (1.0 / D)))
+    g = np.stack(np.meshgrid(*[np.arange(side)] * D, indexing="ij"), -1).reshape(-1, D)[:n]
+    x = (g + 0.5 + rng.uniform(-0.1, 0.1, (n, D))) * (L / side)
+    m = model.Model.from_dict({
+        "n_dim": D, "l": L, "periodic": np.ones(D), "dt": 1e-4, "n_steps": 10, "n_out": 1000000,
+        "tau_by_taud": np.ones(1), "seed": 1,
+        "interactions": [{"type": "yukawa", "pair": [0, 0], "u0": 10.0, "r0": 1.0, "rc": rc}]})
+    mol = np.stack([np.arange(n), np.zeros(n, int), np.zeros(n, int)], 1).astype(np.int32)
+    sd = model.SystemData(m, x, np.zeros(n, np.int32), mol, np.arange(n, dtype=np.int32))
+    e = _engine([sd])
+    assert e.info()["period_kernel"] == period, e.test_lists()
+    e.close()
