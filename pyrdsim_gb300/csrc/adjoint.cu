@@ -70,7 +70,7 @@ struct AdjArgs {
   float Lf[3], Linvf[3];
   int exact_image;              // boxes near 2 rc: float64 decides the image
   float cut2f;                  // float32 screen of the list in use
-  float move2f;                 // displacement^2 allowed while a list is reused                  // float32 screen: above the largest rc^2
+  float move2f;                 // displacement^2 allowed while a list is reused
   double c[MAXT], s[MAXT];      // dt D and sqrt(2 dt D) per type
   double wU, wW;                // loss weights 1/K and 1/(K d V)
   unsigned char lawmask[MAXT * MAXT];  // bit l: law l applies to (ti, tj)
@@ -86,7 +86,7 @@ struct PairEval {
   double U, f, fp, dU[2], df[2];
 };
 
-__host__ __device__ inline double lj_power(double q, int n) {
+inline double lj_power(double q, int n) {
   // (r0 / r)^n from q = r0 / r
   if (n == 6) {
     const double q2 = q * q;
@@ -97,7 +97,7 @@ __host__ __device__ inline double lj_power(double q, int n) {
   return s;
 }
 
-__host__ __device__ inline PairEval eval_law(const Law& w, double r, double ir) {
+inline PairEval eval_law(const Law& w, double r, double ir) {
   PairEval p;
   if (w.law == RDSIM_LAW_LJ) {
     // U = u0 (s^2 - 2 s), s = (r0/r)^n; f = -2 n u0 s (s - 1) / r
@@ -342,7 +342,7 @@ __device__ inline double pair_vec(const AdjArgs& g, const double* __restrict__ x
 }
 
 // One law at squared distance r2 < rc2, in the form the kernels use it:
-// U, fr = f / r, and (WANT_G) fp = f' and the derivatives of U and f / r by
+// U, fr = f / r, fp = f' and the derivatives of U and f / r by
 // (u0, r0).  Lennard-Jones laws of even power take a reciprocal, no root.
 struct PairD {
   double U, fr, fp, dU[2], dfr[2], w;

@@ -219,7 +219,8 @@ struct Args {
   uint4* rec[2];                  // pair words, type word with the step's tag
   uint4* recl[2];                 // low words, tag
   uint4* rech[2];                 // high words, tag
-  long long wait_ns;              // period kernel: limit of one wait (ns)
+  long long wait_ns;              // period kernel: limit of one wait (global
+                                  // timer, ns)
 };
 
 // Type word of a period kernel's record: the type after the step's reactions
@@ -253,7 +254,6 @@ struct PeriodArgs {
                                   // before the launch
   int withhold;                   // test hook: this chunk never publishes
                                   // its records (-1: none)
-  long long wait_ns;              // limit of one wait (global timer, ns)
 };
 
 __device__ inline unsigned long long global_timer() {

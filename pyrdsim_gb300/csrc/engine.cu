@@ -659,7 +659,6 @@ int period_launch(rdsim_handle* h, int kf, bool pre, bool rel = true, long long 
   p.nsteps = rel ? h->freq : nsteps;
   p.first_rx = rel ? 1 : 0;
   p.withhold = h->withhold;
-  p.wait_ns = h->wait_ns;
   // the launch leaves the state where the per-step kernels would: one flip
   // per update, one per reaction step
   const int cx = h->cx ^ (p.nsteps & 1);

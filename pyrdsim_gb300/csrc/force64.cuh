@@ -20,27 +20,6 @@
 
 namespace rd {
 
-// A list entry with the neighbour's full fixed-point words.
-struct NbF {
-  uint32_t h[3], l[3];
-  uint32_t m;
-  int v;
-};
-
-template <int D>
-__device__ inline NbF gather_full(const Args& a, int v) {
-  NbF n;
-  const int j = v & 0x7fffffff;
-  n.v = v;
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    n.h[k] = k < D ? a.xh[k][j] : 0u;
-    n.l[k] = k < D ? a.xl[k][j] : 0u;
-  }
-  n.m = a.meta[j];
-  return n;
-}
-
 __device__ inline unsigned long long fixed_word(uint32_t h, uint32_t l) {
   return ((unsigned long long)h << 32) | l;
 }

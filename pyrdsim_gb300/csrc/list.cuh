@@ -460,11 +460,10 @@ __host__ __device__ constexpr int nlist_lane_threads(int per) {
 template <int D, int TPP, int LPC>
 __global__ void __launch_bounds__(nlist_threads(D, LBLOCK / TPP / LPC)) k_nlist(Args a) {
   constexpr int PER = LBLOCK / TPP / LPC;
-  constexpr int NT = D == 1 ? 1 : 3;
+  static_assert(D < 3, "the lanes form builds rows in 3D");
+  constexpr int NT = D == 1 ? 1 : 3;  // threads per particle, a row of cells each
   constexpr int NTH = PER * NT;
-  constexpr int NROW = D == 3 ? 9 : (D == 2 ? 3 : 1);
-  constexpr int RPT = NROW / NT;  // rows per thread
-  constexpr int NRUN = 2 * RPT;
+  constexpr int NRUN = 2;
   constexpr int U = 4;
   constexpr int BCAP = 24;
   __shared__ SysDev sys;
@@ -512,22 +511,17 @@ __global__ void __launch_bounds__(nlist_threads(D, LBLOCK / TPP / LPC)) k_nlist(
   const uint32_t bmask = tmi != 0xff ? a.tmpl[tmi].bondmask[loci] : 0u;
   const float Rl2 = s.Rl2;
   const int h1 = D > 1 ? s.halo[1] : 0;
-  const int h2 = D > 2 ? s.halo[2] : 0;
   int rb[NRUN], re[NRUN];
-#pragma unroll
-  for (int r = 0; r < RPT; r++) {
-    const int q = t * RPT + r;
-    const int dz = D == 3 ? q / 3 - 1 : 0;
-    const int dy = D >= 2 ? q % 3 - 1 : 0;
+  {
+    const int dy = D == 2 ? t - 1 : 0;
     int row, lo0, hi0, lo1, hi1;
-    const bool ok = valid && dy >= -h1 && dy <= h1 && dz >= -h2 && dz <= h2 &&
-                    row_runs<D>(s, c, dy, dz, row, lo0, hi0, lo1, hi1);
+    const bool ok = valid && dy >= -h1 && dy <= h1 && row_runs<D>(s, c, dy, 0, row, lo0, hi0, lo1, hi1);
     const int* cs = a.cell_start + s.c0 + row;
-    rb[2 * r] = ok ? cs[lo0] : 0;
-    re[2 * r] = ok ? cs[hi0 + 1] : 0;
+    rb[0] = ok ? cs[lo0] : 0;
+    re[0] = ok ? cs[hi0 + 1] : 0;
     const bool two = ok && hi1 >= lo1;
-    rb[2 * r + 1] = two ? cs[lo1] : 0;
-    re[2 * r + 1] = two ? cs[hi1 + 1] : 0;
+    rb[1] = two ? cs[lo1] : 0;
+    re[1] = two ? cs[hi1 + 1] : 0;
   }
   // the listed pairs of this thread's rows, in candidate order: emit(k, entry,
   // squared distance)
