@@ -107,3 +107,34 @@ def test_period_kernel_only_where_its_tables_hold_a_chunk(n, D, rc, period):
     e = _engine([sd])
     assert e.info()["period_kernel"] == period, e.test_lists()
     e.close()
+
+
+@pytest.mark.parametrize("types", [3, 16])
+@pytest.mark.parametrize("tpp", [1, 2, 4, 8])
+@pytest.mark.parametrize("n,D", [(131, 1), (2177, 2), (1031, 3)])
+def test_period_kernel_of_every_variant(n, D, tpp, types):
+    """1 to 8 lanes per particle in 1D to 3D, up to the most species, reflecting and
+    periodic edges, two laws on some pairs, reactions that count neighbours."""
+    from pyrdsim_gb300 import model
+    rng = np.random.default_rng(n + types)
+    side = int(np.ceil(n ** (1.0 / D)))
+    g = np.stack(np.meshgrid(*[np.arange(side)] * D, indexing="ij"), -1).reshape(-1, D)
+    x = (g[rng.permutation(len(g))[:n]] + 0.5 + rng.uniform(-0.1, 0.1, (n, D))) * 1.4
+    pairs = [(a, b) for a in range(3) for b in range(a, 3)] + [(t, t) for t in range(3, types)]
+    m = model.Model.from_dict({
+        "n_dim": D, "l": np.full(D, 1.4 * side), "periodic": np.array([1.0] * (D - 1) + [-1.0]),
+        "dt": 1e-4, "n_steps": 10, "n_out": 1000000, "tau_by_taud": np.ones(types), "seed": n,
+        "rs": 3.6,
+        "interactions": [{"type": "lj", "pair": [a, b], "u0": 1.0, "r0": 1.1, "rc": 2.5, "n": 6}
+                         for a, b in pairs] +
+                        [{"type": "yukawa", "pair": [0, 1], "u0": 3.0, "r0": 1.0, "rc": 2.2}],
+        "reactions": [{"type": "linear", "reactant": 0, "product": types - 1, "rate": 30.0},
+                      {"type": "locally_catalyzed", "reactant": types - 1, "catalyst": 1,
+                       "product": 2, "rate": 5.0, "r0": 1.7},
+                      {"type": "locally_inhibited", "reactant": 2, "product": 0, "rate": 60.0,
+                       "rate_decrease": 2.0, "inhibitor": 1, "r0": 2.0}]})
+    mol = np.stack([np.arange(n), np.zeros(n, int), np.zeros(n, int)], 1).astype(np.int32)
+    sd = model.SystemData(m, x, rng.integers(0, types, n).astype(np.int32), mol,
+                          np.arange(n, dtype=np.int32))
+    lists, changed = _same_as_per_step(sd, (6, 47, 30), threads_per_particle=tpp)
+    assert lists["lanes"] == (4 if tpp == 2 and D < 3 else 1) and changed > 0, (lists, changed)
