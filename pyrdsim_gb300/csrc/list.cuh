@@ -46,9 +46,10 @@
 #endif
 // the same where every pair law is a single Lennard-Jones n = 6 law: more
 // warps in flight are worth the registers there (wall fluid, 1,048,576
-// particles, 40 steps: 5,329 us at 8 with the general walk; the walk of
-// lj_walk 5,676 / 5,059 / 4,860 us at 8 / 10 / 12, 8,450 us at 14, where it
-// spills in the loop; the general walk is slower at 7 and at 10 than at 8)
+// particles, 40 steps: 5,220 us at 8 with the general walk; the walk of
+// lj_walk 4,903 / 4,484 / 4,218 / 4,395 / 4,409 us at 8 / 10 / 12 / 14 / 16; the
+// general walk at 7 / 8 / 9 / 10: ensemble of 64, 30 steps, 2,254 / 2,133 /
+// 2,173 / 2,768 us, LJ fluid at 100,000, 60 steps, 1,120 / 1,125 / 1,179 / 1,405)
 constexpr int LJ_MIN_BLOCKS = 12;
 // list entries loaded per lane before their neighbours are gathered
 #ifndef RD_LIST_BATCH
@@ -1118,8 +1119,8 @@ __device__ __forceinline__ void pair_drift(const ListShared& sh, const Args& a, 
 // = 6 law: pair_drift's sums by a walk that holds no call and reads one row per
 // type pair (fill_rows).  Bound by the latency of the gathers: the neighbour of
 // the next entry and the index of the one after it are in flight while an entry
-// is evaluated (4,860 -> 4,679 us per 40 steps at 1,048,576 particles; two
-// entries at a time 4,679, one 4,630).  False at a distance in a cutoff's guard
+// is evaluated (4 % of the call at 1,048,576 particles; two entries at a time 1 %
+// slower).  False at a distance in a cutoff's guard
 // band (the lane then takes pair_drift).  Rows within the stored width only.
 template <int D, int TPP>
 __device__ __forceinline__ bool lj_walk(const ListShared& sh, const Args& a, const float4* rows,

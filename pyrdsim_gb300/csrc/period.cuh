@@ -18,11 +18,11 @@
 // particle's record of step n is overwritten (at the end of step n + 1) its
 // chunk has seen the step n + 1 record of a particle of every chunk that lists
 // it, and that chunk wrote it after it had read all records of step n.  (A chunk
-// that stages nothing waits for what it lists by gathering it, in every step
-// whose reactions read records, whatever the laws.)  A
-// staged run also holds particles that no row lists; their records may be one
-// buffer ahead, which the tag test accepts (they are not used).  Bonded
-// partners read each other's records and so order each other in the same way.
+// that stages nothing waits for what it lists by gathering it, in every step of
+// a launch with reactions, whatever the laws.)  A staged run also holds particles
+// that no row lists; their records may be one buffer ahead, which the tag test
+// accepts (they are not used).  Bonded partners read each other's records and so
+// order each other in the same way.
 //
 // What bounds it: latency (the staged poll, the pair loop's shared-memory reads,
 // the tail of half the threads) and, with reactions, the resolution of pending
