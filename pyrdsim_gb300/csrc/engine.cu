@@ -1487,6 +1487,13 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
       for (int k = 0; k < D; k++) cells *= sd.nc[k];
       const double rows = D == 3 ? 9 : (D == 2 ? 3 : 1);
       touch = std::max(touch, rows * (per + 3.0 * sd.n / cells));
+      // where a row of cells in 2D holds few chunks, a chunk's run reaches over its
+      // end, and what it touches at both ends of a neighbouring row falls into the
+      // same chunks: all of those rows (one lane per particle, 128 a chunk: 16,000
+      // particles 14.1 us per step without this, half the chunks not staged, 9.4
+      // with it; 8,000, cutoff 4, 32.5 and 23.7)
+      const double row = sd.n / (cells / sd.nc[0]);
+      if (D == 2 && row < 2.5 * per) touch = std::max(touch, (std::ceil(per / row) + 3.0) * row);
       want = std::max(want, touch * (D == 3 ? 1.5 : 1.3) + 64);
       largest = std::max(largest, sd.n);
       h->rows = std::max(h->rows, sd.ntypes * sd.ntypes);
@@ -1498,14 +1505,14 @@ int rdsim_create(const rdsim_system* systems, int32_t n_systems, const rdsim_opt
     const int row = std::min(h->W, (int)(1.5 * list_expect) + 12), lanes = 2 * h->ltpp * h->lpc;
     h->kw = std::min((row + lanes - 1) / lanes, KW_LIMIT);
     // every chunk resident at once (its CTAs wait for each other), with less
-    // room for staging if need be, but for a tenth more than the chunks touch:
-    // where they do not fit their tables the per-step kernels are faster (3D,
-    // 39,304 and 46,656 particles, us per step: 47.3 and 49.1 with tables too
-    // small, 43.4 and 43.9 with the per-step kernels; at 32,768 40.9 with the
-    // latter, 39.8 with the largest table that fits, 1.4 times the touched; 2D,
-    // cutoff 5, 60,000: 33.7 with the latter, 32.6 with 1.2 times)
+    // room for staging if need be, but for a fifth more than the chunks touch, two
+    // fifths in 3D: where some do not fit their tables the per-step kernels are
+    // faster (3D, 39,304 and 46,656 particles, us per step: 47.3 and 49.1 with tables
+    // too small, 43.4 and 43.9 with the per-step kernels; at 45,000 36.9 with 1.1
+    // times the touched, 34.1 with the latter; at 32,768 40.9 with the latter, 39.8
+    // with 1.4 times; 2D, cutoff 5, 60,000: 33.7 with the latter, 32.6 with 1.2 times)
     const PeriodVariant v{D, h->ltpp, h->lpc, h->has_rx};
-    const int least = std::min(h->stg_max, slots(1.1 * touch));
+    const int least = std::min(h->stg_max, slots((D == 3 ? 1.4 : 1.2) * touch));
     for (int m = h->stg_max; m >= least && !h->period_on; m -= 64) {
       const long long room = (long long)period_blocks_per_sm(v, m, h->kw, h->rows) * sms;
       if (room >= nch) {

@@ -138,3 +138,25 @@ def test_period_kernel_of_every_variant(n, D, tpp, types):
                           np.arange(n, dtype=np.int32))
     lists, changed = _same_as_per_step(sd, (6, 47, 30), threads_per_particle=tpp)
     assert lists["lanes"] == (4 if tpp == 2 and D < 3 else 1) and changed > 0, (lists, changed)
+
+
+@pytest.mark.parametrize("n,rc", [(6000, 4.0), (8000, 4.0), (15000, 2.5), (16000, 2.5)])
+def test_tables_hold_chunks_that_reach_over_a_row_of_cells(n, rc):
+    """One lane per particle (chunks of 128) where a row of cells holds one or two
+    chunks: each touches whole rows, which its table has room for."""
+    from pyrdsim_gb300 import model
+    rng = np.random.default_rng(1)
+    side = int(np.ceil(np.sqrt(n)))
+    L = np.sqrt(n / 0.5)
+    g = np.stack(np.meshgrid(np.arange(side), np.arange(side), indexing="ij"), -1)
+    x = (g.reshape(-1, 2)[:n] + 0.5 + rng.uniform(-0.1, 0.1, (n, 2))) * (L / side)
+    m = model.Model.from_dict({
+        "n_dim": 2, "l": np.array([L, L]), "periodic": np.ones(2), "dt": 1e-5, "n_steps": 10,
+        "n_out": 1000000, "tau_by_taud": np.ones(1), "seed": 1,
+        "interactions": [{"type": "yukawa", "pair": [0, 0], "u0": 3.0, "r0": 1.0, "rc": rc}]})
+    mol = np.stack([np.arange(n), np.zeros(n, int), np.zeros(n, int)], 1).astype(np.int32)
+    sd = model.SystemData(m, x, np.zeros(n, np.int32), mol, np.arange(n, dtype=np.int32))
+    e = _engine([sd], threads_per_particle=1)
+    lists = e.test_lists()
+    assert lists["lanes"] == 1 and lists["unstaged"] == 0, lists
+    e.close()
