@@ -189,6 +189,7 @@ __device__ __noinline__ float3 period_gather(const ListShared& sh, const Args& a
 
 // A wait ran out, or another chunk recorded an error: the particles stay where
 // this chunk's last step left them.
+constexpr int GAVE_UP = 2;  // period_failed then
 template <int D, int PER, bool RX>
 __device__ __noinline__ void leave_state(const SysDev& s, const PeriodStage<D, PER>& st,
                                          const Args& a, int i, int p) {
@@ -280,8 +281,10 @@ __device__ __forceinline__ bool period_run_step(PeriodShared& ps,
     if (over) wait_failed(a, n);
   }
   // (a chunk that stages nothing has no wait that would notice an error)
-  if (__syncthreads_or(nstg < 0 && tid == 0 ? *(volatile int*)&a.err->code : period_failed))
+  if (__syncthreads_or(nstg < 0 && tid == 0 ? *(volatile int*)&a.err->code : period_failed)) {
+    period_failed = GAVE_UP;  // (every thread: k_period looks at it without a barrier)
     return false;
+  }
   const int lsmax = min(a.W, a.kw * 2 * TPP * LPC);
   // reactions of step n: each warp resolves the draws of its own particles
   // (no barrier: who needs another's type waits for its record)
@@ -485,10 +488,9 @@ __global__ void __launch_bounds__(LBLOCK, RD_PERIOD_MIN_BLOCKS)
     a0.stamps[((size_t)slot * gridDim.x + blockIdx.x) * 2] = global_timer();
 #pragma unroll 1
   for (int n = 0; n < p.nsteps; n++)
-    if (!period_run_step<D, TPP, LPC, RX>(ps, st, tb, sacc, a0, p, ch, nstg, n)) {
-      if (tid < ch.cnt) leave_state<D, PER, RX>(s, st, a0, ch.beg + tid, tid);
-      return;
-    }
+    if (!period_run_step<D, TPP, LPC, RX>(ps, st, tb, sacc, a0, p, ch, nstg, n)) break;
+  if (period_failed == GAVE_UP && tid < ch.cnt)
+    leave_state<D, PER, RX>(s, st, a0, ch.beg + tid, tid);
   if (a0.stamps && (tid & 31) == 0)
     atomicMax(a0.stamps + ((size_t)slot * gridDim.x + blockIdx.x) * 2 + 1, global_timer());
 }
